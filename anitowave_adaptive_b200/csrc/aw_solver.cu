@@ -21,6 +21,7 @@
 #include <memory>
 
 #include "aw_internal.cuh"
+#include "aw_uniform.cuh"
 
 namespace aw {
 
@@ -51,6 +52,12 @@ struct MGLevel {
     // dynamic shared memory of the batched kernels on this level
     size_t smem_smooth = 0, smem_x64 = 0, smem_prolong = 0, smem_meta = 0;
     int maxres = 0;
+    // the same blocks as warps of the uniform-coefficient kernels (aw_uniform.cuh): colour 0, colour 1
+    int2* udesc = nullptr;  // these four lie in the solver's uslab
+    int4* urec = nullptr;
+    float4* uwt = nullptr;
+    uint16_t* umask = nullptr;
+    int uwarps[2] = {0, 0};
     DBuf<float> W[3], bbar[3];
     DBuf<uint8_t> fluid;
     DBuf<float> x, b, r;
@@ -79,10 +86,15 @@ struct aw_solver {
     // level-0 bindings for the current solve
     float* x0 = nullptr;
     const float* b0 = nullptr;
-    // mixed precision: FP64 vectors of the conjugate-gradient outer loop (residual, direction,
-    // -A d), its scalars {rho, rho_old, d.(-A d)} and a zero right-hand side for applying A
-    aw::DBuf<double> p64tmp;
-    aw::DBuf<double> cg_r, cg_d, cg_q, cg_sc;
+    // the hierarchy can run the uniform-coefficient kernels (FV mode, 8^3 blocks at most, no activation
+    // or early exit), and the current solve does: every block's coefficients are uniform
+    bool uni_able = false, uni = false;
+    aw::DBuf<int4> uslab;  // slot records, weights, masks and warp descriptors of every level
+    // mixed precision: FP64 vectors of the conjugate-gradient outer loop (residual, direction (two
+    // buffers: the uniform form reads the old one while it writes the new), -A d), its scalars
+    // {rho, rho_old, d.(-A d)} and a zero right-hand side for applying A
+    aw::DBuf<double> cg_r, cg_d, cg_d2, cg_q, cg_sc;
+    aw::DBuf<unsigned> ticket;  // last_cta_sum: finished CTAs of the running launch (0 between launches)
     aw::DBuf<float> cg_zero;
     // FP32 conjugate gradients: direction, -A d, scalars {rho, rho_old, d.(-A d)}, partial sums
     aw::DBuf<float> cg32_d, cg32_q, cg32_sc, partials32;
@@ -93,11 +105,13 @@ struct aw_solver {
     cudaGraphExec_t cycle = nullptr;
     const void* cycle_x0 = nullptr;
     const void* cycle_b0 = nullptr;
+    int cycle_form = -1;  // 2 * uni + (level-0 x starts at zero)
     unsigned long long cycle_kernels = 0;
     // the mixed-precision CG iterations as one graph with a device-side while loop, per pressure
     // array; cgst = {iterations, restart flag, iteration limit}, cgprm = {||b||, tolerance}
     cudaGraphExec_t cgloop = nullptr;
     const void* cgloop_p = nullptr;
+    bool cgloop_uni = false;
     unsigned long long cgloop_kernels = 0;
     bool use_devloop = true;
     aw::DBuf<int> cgst;
@@ -105,7 +119,7 @@ struct aw_solver {
     bool use_graph = true;
     bool use_pdl = true;  // V-cycle kernels as programmatic dependent launches
     int tail = 0;         // first level of the uniform tail run as one k_dense_tail launch (0: none)
-    double* h_norm = nullptr;  // pinned host word for the per-iteration residual norm
+    double* h_norm = nullptr;  // pinned host words: a squared norm, the count of non-uniform blocks
     double* h_cg = nullptr;    // pinned host words of the device-loop state
     ~aw_solver() {
         if (cycle) cudaGraphExecDestroy(cycle);
@@ -157,10 +171,6 @@ __device__ inline double block_sum(double v, double* red) {
     return out;  // valid in thread 0
 }
 
-struct Coef3 {
-    const float* w[3];
-};
-
 // ------------------------------------------------------------------------------------------------
 // Batched block kernels.  A CTA serves `count` blocks ("slots") of one resolution r, listed
 // contiguously: 1 block of 8^3 or 16^3 cells, 4 of 4^3, 16 of 2^3, 64 of 1^3.  Every slot keeps
@@ -211,14 +221,6 @@ __device__ inline void cp_async8(void* s, const void* g) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_addr(s)), "l"(g) : "memory");
 }
 __device__ inline void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-// Programmatic dependent launch: the V-cycle's kernels are launched so that each may start while its
-// predecessor drains.  A kernel reads what its predecessor wrote only after pdl_wait() (which returns
-// once the predecessor grid has completed and its memory is visible; at once for a kernel launched
-// without the attribute), and lets its successor start with pdl_trigger() once its own main work is
-// issued.  Descriptors and slot metadata (fixed at solver build) are staged before the wait.
-__device__ inline void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ inline void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" :::); }
-
 // Sources of x for staging: FP32 (copied asynchronously), FP16 + per-block scale (decoded in
 // registers), FP64 (copied asynchronously).
 struct SrcX {
@@ -847,81 +849,105 @@ __global__ void __launch_bounds__(NT) k_prolong(XStore xf, XStore xc, const uint
 }
 
 // ---- conjugate-gradient outer loop of the mixed-precision solve (FP64 vectors) ----------------
-// dot(a, b) over fluid cells (b is FP64, or FP32 when bf is given), per-CTA partial sums
-__global__ void k_dot64(const double* __restrict__ a, const double* __restrict__ b, const float* __restrict__ bf,
-                        const uint8_t* __restrict__ fluid, size_t n, double* __restrict__ part) {
+// *out = dot(a, z) over fluid cells (a FP64, z FP32), two cells per thread and step
+__global__ void __launch_bounds__(256) k_dot64(const double* __restrict__ a, const float* __restrict__ z,
+                                               const uint8_t* __restrict__ fluid, size_t n, double* part,
+                                               unsigned* ticket, double* out) {
     pdl_wait();
     double acc = 0.0;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        if (fluid[i]) acc += a[i] * (bf ? (double)bf[i] : b[i]);
-    __shared__ double red[32];
-    acc = warp_sum(acc);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double t = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-        t = warp_sum(t);
-        if (threadIdx.x == 0) part[blockIdx.x] = t;
+    const size_t n2 = n / 2, step = (size_t)gridDim.x * blockDim.x, t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (size_t i = t0; i < n2; i += step) {
+        const double2 av = reinterpret_cast<const double2*>(a)[i];
+        const float2 zv = reinterpret_cast<const float2*>(z)[i];
+        const uchar2 f = reinterpret_cast<const uchar2*>(fluid)[i];
+        if (f.x) acc += av.x * (double)zv.x;
+        if (f.y) acc += av.y * (double)zv.y;
     }
+    if (t0 == 0 && (n & 1) && fluid[n - 1]) acc += a[n - 1] * (double)z[n - 1];
+    pdl_trigger();
+    last_cta_sum(acc, part, ticket, [&](double t) { *out = t; });
 }
 // z (FP32 V-cycle output) -> search direction d = z + beta d, beta = rho / rho_old (0 when first)
-// first_dev (when given) holds the restart flag on the device
+// *first: the restart flag
 __global__ void k_cg_direction(double* __restrict__ d, const float* __restrict__ z, const uint8_t* __restrict__ fluid,
-                               const double* __restrict__ sc, int first, const int* first_dev, size_t n) {
+                               const double* __restrict__ sc, const int* __restrict__ first, size_t n) {
     pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    if (first_dev) first = *first_dev;
-    const double beta = first ? 0.0 : sc[0] / sc[1];
+    const double beta = *first ? 0.0 : sc[0] / sc[1];
     d[i] = fluid[i] ? (double)z[i] + beta * d[i] : 0.0;
 }
-// qn = -A d (the residual kernel with a zero right-hand side); alpha = rho / (d . A d)
-// p += alpha d; r += alpha qn; and the FP32 copy of r for the next V-cycle
-// ... and the per-CTA partial sums of |r|^2 over fluid cells (grid-stride, part[blockIdx.x]);
-// rho_old = rho for the next iteration's direction (sc[1] is read by no CTA of this kernel)
-__global__ void k_cg_update(double* __restrict__ p, double* __restrict__ r, float* __restrict__ rf,
-                            const double* __restrict__ d, const double* __restrict__ qn, double* __restrict__ sc,
-                            const uint8_t* __restrict__ fluid, size_t n, double* __restrict__ part) {
+// The end of one CG iteration.  qn = -A d; alpha = rho / (d . A d); on fluid cells p += alpha d,
+// r += alpha qn, and the FP32 copy of r for the next V-cycle; rho_old = rho for the next iteration's
+// direction (sc[1] is read by no CTA of this kernel).  The last CTA to finish has |r|^2: it stores it,
+// counts the iteration, clears the restart flag and, in the device-side loop (DEV), runs the loop body
+// again while the residual is finite, at or above the tolerance and the iteration limit is not reached.
+// st = {iterations, restart, limit}, prm = {||b||, tolerance}; the direction is d1 in even iterations,
+// d0 in odd ones (the same buffer twice where it is updated in place).  One pass over the vectors:
+// 32 bytes read and 20 written per cell; two cells per thread and step.
+struct CgVec {
+    double* p;
+    int p_pairs;  // p is 16-byte aligned
+    double* r;
+    float* rf;
+    const double *d0, *d1, *qn;
+    double* sc;
+    const uint8_t* fluid;
+    size_t n;
+    double* norm2;
+    const double* prm;
+    int* st;
+};
+template <bool DEV>
+__global__ void __launch_bounds__(256) k_cg_update(CgVec K, double* part, unsigned* ticket, cudaGraphConditionalHandle h) {
     pdl_wait();
-    const double dq = -sc[2];
-    const double alpha = dq != 0.0 ? sc[0] / dq : 0.0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) sc[1] = sc[0];
+    const double dq = -K.sc[2];
+    const double alpha = dq != 0.0 ? K.sc[0] / dq : 0.0;
+    const double* __restrict__ d = (K.st[0] & 1) ? K.d0 : K.d1;
+    if (blockIdx.x == 0 && threadIdx.x == 0) K.sc[1] = K.sc[0];
     double acc = 0.0;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        p[i] += alpha * d[i];
-        const double rv = r[i] + alpha * qn[i];
-        r[i] = rv;
-        rf[i] = (float)rv;
-        if (fluid[i]) acc += rv * rv;
+    const size_t n2 = K.n / 2, step = (size_t)gridDim.x * blockDim.x, t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (size_t i = t0; i < n2; i += step) {
+        const uchar2 f = reinterpret_cast<const uchar2*>(K.fluid)[i];
+        if (!(f.x | f.y)) continue;
+        const double2 dv = reinterpret_cast<const double2*>(d)[i], qv = reinterpret_cast<const double2*>(K.qn)[i];
+        double2 rv = reinterpret_cast<const double2*>(K.r)[i];
+        double2 pv = K.p_pairs ? reinterpret_cast<const double2*>(K.p)[i] : make_double2(K.p[2 * i], K.p[2 * i + 1]);
+        if (f.x) {
+            pv.x += alpha * dv.x;
+            rv.x = rv.x + alpha * qv.x;
+            acc += rv.x * rv.x;
+        }
+        if (f.y) {
+            pv.y += alpha * dv.y;
+            rv.y = rv.y + alpha * qv.y;
+            acc += rv.y * rv.y;
+        }
+        if (K.p_pairs) {
+            reinterpret_cast<double2*>(K.p)[i] = pv;
+        } else {
+            K.p[2 * i] = pv.x;
+            K.p[2 * i + 1] = pv.y;
+        }
+        reinterpret_cast<double2*>(K.r)[i] = rv;
+        reinterpret_cast<float2*>(K.rf)[i] = make_float2((float)rv.x, (float)rv.y);
     }
-    __shared__ double red[32];
-    acc = warp_sum(acc);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double t = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-        t = warp_sum(t);
-        if (threadIdx.x == 0) part[blockIdx.x] = t;
+    if (t0 == 0 && (K.n & 1) && K.fluid[K.n - 1]) {
+        const size_t i = K.n - 1;
+        K.p[i] += alpha * d[i];
+        const double rv = K.r[i] + alpha * K.qn[i];
+        K.r[i] = rv;
+        K.rf[i] = (float)rv;
+        acc += rv * rv;
     }
-}
-// End of one CG iteration inside the device-side loop (one CTA of 256 threads): ||r||^2 into norm2
-// from k_cg_update's partial sums (the reduction of k_reduce_sum, so the host loop reads the same
-// value), count the iteration, clear the restart flag, and run the loop body again while the
-// residual is finite, at or above the tolerance and the iteration limit is not reached.
-// st = {iterations, restart, limit}, prm = {||b||, tolerance}.
-__global__ void k_cg_check(cudaGraphConditionalHandle h, const double* __restrict__ part, int nparts,
-                           double* __restrict__ norm2, const double* __restrict__ prm, int* st) {
-    __shared__ double red[32];
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x) acc += part[i];
-    const double t = block_sum(acc, red);
-    if (threadIdx.x != 0) return;
-    norm2[0] = t;
-    const double rel = sqrt(t) / prm[0];
-    const int it = st[0] + 1;
-    st[0] = it;
-    st[1] = 0;
-    cudaGraphSetConditional(h, (rel == rel && rel >= prm[1] && it < st[2]) ? 1u : 0u);
+    last_cta_sum(acc, part, ticket, [&](double t) {
+        K.norm2[0] = t;
+        const double rel = sqrt(t) / K.prm[0];
+        const int it = K.st[0] + 1;
+        K.st[0] = it;
+        K.st[1] = 0;
+        if constexpr (DEV) cudaGraphSetConditional(h, (rel == rel && rel >= K.prm[1] && it < K.st[2]) ? 1u : 0u);
+    });
 }
 __global__ void k_fill_zero(float* __restrict__ x, size_t n) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -995,11 +1021,6 @@ __global__ void k_copy_scalar32(float* __restrict__ sc, int dst, int src) {
     sc[dst] = sc[src];
 }
 
-__global__ void k_accum64(double* __restrict__ p, const float* __restrict__ e, size_t n) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] += (double)e[i];
-}
-
 __global__ void k_reduce_sum(const double* __restrict__ part, int n, double* out) {
     pdl_wait();
     __shared__ double red[32];
@@ -1009,22 +1030,14 @@ __global__ void k_reduce_sum(const double* __restrict__ part, int n, double* out
     if (threadIdx.x == 0) *out = t;
 }
 
-// sum of b^2 over fluid cells (or all cells)
-__global__ void k_sumsq(const float* __restrict__ v, const uint8_t* __restrict__ fluid, size_t n, int check_fluid,
-                        double* part) {
-    __shared__ double red[32];
+// *out = sum of v^2 over fluid cells (or all cells)
+__global__ void __launch_bounds__(256) k_sumsq(const float* __restrict__ v, const uint8_t* __restrict__ fluid, size_t n,
+                                               int check_fluid, double* part, unsigned* ticket, double* out) {
     double acc = 0.0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         if (!check_fluid || fluid[i]) acc += (double)v[i] * (double)v[i];
-    double t = block_sum(acc, red);
-    if (threadIdx.x == 0) part[blockIdx.x] = t;
+    last_cta_sum(acc, part, ticket, [&](double t) { *out = t; });
 }
-
-__global__ void k_zero_scale(float* s, int n) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) s[i] = 0.f;
-}
-
 // ---------------------------------- uniform (dense) levels ------------------------------------
 struct DenseArgs {
     DenseView d;
@@ -1736,10 +1749,6 @@ static Batch batch(const MGLevel& L, int k) { return Batch{L.desc[k].p, L.meta[k
 // Slot metadata of one batch of level m, laid out in batch order (field-major): block id, offsets,
 // the six face neighbours (cell offset, kind, block) and the block's cells on the adjacent levels.
 // One thread per slot, from the level arrays already on the device (no host copy of the offsets).
-struct MetaSrc {
-    const int* res;
-    const uint32_t* off[4];
-};
 __global__ void k_build_meta(Geo geo, const int* __restrict__ blocks, int n, MetaSrc h, MetaSrc finer, MetaSrc coarser,
                              int* __restrict__ mt) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2008,6 +2017,228 @@ static aw_status vcycle(aw_solver* S, int m, cudaStream_t s) {
     return AW_OK;
 }
 
+// ---- uniform coefficients: the register-resident kernels of aw_uniform.cuh -----------------------
+// Slots, warps and slot records of every block-structured level.  All levels list their blocks in one
+// order (colour 0 then 1, native resolutions descending: a level's resolutions then descend too), in
+// one device allocation filled by one copy.
+static aw_status build_uniform(aw_solver* S, cudaStream_t s) {
+    const Geo& geo = S->g->st.geo;
+    const std::vector<int>& res = S->lv[0].h_res;
+    const int nl = S->nmsbg;
+    size_t cnt[2][UNI_MAX_RES + 1] = {}, at[2][UNI_MAX_RES + 1];
+    auto each = [&](auto f) {
+        int b = 0;
+        for (int z = 0; z < geo.D[2]; ++z)
+            for (int y = 0; y < geo.D[1]; ++y)
+                for (int x = 0; x < geo.D[0]; ++x, ++b)
+                    if (res[b]) f(b, (x + y + z) & 1, res[b]);
+    };
+    each([&](int, int k, int r) { ++cnt[k][r]; });
+    size_t n = 0;
+    for (int k = 0; k < 2; ++k)
+        for (int r = UNI_MAX_RES; r >= 1; --r) {
+            at[k][r] = n;
+            n += cnt[k][r];
+        }
+    // host image: the blocks of the slots, then every level's warp descriptors
+    std::vector<int> img(n);
+    each([&](int b, int k, int r) { img[at[k][r]++] = b; });
+    size_t ndesc[UNI_MAX_LEVELS] = {}, d0[UNI_MAX_LEVELS] = {};
+    if (img.size() & 1) img.push_back(0);
+    for (int m = 0; m < nl; ++m) {
+        d0[m] = img.size();
+        size_t first = 0;
+        for (int k = 0; k < 2; ++k) {
+            const size_t w0 = ndesc[m];
+            for (int r = UNI_MAX_RES >> m; r >= 1; r >>= 1) {
+                size_t c = 0;  // native resolutions that are r here (1 takes all that vanish)
+                for (int q = 1; q <= UNI_MAX_RES; q <<= 1)
+                    if (std::max(q >> m, 1) == r) c += cnt[k][q];
+                const size_t G = (size_t)uni_blocks_per_warp(r);
+                for (size_t i = 0; i < c; i += G, ++ndesc[m]) {
+                    img.push_back((int)(first + i));
+                    img.push_back((int)std::min(G, c - i) | (r << 8));
+                }
+                first += c;
+            }
+            S->lv[m].uwarps[k] = (int)(ndesc[m] - w0);
+        }
+    }
+    auto q16 = [](size_t bytes) { return (bytes + 15) / 16; };
+    size_t tot = q16(img.size() * sizeof(int)), o_rec[UNI_MAX_LEVELS], o_wt[UNI_MAX_LEVELS], o_mask[UNI_MAX_LEVELS];
+    for (int m = 0; m < nl; ++m) {
+        o_rec[m] = tot;
+        o_wt[m] = o_rec[m] + n * UREC;
+        o_mask[m] = o_wt[m] + 2 * n;
+        tot = o_mask[m] + q16(ndesc[m] * 32 * sizeof(uint16_t));
+    }
+    AW_TRY(S->uslab.ensure(std::max<size_t>(tot, 1)));
+    if (!n) return AW_OK;
+    AW_CUDA(cudaMemcpyAsync(S->uslab.p, img.data(), img.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+    const int* blk = reinterpret_cast<const int*>(S->uslab.p);
+    for (int m = 0; m < nl; ++m) {
+        MGLevel& L = S->lv[m];
+        L.udesc = reinterpret_cast<int2*>(S->uslab.p) + d0[m] / 2;
+        L.urec = S->uslab.p + o_rec[m];
+        L.uwt = reinterpret_cast<float4*>(S->uslab.p + o_wt[m]);
+        L.umask = reinterpret_cast<uint16_t*>(S->uslab.p + o_mask[m]);
+        k_build_records<<<nblk(n), 256, 0, s>>>(geo, blk, (int)n, meta_src(&L), meta_src(m + 1 < nl ? &S->lv[m + 1] : nullptr),
+                                                reinterpret_cast<int*>(L.urec));
+        AW_LAUNCH();
+    }
+    return AW_OK;
+}
+
+static UniView uview(const MGLevel& L, int k) {  // k: colour 0, 1, or 2 for both
+    UniView V;
+    V.desc = L.udesc;
+    V.rec = L.urec;
+    V.wt = L.uwt;
+    V.mask = L.umask;
+    V.first = k == 1 ? L.uwarps[0] : 0;
+    V.nwarp = k == 2 ? L.uwarps[0] + L.uwarps[1] : L.uwarps[k];
+    return V;
+}
+static unsigned ugrid(const UniView& V) { return (unsigned)((V.nwarp + UWARPS - 1) / UWARPS); }
+template <bool HALF>
+static UX<HALF> ux(const XStore& x) {
+    return UX<HALF>{x.f, x.h, x.scale};
+}
+
+// Which blocks of which levels are uniform; *S->norm[1] (as an int) receives the number of live blocks
+// that are not.  Clears x of the blocks without fluid on the levels whose x starts at zero (level 0
+// too with own_x0: then x0 is the solver's array), and both direction buffers there.
+static aw_status uniform_check(aw_solver* S, bool own_x0, cudaStream_t s) {
+    UCheckAll K{};
+    unsigned grid = 1;
+    for (int m = 0; m < S->nmsbg; ++m) {
+        MGLevel& L = S->lv[m];
+        K.v[m] = uview(L, 2);
+        UCheck& c = K.k[m];
+        c.W = coef(L);
+        c.fluid = L.fluid.p;
+        if (m > 0 || own_x0) {
+            c.x = L.half ? nullptr : L.x.p;
+            c.xh = L.half ? L.xh.p : nullptr;
+            c.scale = L.xscale.p;
+        }
+        if (m == 0 && own_x0 && S->d.precision == AW_PRECISION_MIXED) {
+            c.d0 = S->cg_d.p;
+            c.d1 = S->cg_d2.p;
+        }
+        c.wt = L.uwt;
+        c.mask = L.umask;
+        c.counts = reinterpret_cast<int*>(S->norm.p + 1);
+        grid = std::max(grid, ugrid(K.v[m]));
+    }
+    AW_CUDA(cudaMemsetAsync(S->norm.p + 1, 0, sizeof(double), s));
+    k_uni_check<<<dim3(grid, S->nmsbg), UNT, 0, s>>>(K);
+    AW_LAUNCH();
+    return AW_OK;
+}
+
+// One colour of one smoothing iteration on level m in the given mode.
+template <bool HALF, int MODE, bool HC>
+static aw_status uni_smooth_t(aw_solver* S, int m, int k, int rev, cudaStream_t s) {
+    MGLevel& L = S->lv[m];
+    const UniView V = uview(L, k);
+    if (!V.nwarp) return AW_OK;
+    const bool prol = MODE == UM_PROLONG_ALL || MODE == UM_PROLONG_OWN;
+    return launch_dep(S, k_uni_smooth<HALF, MODE, HC>, ugrid(V), UNT, 0, s, V, ux<HALF>(xstore(S, m)),
+                      prol ? ux<HC>(xstore(S, m + 1)) : UX<HC>{}, bptr(S, m), S->d.omega, (int)S->d.block_iterations, rev);
+}
+static aw_status uni_smooth(aw_solver* S, int m, int k, int rev, int mode, cudaStream_t s) {
+    const bool half = S->lv[m].half && !(m == 0 && S->x0);
+    if (mode == UM_PROLONG_ALL || mode == UM_PROLONG_OWN) {
+        const bool hc = S->lv[m + 1].half, all = mode == UM_PROLONG_ALL;
+        if (hc) return all ? uni_smooth_t<false, UM_PROLONG_ALL, true>(S, m, k, rev, s)
+                           : uni_smooth_t<false, UM_PROLONG_OWN, true>(S, m, k, rev, s);
+        return all ? uni_smooth_t<false, UM_PROLONG_ALL, false>(S, m, k, rev, s)
+                   : uni_smooth_t<false, UM_PROLONG_OWN, false>(S, m, k, rev, s);
+    }
+    switch (mode) {
+        case UM_ZERO_ALL:
+            return half ? uni_smooth_t<true, UM_ZERO_ALL, false>(S, m, k, rev, s)
+                        : uni_smooth_t<false, UM_ZERO_ALL, false>(S, m, k, rev, s);
+        case UM_ZERO_OWN:
+            return half ? uni_smooth_t<true, UM_ZERO_OWN, false>(S, m, k, rev, s)
+                        : uni_smooth_t<false, UM_ZERO_OWN, false>(S, m, k, rev, s);
+        default:
+            return half ? uni_smooth_t<true, UM_PLAIN, false>(S, m, k, rev, s)
+                        : uni_smooth_t<false, UM_PLAIN, false>(S, m, k, rev, s);
+    }
+}
+
+// r = b - A x of level m: into out (r, or restricted), with the sum of r^2 into *sum when given
+static aw_status uni_residual(aw_solver* S, int m, const XStore& x, const float* b, const UOut& out, double* sum,
+                              cudaStream_t s) {
+    const UniView V = uview(S->lv[m], 2);
+    if (!V.nwarp) return AW_OK;
+    if (x.h)
+        return launch_dep(S, k_uni_residual<true>, ugrid(V), UNT, 0, s, V, ux<true>(x), b, out, S->partials.p,
+                          S->ticket.p, sum);
+    return launch_dep(S, k_uni_residual<false>, ugrid(V), UNT, 0, s, V, ux<false>(x), b, out, S->partials.p, S->ticket.p,
+                      sum);
+}
+
+// The V-cycle on a hierarchy whose live blocks are all uniform: the steps of vcycle() with the
+// residual restricted as it is taken, levels starting at zero without a clearing pass (zero: this
+// level does), and the correction of an FP32 level added where its first post-smoothing reads it.
+static aw_status uni_vcycle(aw_solver* S, int m, bool zero, cudaStream_t s) {
+    const int last = (int)S->lv.size() - 1;
+    MGLevel& L = S->lv[m];
+    if (m == last || L.dense) {
+        if (zero) AW_TRY(zero_x(S, m, s));
+        return vcycle(S, m, s);
+    }
+    if (zero && S->d.pre_smooth == 0) AW_TRY(zero_x(S, m, s));
+    for (int it = 0; it < S->d.pre_smooth; ++it)
+        for (int k = 0; k < 2; ++k) {
+            const int mode = zero && it == 0 ? (k == 0 ? UM_ZERO_ALL : UM_ZERO_OWN) : UM_PLAIN;
+            AW_TRY(uni_smooth(S, m, k, 0, mode, s));
+        }
+    MGLevel& K = S->lv[m + 1];
+    const XStore x = xstore(S, m);
+    UOut out{};
+    if (K.dense) {
+        out.r = L.r.p;
+    } else {
+        out.bc = K.b.p;
+        out.fluid_c = K.fluid.p;
+    }
+    AW_TRY(uni_residual(S, m, x, bptr(S, m), out, nullptr, s));
+    int mode = UM_PLAIN;
+    if (S->tail && m + 1 == S->tail) {
+        AW_TRY(dense_tail(S, m, s));
+    } else if (K.dense) {
+        AW_TRY(restrict_level(S, m, s));
+        AW_TRY(zero_x(S, m + 1, s));
+        AW_TRY(vcycle(S, m + 1, s));
+        AW_TRY(prolong_level(S, m, s));
+    } else {
+        AW_TRY(uni_vcycle(S, m + 1, true, s));
+        if (x.h || S->d.post_smooth == 0) {
+            const UniView V = uview(L, 2);
+            if (x.h && K.half)
+                AW_TRY(launch_dep(S, k_uni_prolong<true, true>, ugrid(V), UNT, 0, s, V, ux<true>(x), ux<true>(xstore(S, m + 1))));
+            else if (x.h)
+                AW_TRY(launch_dep(S, k_uni_prolong<true, false>, ugrid(V), UNT, 0, s, V, ux<true>(x), ux<false>(xstore(S, m + 1))));
+            else if (K.half)
+                AW_TRY(launch_dep(S, k_uni_prolong<false, true>, ugrid(V), UNT, 0, s, V, ux<false>(x), ux<true>(xstore(S, m + 1))));
+            else
+                AW_TRY(launch_dep(S, k_uni_prolong<false, false>, ugrid(V), UNT, 0, s, V, ux<false>(x), ux<false>(xstore(S, m + 1))));
+        } else {
+            mode = UM_PROLONG_ALL;
+        }
+    }
+    for (int it = 0; it < S->d.post_smooth; ++it)
+        for (int k = 1; k >= 0; --k) {
+            const int md = it == 0 && mode == UM_PROLONG_ALL ? (k == 1 ? UM_PROLONG_ALL : UM_PROLONG_OWN) : UM_PLAIN;
+            AW_TRY(uni_smooth(S, m, k, 1, md, s));
+        }
+    return AW_OK;
+}
+
 }  // namespace aw
 
 using namespace aw;
@@ -2220,6 +2451,14 @@ static aw_status solver_build(aw_solver* S) {
         S->smem_max = std::max({S->smem_max, L.smem_smooth, L.smem_prolong, L.smem_meta});
         S->smem_max64 = std::max(S->smem_max64, L.smem_x64);
     }
+    // the uniform-coefficient kernels take FV levels of at most 8^3 blocks without activation flags or
+    // per-block early exit (the FV defaults; k_smooth tracks block residuals otherwise)
+    const bool track = S->d.target_reduction > 0.f && (S->d.block_iterations > 2 ||
+                                                      (S->d.block_iterations == 2 && S->d.target_reduction >= 1.f));
+    S->uni_able = !ref && S->d.theta < 0.f && !track && G.geo.R0 <= UNI_MAX_RES && S->nmsbg > 0 &&
+                  S->nmsbg <= UNI_MAX_LEVELS && getenv("AW_NO_UNIFORM") == nullptr;
+    S->uni = false;
+    if (S->uni_able) AW_TRY(build_uniform(S, s));
     // uniform continuation below one cell per block (FV mode)
     size_t used = (size_t)S->nmsbg;
     if (!ref && S->nmsbg > 0 && S->lv[S->nmsbg - 1].maxres == 1) {
@@ -2277,11 +2516,17 @@ static aw_status solver_build(aw_solver* S) {
         const size_t nc0 = S->lv[0].ncell();
         AW_TRY(S->cg_r.ensure(nc0));
         AW_TRY(S->cg_d.ensure(nc0));
+        AW_TRY(S->cg_d2.ensure(nc0));
         AW_TRY(S->cg_q.ensure(nc0));
         AW_TRY(S->cg_sc.ensure(4));
         AW_TRY(S->cg_zero.ensure(nc0));
         AW_CUDA(cudaMemset(S->cg_zero.p, 0, nc0 * sizeof(float)));
         AW_CUDA(cudaMemset(S->cg_d.p, 0, nc0 * sizeof(double)));
+        AW_CUDA(cudaMemset(S->cg_d2.p, 0, nc0 * sizeof(double)));
+        AW_CUDA(cudaMemset(S->cg_r.p, 0, nc0 * sizeof(double)));
+        AW_CUDA(cudaMemset(S->cg_q.p, 0, nc0 * sizeof(double)));
+        AW_TRY(S->cgst.ensure(4));
+        AW_TRY(S->cgprm.ensure(2));
     }
     if (S->d.precision == AW_PRECISION_FP32_PCG) {
         const size_t nc0 = S->lv[0].ncell();
@@ -2292,10 +2537,14 @@ static aw_status solver_build(aw_solver* S) {
         AW_TRY(S->partials32.ensure(4096));
         AW_CUDA(cudaMemset(S->cg_zero.p, 0, std::max<size_t>(nc0, 1) * sizeof(float)));
         AW_CUDA(cudaMemset(S->cg32_d.p, 0, std::max<size_t>(nc0, 1) * sizeof(float)));
+        AW_CUDA(cudaMemset(S->cg32_q.p, 0, std::max<size_t>(nc0, 1) * sizeof(float)));
     }
-    size_t nparts = (size_t)nb + 1024;
+    // partial sums: one per CTA of the widest launch (batches and uniform warps hold at least one block)
+    size_t nparts = (size_t)nb + 2048;
     AW_TRY(S->partials.ensure(nparts));
     AW_TRY(S->norm.ensure(2));
+    AW_TRY(S->ticket.ensure(1));
+    AW_CUDA(cudaMemset(S->ticket.p, 0, sizeof(unsigned)));
     S->use_graph = getenv("AW_NO_GRAPH") == nullptr;
     S->use_pdl = getenv("AW_NO_PDL") == nullptr;
     S->use_devloop = getenv("AW_NO_DEVLOOP") == nullptr;
@@ -2435,12 +2684,19 @@ extern "C" aw_status aw_mg_prolongate(aw_solver* S, int32_t m, aw_stream s) {
     AW_CHECK_ARG(S && m >= 0 && m + 1 < (int)S->lv.size(), "bad argument");
     return prolong_level(S, m, (cudaStream_t)s);
 }
-// One V-cycle, replayed from a CUDA graph (captured on first use for the current level-0 x/b).
-static aw_status run_vcycle(aw_solver* S, cudaStream_t s) {
-    if (!S->use_graph) return vcycle(S, 0, s);
+// One V-cycle of the current solve; zero: the level-0 x starts at zero (whatever it holds).
+static aw_status solve_vcycle(aw_solver* S, bool zero, cudaStream_t s) {
+    if (S->uni) return uni_vcycle(S, 0, zero, s);
+    if (zero) AW_TRY(zero_x(S, 0, s));
+    return vcycle(S, 0, s);
+}
+// ... replayed from a CUDA graph (captured on first use for the current level-0 x/b and form).
+static aw_status run_vcycle(aw_solver* S, bool zero, cudaStream_t s) {
+    if (!S->use_graph) return solve_vcycle(S, zero, s);
     const void* x0 = S->x0 ? (const void*)S->x0 : (const void*)S->lv[0].x.p;
     const void* b0 = S->b0 ? (const void*)S->b0 : (const void*)S->lv[0].b.p;
-    if (!S->cycle || S->cycle_x0 != x0 || S->cycle_b0 != b0) {
+    const int form = (S->uni ? 2 : 0) + (zero ? 1 : 0);
+    if (!S->cycle || S->cycle_x0 != x0 || S->cycle_b0 != b0 || S->cycle_form != form) {
         if (S->cycle) {
             cudaGraphExecDestroy(S->cycle);
             S->cycle = nullptr;
@@ -2448,7 +2704,7 @@ static aw_status run_vcycle(aw_solver* S, cudaStream_t s) {
         if (!S->cap) AW_CUDA(cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking));
         const unsigned long long l0 = g_launches;
         AW_CUDA(cudaStreamBeginCapture(S->cap, cudaStreamCaptureModeThreadLocal));
-        aw_status st = vcycle(S, 0, S->cap);
+        aw_status st = solve_vcycle(S, zero, S->cap);
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(S->cap, &graph);
         S->cycle_kernels = g_launches - l0;
@@ -2466,6 +2722,7 @@ static aw_status run_vcycle(aw_solver* S, cudaStream_t s) {
         }
         S->cycle_x0 = x0;
         S->cycle_b0 = b0;
+        S->cycle_form = form;
     }
     AW_CUDA(cudaGraphLaunch(S->cycle, s));
     g_launches += S->cycle_kernels;
@@ -2481,52 +2738,107 @@ extern "C" aw_status aw_vcycle_run(aw_solver* S, aw_stream s) {
     return vcycle(S, 0, (cudaStream_t)s);
 }
 
+// *out = sqrt of the sum in S->norm[0], read back (syncs); counts the non-uniform blocks too
+static aw_status fetch_norm(aw_solver* S, cudaStream_t s, double* out) {
+    if (!S->h_norm) AW_CUDA(cudaHostAlloc((void**)&S->h_norm, 2 * sizeof(double), cudaHostAllocDefault));
+    AW_CUDA(cudaMemcpyAsync(S->h_norm, S->norm.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
+    AW_CUDA(cudaStreamSynchronize(s));
+    *out = std::sqrt(S->h_norm[0]);
+    return AW_OK;
+}
 static aw_status read_norm(aw_solver* S, int nparts, cudaStream_t s, double* out) {
     k_reduce_sum<<<1, 256, 0, s>>>(S->partials.p, nparts, S->norm.p);
     AW_LAUNCH();
-    if (!S->h_norm) AW_CUDA(cudaHostAlloc((void**)&S->h_norm, sizeof(double), cudaHostAllocDefault));
-    AW_CUDA(cudaMemcpyAsync(S->h_norm, S->norm.p, sizeof(double), cudaMemcpyDeviceToHost, s));
-    AW_CUDA(cudaStreamSynchronize(s));
-    *out = std::sqrt(*S->h_norm);
-    return AW_OK;
+    return fetch_norm(S, s, out);
 }
 
-// Mixed-precision CG iterations on the device until the recursive residual falls below the
-// tolerance, turns NaN or the iteration limit is reached: one graph whose while node repeats the
-// iteration (V-cycle preconditioner, the two dot products, the direction, A d and the update) and
-// a check kernel that sets the loop condition, so no host round trip separates iterations.  The
-// kernels and their order are those of the host-driven loop, so the results are identical.  The
-// graph is built per pressure array.  Returns false (state unchanged) when the device cannot
-// build such a graph; the caller then keeps the host loop.
-static aw_status cg_body(aw_solver* S, double* p, unsigned ndot, cudaStream_t s, cudaGraphConditionalHandle h) {
+// r = b - A p into r (FP32) and r64, and ||r||: the true residual of the outer loops (FP32 or FP64 p)
+static aw_status true_residual(aw_solver* S, const float* p32, const double* p64, const float* b, float* r, double* r64,
+                               cudaStream_t s, double* norm) {
+    MGLevel& L0 = S->lv[0];
+    const int cf = fv(S) ? 1 : 0;
+    XStore xp;
+    xp.f = const_cast<float*>(p32);
+    if (S->uni) {
+        UOut out{};
+        out.r = r;
+        out.r64 = r64;
+        const UniView V = uview(L0, 2);
+        if (!V.nwarp) AW_CUDA(cudaMemsetAsync(S->norm.p, 0, sizeof(double), s));
+        else if (p64) {
+            k_uni_residual64<<<ugrid(V), UNT, 0, s>>>(V, USrcD{p64}, b, out, S->partials.p, S->ticket.p, S->norm.p);
+            AW_LAUNCH();
+        } else {
+            AW_TRY(uni_residual(S, 0, xp, b, out, S->norm.p, s));
+        }
+        return fetch_norm(S, s, norm);
+    }
+    if (L0.ndesc[2]) {
+        if (p64)
+            k_residual<SrcD><<<L0.ndesc[2], 256, L0.smem_x64, s>>>(SrcD{p64}, b, coef(L0), L0.fluid.p, batch(L0, 2), cf, r,
+                                                                   r64, S->partials.p);
+        else
+            k_residual<SrcX><<<L0.ndesc[2], 256, L0.smem_smooth, s>>>(SrcX{xp}, b, coef(L0), L0.fluid.p, batch(L0, 2), cf,
+                                                                      r, r64, S->partials.p);
+        AW_LAUNCH();
+    }
+    return read_norm(S, L0.ndesc[2], s, norm);
+}
+
+// One mixed-precision CG iteration: z = V(r) (r in FP32 in the level-0 right-hand side), rho = r . z,
+// d = z + (rho / rho_old) d, q = -A d with d . q, then k_cg_update.  The same kernels in the
+// device-side loop (h given) and in the host-driven one.
+static aw_status cg_iteration(aw_solver* S, double* p, unsigned ndot, cudaStream_t s, const cudaGraphConditionalHandle* h) {
     MGLevel& L0 = S->lv[0];
     const size_t nc = L0.ncell();
     const int cf = fv(S) ? 1 : 0;
     double* sc = S->cg_sc.p;
-    k_fill_zero<<<nblk(nc), 256, 0, s>>>(L0.x.p, nc);
-    AW_LAUNCH();
-    AW_TRY(vcycle(S, 0, s));
-    AW_TRY(launch_dep(S, k_dot64, ndot, 256, 0, s, S->cg_r.p, (const double*)nullptr, L0.x.p, L0.fluid.p, nc,
-                      S->partials.p));
-    AW_TRY(launch_dep(S, k_reduce_sum, 1, 256, 0, s, S->partials.p, (int)ndot, sc + 0));
-    AW_TRY(launch_dep(S, k_cg_direction, nblk(nc), 256, 0, s, S->cg_d.p, L0.x.p, L0.fluid.p, sc, 0,
-                      (const int*)(S->cgst.p + 1), nc));
-    AW_TRY(launch_dep(S, k_apply_dot, (unsigned)L0.ndesc[2], 256, L0.smem_x64, s, SrcD{S->cg_d.p}, S->cg_zero.p,
-                      coef(L0), L0.fluid.p, batch(L0, 2), cf, S->cg_q.p, S->partials.p));
-    AW_TRY(launch_dep(S, k_reduce_sum, 1, 256, 0, s, S->partials.p, L0.ndesc[2], sc + 2));
-    AW_TRY(launch_dep(S, k_cg_update, ndot, 256, 0, s, p, S->cg_r.p, L0.b.p, S->cg_d.p, S->cg_q.p, sc, L0.fluid.p, nc,
-                      S->partials.p));
-    k_cg_check<<<1, 256, 0, s>>>(h, (const double*)S->partials.p, (int)ndot, S->norm.p, S->cgprm.p, S->cgst.p);
-    AW_LAUNCH();
-    return AW_OK;
+    if (h) AW_TRY(solve_vcycle(S, true, s));
+    else AW_TRY(run_vcycle(S, true, s));
+    AW_TRY(launch_dep(S, k_dot64, ndot, 256, 0, s, (const double*)S->cg_r.p, (const float*)L0.x.p,
+                      (const uint8_t*)L0.fluid.p, nc, S->partials.p, S->ticket.p, sc + 0));
+    CgVec K{};
+    if (S->uni) {
+        K.d0 = S->cg_d.p;
+        K.d1 = S->cg_d2.p;
+        UOut out{};
+        out.r64 = S->cg_q.p;
+        const UniView V = uview(L0, 2);
+        AW_TRY(launch_dep(S, k_uni_apply, ugrid(V), UNT, 0, s, V, (const float*)L0.x.p, S->cg_d.p, S->cg_d2.p, out,
+                          (const double*)sc, (const int*)S->cgst.p, S->partials.p, S->ticket.p, sc + 2));
+    } else {
+        K.d0 = K.d1 = S->cg_d.p;
+        AW_TRY(launch_dep(S, k_cg_direction, nblk(nc), 256, 0, s, S->cg_d.p, (const float*)L0.x.p,
+                          (const uint8_t*)L0.fluid.p, (const double*)sc, (const int*)(S->cgst.p + 1), nc));
+        AW_TRY(launch_dep(S, k_apply_dot, (unsigned)L0.ndesc[2], 256, L0.smem_x64, s, SrcD{S->cg_d.p}, S->cg_zero.p,
+                          coef(L0), L0.fluid.p, batch(L0, 2), cf, S->cg_q.p, S->partials.p));
+        AW_TRY(launch_dep(S, k_reduce_sum, 1, 256, 0, s, S->partials.p, L0.ndesc[2], sc + 2));
+    }
+    K.p = p;
+    K.p_pairs = ((uintptr_t)p & 15u) == 0;
+    K.r = S->cg_r.p;
+    K.rf = L0.b.p;
+    K.qn = S->cg_q.p;
+    K.sc = sc;
+    K.fluid = L0.fluid.p;
+    K.n = nc;
+    K.norm2 = S->norm.p;
+    K.prm = S->cgprm.p;
+    K.st = S->cgst.p;
+    if (h) return launch_dep(S, k_cg_update<true>, ndot, 256, 0, s, K, S->partials.p, S->ticket.p, *h);
+    return launch_dep(S, k_cg_update<false>, ndot, 256, 0, s, K, S->partials.p, S->ticket.p, cudaGraphConditionalHandle{});
 }
 
+// Mixed-precision CG iterations on the device until the recursive residual falls below the
+// tolerance, turns NaN or the iteration limit is reached: one graph whose while node repeats the
+// iteration; the update kernel's last CTA sets the loop condition, so no host round trip separates
+// iterations.  The graph is built per pressure array and form.  Returns false (state unchanged) when
+// the device cannot build such a graph; the caller then keeps the host loop.
 static bool cg_devloop_build(aw_solver* S, double* p, unsigned ndot) {
     if (S->cgloop) {
         cudaGraphExecDestroy(S->cgloop);
         S->cgloop = nullptr;
     }
-    if (S->cgst.ensure(4) != AW_OK || S->cgprm.ensure(2) != AW_OK) return false;
     if (!S->cap && cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking) != cudaSuccess) return false;
     cudaGraph_t g = nullptr;
     if (cudaGraphCreate(&g, 0) != cudaSuccess) return false;
@@ -2544,7 +2856,7 @@ static bool cg_devloop_build(aw_solver* S, double* p, unsigned ndot) {
             const unsigned long long l0 = g_launches;
             if (cudaStreamBeginCaptureToGraph(S->cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) ==
                 cudaSuccess) {
-                const aw_status st = cg_body(S, p, ndot, S->cap, h);
+                const aw_status st = cg_iteration(S, p, ndot, S->cap, &h);
                 cudaGraph_t out = nullptr;
                 const cudaError_t e = cudaStreamEndCapture(S->cap, &out);
                 S->cgloop_kernels = g_launches - l0;
@@ -2560,6 +2872,7 @@ static bool cg_devloop_build(aw_solver* S, double* p, unsigned ndot) {
         return false;
     }
     S->cgloop_p = p;
+    S->cgloop_uni = S->uni;
     return true;
 }
 
@@ -2570,14 +2883,24 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
     MGLevel& L0 = S->lv[0];
     const int cf = fv(S) ? 1 : 0;
     const size_t nc = L0.ncell();
-    // ||b||
-    int nparts = 256;
-    k_sumsq<<<nparts, 256, 0, s>>>(d_b, L0.fluid.p, nc, cf, S->partials.p);
+    int nsm = 148;
+    {
+        int dev = 0;
+        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    }
+    // reductions over the level-0 cells: at most 8 CTAs per SM, two cells per thread and step, grid-stride
+    const unsigned ndot = (unsigned)std::max<size_t>(1, std::min<size_t>({(size_t)nsm * 8, nc / 512 + 1, S->partials.n}));
+    // ||b||, and whether the uniform-coefficient kernels apply to this solve
+    if (S->uni_able) AW_TRY(uniform_check(S, S->d.precision != AW_PRECISION_FP32, s));
+    k_sumsq<<<ndot, 256, 0, s>>>(d_b, L0.fluid.p, nc, cf, S->partials.p, S->ticket.p, S->norm.p);
     AW_LAUNCH();
     double bn;
-    AW_TRY(read_norm(S, nparts, s, &bn));
+    AW_TRY(fetch_norm(S, s, &bn));
     if (!(bn == bn) || std::isinf(bn)) return set_error(AW_ERR_NAN, "right-hand side contains NaN/Inf");
     if (bn == 0.0) bn = 1.0;
+    int general = 0;
+    memcpy(&general, S->h_norm + 1, sizeof general);
+    S->uni = S->uni_able && general == 0;
     const int nlist = L0.ndesc[2];
     int it = 0;
     double rel = 0;
@@ -2586,10 +2909,8 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
         S->x0 = (float*)d_p;
         S->b0 = d_b;
         for (;; ++it) {
-            st = residual_level(S, 0, S->partials.p, s);
-            if (st != AW_OK) break;
             double rn;
-            st = read_norm(S, nlist, s, &rn);
+            st = true_residual(S, (const float*)d_p, nullptr, d_b, L0.r.p, nullptr, s, &rn);
             if (st != AW_OK) break;
             rel = rn / bn;
             if (!(rel == rel)) {
@@ -2601,7 +2922,7 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
                 st = set_error(AW_ERR_NOT_CONVERGED, "relative residual %.3e after %d cycles", rel, it);
                 break;
             }
-            st = run_vcycle(S, s);
+            st = run_vcycle(S, false, s);
             if (st != AW_OK) break;
         }
         S->x0 = nullptr;
@@ -2612,14 +2933,8 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
         // precision).  r lives in the level-0 right-hand side array, the V-cycle's input.
         float* p = (float*)d_p;
         float* sc = S->cg32_sc.p;
-        int nsm = 148;
-        {
-            int dev = 0;
-            if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        }
-        const unsigned ndot = (unsigned)std::min<size_t>((size_t)nsm * 8, S->partials32.n);
-        XStore xp, xd;
-        xp.f = p;
+        const unsigned ndot32 = (unsigned)std::min<size_t>((size_t)nsm * 8, S->partials32.n);
+        XStore xd;
         xd.f = S->cg32_d.p;
         auto launch_err = [&](const char* what) -> aw_status {
             ++g_launches;
@@ -2627,9 +2942,8 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
             return e == cudaSuccess ? AW_OK : set_error(AW_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
         };
         auto read_norm32 = [&](double* out) -> aw_status {
-            k_reduce_sum32<<<1, 256, 0, s>>>(S->partials32.p, (int)ndot, sc + 3);
+            k_reduce_sum32<<<1, 256, 0, s>>>(S->partials32.p, (int)ndot32, sc + 3);
             AW_TRY(launch_err("k_reduce_sum32"));
-            if (!S->h_norm) AW_CUDA(cudaHostAlloc((void**)&S->h_norm, sizeof(double), cudaHostAllocDefault));
             AW_CUDA(cudaMemcpyAsync(S->h_norm, sc + 3, sizeof(float), cudaMemcpyDeviceToHost, s));
             AW_CUDA(cudaStreamSynchronize(s));
             float f;
@@ -2638,14 +2952,11 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
             return AW_OK;
         };
         // r = b - A p into the V-cycle's input; its norm (FP64 partial sums) for the stopping test
-        auto true_residual = [&]() -> aw_status {
-            k_residual<SrcX><<<L0.ndesc[2], 256, L0.smem_smooth, s>>>(SrcX{xp}, d_b, coef(L0), L0.fluid.p, batch(L0, 2),
-                                                                       cf, L0.b.p, nullptr, S->partials.p);
-            return launch_err("k_residual");
+        auto residual32 = [&](double* out) -> aw_status {
+            return true_residual(S, p, nullptr, d_b, L0.b.p, nullptr, s, out);
         };
-        st = L0.ndesc[2] ? true_residual() : AW_OK;
         double rn = 0;
-        if (st == AW_OK) st = read_norm(S, nlist, s, &rn);
+        st = residual32(&rn);
         bool restart = true;
         while (st == AW_OK) {
             rel = rn / bn;
@@ -2655,8 +2966,7 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
             }
             if (rel < S->d.tolerance) {
                 if (restart) break;
-                st = true_residual();
-                if (st == AW_OK) st = read_norm(S, nlist, s, &rn);
+                st = residual32(&rn);
                 restart = true;
                 continue;
             }
@@ -2664,24 +2974,29 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
                 st = set_error(AW_ERR_NOT_CONVERGED, "relative residual %.3e after %d iterations", rel, it);
                 break;
             }
-            st = zero_x(S, 0, s);
-            if (st == AW_OK) st = run_vcycle(S, s);
+            st = run_vcycle(S, true, s);
             if (st != AW_OK) break;
             // the kernels of one iteration as programmatic dependents of one another
-            if ((st = launch_dep(S, k_dot32, ndot, 256, 0, s, L0.b.p, L0.x.p, L0.fluid.p, nc, S->partials32.p)) != AW_OK) break;
-            if ((st = launch_dep(S, k_reduce_sum32, 1, 256, 0, s, S->partials32.p, (int)ndot, sc + 0)) != AW_OK) break;
+            if ((st = launch_dep(S, k_dot32, ndot32, 256, 0, s, L0.b.p, L0.x.p, L0.fluid.p, nc, S->partials32.p)) != AW_OK) break;
+            if ((st = launch_dep(S, k_reduce_sum32, 1, 256, 0, s, S->partials32.p, (int)ndot32, sc + 0)) != AW_OK) break;
             if ((st = launch_dep(S, k_cg_direction32, nblk(nc), 256, 0, s, S->cg32_d.p, L0.x.p, L0.fluid.p, sc,
                                  restart ? 1 : 0, nc)) != AW_OK)
                 break;
-            if ((st = launch_dep(S, k_residual<SrcX>, (unsigned)L0.ndesc[2], 256, L0.smem_smooth, s, SrcX{xd},
-                                 S->cg_zero.p, coef(L0), L0.fluid.p, batch(L0, 2), cf, S->cg32_q.p, (double*)nullptr,
-                                 (double*)nullptr)) != AW_OK)
-                break;
-            if ((st = launch_dep(S, k_dot32, ndot, 256, 0, s, S->cg32_d.p, S->cg32_q.p, L0.fluid.p, nc,
+            if (S->uni) {
+                UOut out{};
+                out.r = S->cg32_q.p;
+                st = uni_residual(S, 0, xd, nullptr, out, nullptr, s);
+            } else {
+                st = launch_dep(S, k_residual<SrcX>, (unsigned)nlist, 256, L0.smem_smooth, s, SrcX{xd}, S->cg_zero.p,
+                                coef(L0), L0.fluid.p, batch(L0, 2), cf, S->cg32_q.p, (double*)nullptr,
+                                (double*)nullptr);
+            }
+            if (st != AW_OK) break;
+            if ((st = launch_dep(S, k_dot32, ndot32, 256, 0, s, S->cg32_d.p, S->cg32_q.p, L0.fluid.p, nc,
                                  S->partials32.p)) != AW_OK)
                 break;
-            if ((st = launch_dep(S, k_reduce_sum32, 1, 256, 0, s, S->partials32.p, (int)ndot, sc + 2)) != AW_OK) break;
-            if ((st = launch_dep(S, k_cg_update32, ndot, 256, 0, s, p, L0.b.p, S->cg32_d.p, S->cg32_q.p, sc, L0.fluid.p,
+            if ((st = launch_dep(S, k_reduce_sum32, 1, 256, 0, s, S->partials32.p, (int)ndot32, sc + 2)) != AW_OK) break;
+            if ((st = launch_dep(S, k_cg_update32, ndot32, 256, 0, s, p, L0.b.p, S->cg32_d.p, S->cg32_q.p, sc, L0.fluid.p,
                                  nc, S->partials32.p)) != AW_OK)
                 break;
             if ((st = launch_dep(S, k_copy_scalar32, 1, 1, 0, s, sc, 1, 0)) != AW_OK) break;
@@ -2697,28 +3012,13 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
         // cycle converges on every configuration.  The iterations run in a device-side loop
         // (cg_devloop_build) when the device can build it, else with one host read (||r||) each.
         double* p = (double*)d_p;
-        double* sc = S->cg_sc.p;
-        // reductions over the level-0 cells: 8 CTAs per SM, grid-stride
-        int nsm = 148;
-        {
-            int dev = 0;
-            if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        }
-        const unsigned ndot = (unsigned)std::min<size_t>((size_t)nsm * 8, S->partials.n);
-        auto launch_err = [&](const char* what) -> aw_status {
-            ++g_launches;
-            cudaError_t e = cudaGetLastError();
-            return e == cudaSuccess ? AW_OK : set_error(AW_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+        auto residual64 = [&](double* out) -> aw_status {
+            return true_residual(S, nullptr, p, d_b, L0.b.p, S->cg_r.p, s, out);
         };
-        auto true_residual = [&]() -> aw_status {
-            k_residual<SrcD><<<L0.ndesc[2], 256, L0.smem_x64, s>>>(SrcD{p}, d_b, coef(L0), L0.fluid.p, batch(L0, 2), cf,
-                                                                    L0.b.p, S->cg_r.p, S->partials.p);
-            return launch_err("k_residual64");
-        };
-        st = true_residual();
         double rn = 0;
-        if (st == AW_OK) st = read_norm(S, nlist, s, &rn);
+        st = residual64(&rn);
         bool restart = true;
+        if (!S->h_cg) AW_CUDA(cudaHostAlloc((void**)&S->h_cg, 4 * sizeof(double), cudaHostAllocDefault));
         while (st == AW_OK) {
             rel = rn / bn;
             if (!(rel == rel)) {
@@ -2728,8 +3028,7 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
             if (rel < S->d.tolerance) {
                 if (restart) break;  // rn is a true residual
                 // confirm with the true FP64 residual (the recursive one can drift)
-                st = true_residual();
-                if (st == AW_OK) st = read_norm(S, nlist, s, &rn);
+                st = residual64(&rn);
                 restart = true;
                 continue;
             }
@@ -2737,18 +3036,22 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
                 st = set_error(AW_ERR_NOT_CONVERGED, "relative residual %.3e after %d iterations", rel, it);
                 break;
             }
-            if (S->use_graph && S->use_devloop && S->cgloop_p != (const void*)p && !cg_devloop_build(S, p, ndot))
+            if (S->use_graph && S->use_devloop && (S->cgloop_p != (const void*)p || S->cgloop_uni != S->uni) &&
+                !cg_devloop_build(S, p, ndot))
                 S->use_devloop = false;  // no such graph on this device: the host loop below
-            if (S->use_graph && S->use_devloop) {
-                // iterations on the device until the recursive residual converges, turns NaN or the
-                // limit is reached; then one read-back of ||r||^2 and the iteration count
-                const int st0[4] = {it, restart ? 1 : 0, S->d.max_cycles, 0};
+            if (restart) {
+                // {iterations, restart flag, limit} and {||b||, tolerance}, kept on the device by the iterations
+                const int st0[4] = {it, 1, S->d.max_cycles, 0};
                 const double prm[2] = {bn, S->d.tolerance};
-                if (!S->h_cg) AW_CUDA(cudaHostAlloc((void**)&S->h_cg, 4 * sizeof(double), cudaHostAllocDefault));
                 memcpy(S->h_cg, st0, sizeof st0);
                 memcpy(S->h_cg + 2, prm, sizeof prm);
                 AW_CUDA(cudaMemcpyAsync(S->cgst.p, S->h_cg, sizeof st0, cudaMemcpyHostToDevice, s));
                 AW_CUDA(cudaMemcpyAsync(S->cgprm.p, S->h_cg + 2, sizeof prm, cudaMemcpyHostToDevice, s));
+                restart = false;
+            }
+            if (S->use_graph && S->use_devloop) {
+                // iterations on the device until the recursive residual converges, turns NaN or the
+                // limit is reached; then one read-back of ||r||^2 and the iteration count
                 AW_CUDA(cudaGraphLaunch(S->cgloop, s));
                 AW_CUDA(cudaMemcpyAsync(S->h_cg, S->norm.p, sizeof(double), cudaMemcpyDeviceToHost, s));
                 AW_CUDA(cudaMemcpyAsync(S->h_cg + 1, S->cgst.p, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -2758,35 +3061,11 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
                 g_launches += S->cgloop_kernels * (unsigned long long)(it1 - it);
                 it = it1;
                 rn = std::sqrt(S->h_cg[0]);
-                restart = false;
                 continue;
             }
-            // z = V(r): one V-cycle on the FP32 copy of r (in L0.b), from zero
-            st = zero_x(S, 0, s);
-            if (st == AW_OK) st = run_vcycle(S, s);
-            if (st != AW_OK) break;
-            // rho = r . z ; d = z + (rho / rho_old) d
-            // the kernels of one iteration as programmatic dependents of one another
-            if ((st = launch_dep(S, k_dot64, ndot, 256, 0, s, S->cg_r.p, (const double*)nullptr, L0.x.p, L0.fluid.p, nc,
-                                 S->partials.p)) != AW_OK)
-                break;
-            if ((st = launch_dep(S, k_reduce_sum, 1, 256, 0, s, S->partials.p, (int)ndot, sc + 0)) != AW_OK) break;
-            if ((st = launch_dep(S, k_cg_direction, nblk(nc), 256, 0, s, S->cg_d.p, L0.x.p, L0.fluid.p, sc,
-                                 restart ? 1 : 0, (const int*)nullptr, nc)) != AW_OK)
-                break;
-            // qn = -A d ; sc[2] = d . qn
-            if ((st = launch_dep(S, k_apply_dot, (unsigned)L0.ndesc[2], 256, L0.smem_x64, s, SrcD{S->cg_d.p},
-                                 S->cg_zero.p, coef(L0), L0.fluid.p, batch(L0, 2), cf, S->cg_q.p, S->partials.p)) !=
-                AW_OK)
-                break;
-            if ((st = launch_dep(S, k_reduce_sum, 1, 256, 0, s, S->partials.p, L0.ndesc[2], sc + 2)) != AW_OK) break;
-            // p += alpha d ; r -= alpha A d ; FP32 copy of r for the next V-cycle ; rho_old = rho
-            if ((st = launch_dep(S, k_cg_update, ndot, 256, 0, s, p, S->cg_r.p, L0.b.p, S->cg_d.p, S->cg_q.p, sc,
-                                 L0.fluid.p, nc, S->partials.p)) != AW_OK)
-                break;
+            st = cg_iteration(S, p, ndot, s, nullptr);
             ++it;
-            restart = false;
-            st = read_norm(S, ndot, s, &rn);  // ||r|| from k_cg_update's partial sums
+            if (st == AW_OK) st = fetch_norm(S, s, &rn);  // ||r|| from k_cg_update
         }
     }
     if (cycles) *cycles = it;

@@ -27,7 +27,8 @@ def needs_build() -> bool:
     if not os.path.exists(OUT):
         return True
     t = os.path.getmtime(OUT)
-    deps = sources() + [os.path.join(HERE, "aw_internal.cuh"), os.path.join(ROOT, "include", "anitowave.h")]
+    deps = sources() + [os.path.join(HERE, "aw_internal.cuh"), os.path.join(HERE, "aw_uniform.cuh"),
+                        os.path.join(ROOT, "include", "anitowave.h")]
     return any(os.path.getmtime(d) > t for d in deps)
 
 
