@@ -43,11 +43,13 @@ struct MGLevel {
     std::vector<int> h_res;
     DBuf<uint32_t> off[4];
     uint32_t tot[4] = {0, 0, 0, 0};
-    // CTA batches: [0]/[1] blocks of one colour, [2] all blocks; each entry {first, count, res, 0}
-    DBuf<int4> desc[3];
-    std::vector<int> h_blocks[3];  // block of every slot, batch order
-    DBuf<int> meta[3];             // slot metadata (NMETA fields x slots, field-major)
-    DBuf<int> blk[3];              // block of every slot, batch order, on the device
+    // CTA batches: [0]/[1] blocks of one colour, [2] all blocks; each entry {first, count, res, 0}, the
+    // block of every slot and the slot metadata (NMETA fields x slots, field-major), in one allocation
+    DBuf<int4> batches;
+    int4* desc[3] = {};
+    int* blk[3] = {};
+    int* meta[3] = {};
+    int nslots[3] = {0, 0, 0};
     int ndesc[3] = {0, 0, 0};
     // dynamic shared memory of the batched kernels on this level
     size_t smem_smooth = 0, smem_x64 = 0, smem_prolong = 0, smem_meta = 0;
@@ -1065,7 +1067,7 @@ __device__ inline float dense_Ax(const DenseArgs& A, const float* x, int i, int 
 }
 
 // Per-cell values of the uniform-level kernels (the caller stores them), shared by the
-// one-launch-per-step kernels below and by k_dense_tail, so both forms do the same arithmetic in
+// one-launch-per-step kernels below; k_dense_tail does the same arithmetic in
 // the same order.  Each returns false where the kernel leaves the cell unchanged.
 __device__ inline bool dense_smooth_value(const DenseArgs& A, const float* x, const float* __restrict__ b, int t,
                                           int col, float omega, float* out) {
@@ -1501,159 +1503,420 @@ __global__ void __launch_bounds__(512) k_coarse_factor(Uniform U, int* pos_of, i
     if (threadIdx.x == 0) ex_n[0] = n;
 }
 
-// x = Minv b on the fluid cells of the coarsest level (FP64 accumulation)
-// row i of x = Minv b over the n fluid cells of the coarsest level
-__device__ inline void coarse_apply_row(const Uniform& U, const int* __restrict__ idx, int n,
-                                        const double* __restrict__ Minv, const float* b, float* x, int i) {
-    double s = 0.0;
-    for (int j = 0; j < n; ++j) s += Minv[(size_t)i * n + j] * (double)b[uni_cell(U, idx[j])];
-    x[uni_cell(U, idx[i])] = (float)s;
-}
-__global__ void k_coarse_apply(Uniform U, const int* __restrict__ idx, const int* __restrict__ ex_n,
-                               const double* __restrict__ Minv, const float* __restrict__ b, float* __restrict__ x) {
+// x = Minv b on the fluid cells of the coarsest level (FP64 accumulation), a warp per row (a thread per
+// row walked 512 uncoalesced values one after the other)
+__global__ void __launch_bounds__(256) k_coarse_apply(Uniform U, const int* __restrict__ idx, const int* __restrict__ ex_n,
+                                                      const double* __restrict__ Minv, const float* __restrict__ b,
+                                                      float* __restrict__ x) {
     pdl_wait();
-    const int n = ex_n[0];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        coarse_apply_row(U, idx, n, Minv, b, x, i);
+    const int n = ex_n[0], lane = threadIdx.x & 31;
+    for (int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < n; i += (int)(gridDim.x * blockDim.x) >> 5) {
+        double s = 0.0;
+        for (int j = lane; j < n; j += 32) s += Minv[(size_t)i * n + j] * (double)b[uni_cell(U, idx[j])];
+        s = warp_sum(s);
+        if (lane == 0) x[uni_cell(U, idx[i])] = (float)s;
+    }
 }
 
-// The uniform tail of an FV V-cycle in one CTA: the restriction from the level above the tail (the
-// last MSBG level, one cell per block, or a larger uniform level) into the first tail level, the
-// V-cycle over the tail levels down to the coarsest solve and back, and the prolongation into the
-// level above.  Tail levels hold at most TAIL_MAX_CELLS cells, so as separate launches (about 14 on
-// a 512/64-cell tail) each step costs a launch's latency rather than its work; here the steps are
-// separated by CTA barriers instead.  (A 4096-cell level measured slower in one CTA than as
-// launches, so larger uniform levels keep their own launches.)
-// Every step applies the per-cell value functions of the separate kernels in the same order, so the
-// results are bit-identical to the launch-per-step form.  The CTA reads and writes the levels in
-// global memory; __syncthreads orders one step's writes before the next step's reads.  Within a
-// step a thread computes the values of up to TAIL_K cells before it stores any of them, so their
-// loads are in flight together (a store between them could alias the next cell's loads).
-constexpr int TAIL_THREADS = 1024;
-constexpr int TAIL_K = 4;             // cells per thread whose loads are issued together
-constexpr int TAIL_MAX = 4;           // uniform levels the fused tail handles
-constexpr int TAIL_MAX_CELLS = 512;   // largest uniform level it handles
-struct TailLevel {
-    DenseArgs A;
-    float* x;
-    float* b;
-    float* r;
-};
+// The tail of an FV V-cycle in one CTA: from the first level of at most TAIL_TOP cells on a uniform
+// lattice (the last MSBG level, one cell per block, or a uniform level) down to the coarsest solve and
+// back up, from a zero guess.  As separate launches each of these steps costs a launch's latency rather
+// than its work; here a step is a shared-memory pass and a barrier.
+// - The top level's weights, right-hand side, flags and x sit in registers.  Its x extent is even, so its
+//   cells split into x pairs of one cell of each colour: a thread owns 4 pairs and every lane works in
+//   every colour pass.  The cells of a colour have a shared-memory array of their own for the neighbours'
+//   reads (without bank conflicts), with a layer of ghost zeros around it (no neighbour tests).
+// - The levels below (at most 512 cells, one per thread) sit in shared memory and are walked by just
+//   enough warps, on a barrier of their own.
+// - Weights, flags and the inverse of the coarsest operator are fixed during a solve, so they are read
+//   before the wait for the preceding kernel, every load of a step issued before the first is used.
+// Every cell's arithmetic is that of the separate kernels in the same order, so the results are
+// bit-identical to the launch-per-step form up to the coarsest solve, whose FP64 row sums are taken by a
+// warp.  What bounds it is instruction issue and barrier latency of one SM.
+constexpr int TAIL_THREADS = 512;
+constexpr int TAIL_TOP = 4096;        // cells of the top level
+constexpr int TAIL_PAIRS = TAIL_TOP / (2 * TAIL_THREADS);
+constexpr int TAIL_MAX = 4;           // uniform levels below the top
+constexpr int TAIL_MAX_CELLS = 512;   // cells of each of them
+constexpr int TAIL_INV = 64;          // inverses up to this size are kept in shared memory
 struct DenseTail {
-    TailLevel lv[TAIL_MAX];
-    int n;                    // uniform levels, lv[n - 1] the coarsest
-    int from_msbg;            // the level above is the last MSBG level (F), else a uniform level (Fd)
+    DenseArgs top;            // lattice, weights and fluid flags of a uniform top level
+    int from_msbg;            // the top is the one-cell MSBG level F (lattice in top.d)
     LevelView F;
-    DenseView Fd;
-    const float* rf;          // its residual
-    float* xf;                // its x (FP32)
-    const uint8_t* fluid_f;   // its fluid flags
+    float* x;
+    const float* b;
+    DenseArgs lv[TAIL_MAX];   // uniform levels below, lv[n - 1] the coarsest
+    int low[TAIL_MAX];        // their places in shared memory, in floats behind the top's arrays
+    int n;
+    int pre, post, local;     // smoothing of the top: sweeps, updates of a cell per colour (MSBG)
     int sweeps, coarsest_iters, exact;
     float omega;
-    Uniform U;                // exact coarsest solve
     const int* idx;
     const int* ex_n;
     const double* Minv;
 };
-__device__ inline int tail_cells(const TailLevel& L) { return L.A.d.D[0] * L.A.d.D[1] * L.A.d.D[2]; }
-// One step over n items: value(t, &at, &v) says whether item t writes v at index at; then store.
-template <class V, class S>
-__device__ __forceinline__ void tail_step(int n, V value, S store) {
-    for (int t0 = threadIdx.x; t0 < n; t0 += TAIL_K * blockDim.x) {
-        float v[TAIL_K];
-        uint32_t at[TAIL_K];
-        bool w[TAIL_K];
-#pragma unroll
-        for (int k = 0; k < TAIL_K; ++k) {
-            const int t = t0 + k * (int)blockDim.x;
-            w[k] = t < n && value(t, &at[k], &v[k]);
-        }
-#pragma unroll
-        for (int k = 0; k < TAIL_K; ++k)
-            if (w[k]) store(at[k], v[k]);
-    }
-    __syncthreads();
+__host__ __device__ inline int lattice_cells(const DenseView& d) { return d.D[0] * d.D[1] * d.D[2]; }
+__host__ __device__ inline int lattice_padded(const DenseView& d) { return (d.D[0] + 2) * (d.D[1] + 2) * (d.D[2] + 2); }
+// the pairs of a lattice of even x extent, one value per pair
+__host__ __device__ inline DenseView lattice_pairs(const DenseView& d) { return DenseView{{d.D[0] / 2, d.D[1], d.D[2]}}; }
+// padded index of a cell
+__host__ __device__ inline int pad_index(const DenseView& d, int i, int j, int k) {
+    return (i + 1) + (d.D[0] + 2) * ((j + 1) + (d.D[1] + 2) * (k + 1));
 }
-__device__ inline void tail_smooth(const TailLevel& L, int iters, int rev, float omega) {
-    const int n = tail_cells(L);
+// shared memory: inverse, indices of the coarsest system, padded x of both colours and r of the top, then
+// per level below
+// padded x | b | r | six weights | fluid | two packed index words per cell (TAIL_CELL_WORDS)
+constexpr int TAIL_CELL_WORDS = 11;
+inline size_t tail_layout(DenseTail& T) {  // fills T.low, returns the bytes
+    int f = 0;
+    for (int l = 0; l < T.n; ++l) {
+        T.low[l] = f;
+        f += lattice_padded(T.lv[l].d) + TAIL_CELL_WORDS * lattice_cells(T.lv[l].d);
+    }
+    return ((size_t)f + 2 * lattice_padded(lattice_pairs(T.top.d)) + lattice_cells(T.top.d) + TAIL_MAX_CELLS) * sizeof(float) +
+           (size_t)TAIL_INV * TAIL_INV * sizeof(double);
+}
+// A x at a cell, with the roundings of the separate kernels: the residual of the MSBG level starts with
+// the diagonal, its smoother and the uniform levels end with it.  w, v: W, E, S, N, B, T
+__device__ __forceinline__ float tail_sum(const float* w, const float* v, float a) {
+    a = ufma(w[2], v[2], a);
+    a = ufma(w[3], v[3], a);
+    a = ufma(w[4], v[4], a);
+    return ufma(w[5], v[5], a);
+}
+__device__ __forceinline__ float tail_uniform(const float* w, const float* v) {
+    return tail_sum(w, v, ufma(w[1], v[1], umul(w[0], v[0])));
+}
+__device__ __forceinline__ float tail_block(const float* w, const float* v) {
+    return tail_sum(w, v, ufma(w[0], v[0], umul(w[1], v[1])));
+}
+__device__ __forceinline__ float tail_block_resid(const float* w, const float* v, float diag, float x) {
+    return tail_sum(w, v, ufma(w[1], v[1], ufma(w[0], v[0], umul(diag, x))));
+}
+__device__ __forceinline__ float tail_diag(const float* w) { return -(w[0] + w[1] + w[2] + w[3] + w[4] + w[5]); }
+__device__ __forceinline__ void tail_nb(const float* x, int sy, int sz, float v[6]) {
+    v[0] = x[-1];
+    v[1] = x[1];
+    v[2] = x[-sy];
+    v[3] = x[sy];
+    v[4] = x[-sz];
+    v[5] = x[sz];
+}
+__device__ __forceinline__ void tail_bar(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
+
+// this thread's cell of a level below the top
+struct TailLow {
+    float *x, *b, *r;     // x: the level's padded lattice; b, r: unpadded
+    float* own;           // this cell in x
+    float w[6], diag, rcp;
+    int n, sy, sz, parent, child;  // parent: in the next level's padded x; child: its first child in r of the level above
+    bool mine, fluid;
+    int col;
+};
+__device__ __forceinline__ TailLow tail_low(const DenseTail& T, float* low, int l) {
+    TailLow L;
+    const DenseView& d = T.lv[l].d;
+    float* f = low + T.low[l];
+    L.n = lattice_cells(d);
+    L.sy = d.D[0] + 2;
+    L.sz = L.sy * (d.D[1] + 2);
+    L.x = f;
+    f += lattice_padded(d);
+    L.b = f;
+    L.r = f + L.n;
+    const int t = threadIdx.x;
+    L.mine = t < L.n;
+    const int at = L.mine ? t : 0;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) L.w[k] = f[(2 + k) * L.n + at];
+    L.fluid = L.mine && f[8 * L.n + at] != 0.f;
+    const int p0 = __float_as_int(f[9 * L.n + at]);
+    L.child = __float_as_int(f[10 * L.n + at]);
+    L.own = L.x + (p0 & 0x7FFF);
+    L.col = (p0 >> 15) & 1;
+    L.parent = p0 >> 16;
+    L.diag = tail_diag(L.w);
+    L.rcp = urcp(L.diag);
+    return L;
+}
+__device__ __forceinline__ void tail_low_smooth(const TailLow& L, int iters, int rev, float omega, int threads) {
+    const bool on = L.fluid && !(fabsf(L.diag) < 1e-30f);
+    const float b = L.b[L.mine ? threadIdx.x : 0];
     for (int it = 0; it < iters; ++it)
         for (int k = 0; k < 2; ++k) {
-            const int col = rev ? 1 - k : k;
-            tail_step(
-                n,
-                [&](int t, uint32_t* at, float* v) {
-                    *at = (uint32_t)t;
-                    return dense_smooth_value(L.A, L.x, L.b, t, col, omega, v);
-                },
-                [&](uint32_t at, float v) { L.x[at] = v; });
+            if (on && L.col == (rev ? 1 - k : k)) {
+                float v[6];
+                tail_nb(L.own, L.sy, L.sz, v);
+                const float x = *L.own;
+                *L.own = ufma(omega, umul(b - ufma(L.diag, x, tail_uniform(L.w, v)), L.rcp), x);
+            }
+            tail_bar(threads);
         }
 }
-__global__ void __launch_bounds__(TAIL_THREADS) k_dense_tail(DenseTail T) {
-    pdl_wait();
-    {  // restriction from the level above; the first tail level's x starts at zero
-        const TailLevel& C = T.lv[0];
-        tail_step(
-            tail_cells(C),
-            [&](int t, uint32_t* at, float* v) {
-                *at = (uint32_t)t;
-                *v = dense_restrict_value(C.A.d, C.A.fluid, T.from_msbg, T.F, T.Fd, T.rf, t);
-                return true;
-            },
-            [&](uint32_t at, float v) {
-                C.b[at] = v;
-                C.x[at] = 0.f;
-            });
+// sum of the 8 fine values under a coarse cell (children in x, y, z order)
+__device__ __forceinline__ float tail_restrict(const float* r, const DenseView& f) {
+    const int sy = f.D[0], sz = f.D[0] * f.D[1];
+    float s = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s += r[(e & 1) + ((e >> 1) & 1) * sy + (e >> 2) * sz];
+    return s;
+}
+__global__ void __launch_bounds__(TAIL_THREADS, 1) k_dense_tail(const __grid_constant__ DenseTail T) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int tid = threadIdx.x;
+    const DenseView& d0 = T.top.d;
+    const DenseView dp = lattice_pairs(d0);
+    const int n0 = lattice_cells(d0), np0 = lattice_padded(dp);
+    const int sy0 = dp.D[0] + 2, sz0 = sy0 * (d0.D[1] + 2);
+    double* inv = reinterpret_cast<double*>(smraw);
+    int* idx = reinterpret_cast<int*>(inv + TAIL_INV * TAIL_INV);
+    float* xs = reinterpret_cast<float*>(idx + TAIL_MAX_CELLS);
+    float* rs = xs + 2 * np0;
+    float* low = rs + n0;
+    // ---- fixed data, before the wait
+    const int nex = T.exact ? T.ex_n[0] : 0;
+    // top level: pair p = tid + i * TAIL_THREADS is the cells 2 p, 2 p + 1; slot 2 i + c its cell of colour c
+    float w[2 * TAIL_PAIRS][6], diag[2 * TAIL_PAIRS], rcp[2 * TAIL_PAIRS], b[2 * TAIL_PAIRS];
+    float x[2 * TAIL_PAIRS];
+    int cell[TAIL_PAIRS], odd[TAIL_PAIRS], parent[TAIL_PAIRS];  // padded index of the pair; colour of its first cell
+    uint32_t at[2 * TAIL_PAIRS], act = 0, fl = 0;               // cell offsets; bit masks over the slots
+    {
+        int2 res[TAIL_PAIRS];
+        uint2 oc[TAIL_PAIRS], of[TAIL_PAIRS][3];
+        const int hx = d0.D[0] >> 1;
+#pragma unroll
+        for (int i = 0; i < TAIL_PAIRS; ++i) {
+            const int pr = tid + i * TAIL_THREADS;
+            const bool in = 2 * pr < n0;
+            const int p = in ? pr : 0;
+            const int x2 = p % hx, yz = p / hx, y = yz % d0.D[1], z = yz / d0.D[1];
+            cell[i] = pad_index(dp, x2, y, z);
+            odd[i] = (y + z) & 1;
+            parent[i] = T.n ? pad_index(T.lv[0].d, x2, y >> 1, z >> 1) : 0;
+            res[i] = make_int2(in, in);
+            oc[i] = make_uint2(2 * p, 2 * p + 1);
+            if (T.from_msbg) {
+                const int2 r = reinterpret_cast<const int2*>(T.F.res)[p];
+                res[i] = make_int2(in && r.x, in && r.y);
+                oc[i] = reinterpret_cast<const uint2*>(T.F.off[0])[p];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) of[i][a] = reinterpret_cast<const uint2*>(T.F.off[1 + a])[p];
+            } else {
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    of[i][a].x = dfidx(d0, a, 2 * x2, y, z);
+                    of[i][a].y = of[i][a].x + 1;
+                }
+            }
+        }
+        float lo[TAIL_PAIRS][2][3], hi[TAIL_PAIRS][2][3];
+#pragma unroll
+        for (int i = 0; i < TAIL_PAIRS; ++i) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                // an inactive block owns no face: its offset may lie at the array's end
+                const uint32_t f0 = res[i].x ? of[i][a].x : 0, f1 = res[i].y ? of[i][a].y : 0;
+                const uint32_t up = T.from_msbg || a == 0 ? 1u : (a == 1 ? (uint32_t)d0.D[0] : (uint32_t)(d0.D[0] * d0.D[1]));
+                if (T.from_msbg && f1 == f0 + 2 && (f0 & 3u) == 0) {  // both blocks' two faces: 16 bytes
+                    const float4 v = *reinterpret_cast<const float4*>(T.top.W[a] + f0);
+                    lo[i][0][a] = v.x;
+                    hi[i][0][a] = v.y;
+                    lo[i][1][a] = v.z;
+                    hi[i][1][a] = v.w;
+                } else {
+                    lo[i][0][a] = T.top.W[a][f0];
+                    hi[i][0][a] = T.top.W[a][f0 + up];
+                    lo[i][1][a] = T.top.W[a][f1];
+                    hi[i][1][a] = T.top.W[a][f1 + up];
+                }
+            }
+        }
+        bool f[TAIL_PAIRS][2];
+#pragma unroll
+        for (int i = 0; i < TAIL_PAIRS; ++i) {
+            if (!res[i].x) oc[i].x = 0;
+            if (!res[i].y) oc[i].y = 0;
+            f[i][0] = T.top.fluid[oc[i].x] != 0;
+            f[i][1] = T.top.fluid[oc[i].y] != 0;
+        }
+#pragma unroll
+        for (int i = 0; i < TAIL_PAIRS; ++i)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const int j = 2 * i + c;
+                const bool second = (odd[i] ^ c) != 0;  // the pair's cell of colour c
+                at[j] = second ? oc[i].y : oc[i].x;
+                const bool on = second ? res[i].y : res[i].x;
+                act |= (on ? 1u : 0u) << j;
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    w[j][2 * a] = second ? lo[i][1][a] : lo[i][0][a];
+                    w[j][2 * a + 1] = second ? hi[i][1][a] : hi[i][0][a];
+                }
+                diag[j] = tail_diag(w[j]);
+                rcp[j] = urcp(diag[j]);
+                const bool fluid = second ? f[i][1] : f[i][0];
+                if (on && fluid) fl |= 1u << j;
+            }
     }
-    for (int m = 0; m + 1 < T.n; ++m) {
-        const TailLevel& L = T.lv[m];
-        const TailLevel& K = T.lv[m + 1];
-        tail_smooth(L, T.sweeps, 0, T.omega);
-        tail_step(
-            tail_cells(L),
-            [&](int t, uint32_t* at, float* v) {
-                *at = (uint32_t)t;
-                *v = dense_residual_value(L.A, L.x, L.b, t);
-                return true;
-            },
-            [&](uint32_t at, float v) { L.r[at] = v; });
-        tail_step(
-            tail_cells(K),
-            [&](int t, uint32_t* at, float* v) {
-                *at = (uint32_t)t;
-                *v = dense_restrict_value(K.A.d, K.A.fluid, 0, T.F, L.A.d, L.r, t);
-                return true;
-            },
-            [&](uint32_t at, float v) {
-                K.b[at] = v;
-                K.x[at] = 0.f;
-            });
-    }
-    const TailLevel& C = T.lv[T.n - 1];
+    // update mask: fluid cells that are not cut off from every neighbour
+    uint32_t upd = 0;
+#pragma unroll
+    for (int j = 0; j < 2 * TAIL_PAIRS; ++j)
+        if (((fl >> j) & 1u) && !(fabsf(diag[j]) < (T.from_msbg ? 1e-9f : 1e-30f))) upd |= 1u << j;
     if (T.exact) {
-        const int n = T.ex_n[0];
-        for (int i = threadIdx.x; i < n; i += blockDim.x) coarse_apply_row(T.U, T.idx, n, T.Minv, C.b, C.x, i);
+        for (int i = tid; i < nex; i += TAIL_THREADS) idx[i] = T.idx[i];
+        if (nex <= TAIL_INV)
+            for (int i = tid; i < nex * nex; i += TAIL_THREADS) inv[i] = T.Minv[i];
+    }
+    for (int l = 0; l < T.n; ++l) {
+        const DenseArgs& A = T.lv[l];
+        const DenseView& d = A.d;
+        const int n = lattice_cells(d), np = lattice_padded(d);
+        float* f = low + T.low[l];
+        for (int i = tid; i < np; i += TAIL_THREADS) f[i] = 0.f;
+        f += np;
+        if (tid >= n) continue;
+        const int q0 = tid % d.D[0], q1 = (tid / d.D[0]) % d.D[1], q2 = tid / (d.D[0] * d.D[1]);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            f[(2 + 2 * a) * n + tid] = A.W[a][dfidx(d, a, q0, q1, q2)];
+            f[(3 + 2 * a) * n + tid] = A.W[a][dfidx(d, a, q0 + (a == 0), q1 + (a == 1), q2 + (a == 2))];
+        }
+        f[8 * n + tid] = A.fluid[tid] ? 1.f : 0.f;
+        const int par = l + 1 < T.n ? pad_index(T.lv[l + 1].d, q0 >> 1, q1 >> 1, q2 >> 1) : 0;
+        f[9 * n + tid] = __int_as_float(pad_index(d, q0, q1, q2) | ((q0 + q1 + q2) & 1) << 15 | par << 16);
+        const DenseView& u = l ? T.lv[l - 1].d : d0;
+        f[10 * n + tid] = __int_as_float(2 * q0 + u.D[0] * (2 * q1 + u.D[1] * 2 * q2));
+    }
+    for (int t = tid; t < 2 * np0 + n0; t += TAIL_THREADS) xs[t] = 0.f;  // x and r
+    pdl_wait();
+#pragma unroll
+    for (int j = 0; j < 2 * TAIL_PAIRS; ++j) {
+        b[j] = T.b[at[j]];
+        x[j] = 0.f;
+    }
+    __syncthreads();
+    // neighbours of slot 2 i + c: the partner on one x side, the next pair's cell on the other
+    auto neighbours = [&](int i, int c, float v[6]) {
+        const bool second = (odd[i] ^ c) != 0;
+        const float* o = xs + (1 - c) * np0 + cell[i];
+        const float outer = o[second ? 1 : -1], partner = x[2 * i + (1 - c)];
+        v[0] = second ? partner : outer;
+        v[1] = second ? outer : partner;
+        v[2] = o[-sy0];
+        v[3] = o[sy0];
+        v[4] = o[-sz0];
+        v[5] = o[sz0];
+    };
+    const bool msbg = T.from_msbg != 0;
+    const int local = msbg ? T.local : 1;
+    auto pass = [&](int c) {
+        float v[TAIL_PAIRS][6];
+#pragma unroll
+        for (int i = 0; i < TAIL_PAIRS; ++i) neighbours(i, c, v[i]);
+        // (a uniform cell differs in the order of its x products and in being updated once)
+        float y[TAIL_PAIRS], a[TAIL_PAIRS];
+#pragma unroll
+        for (int i = 0; i < TAIL_PAIRS; ++i) {
+            const int j = 2 * i + c;
+            y[i] = x[j];
+            a[i] = msbg ? tail_block(w[j], v[i]) : tail_uniform(w[j], v[i]);
+        }
+        for (int u = 0; u < local; ++u)
+#pragma unroll
+            for (int i = 0; i < TAIL_PAIRS; ++i) {
+                const int j = 2 * i + c;
+                y[i] = ufma(T.omega, umul(b[j] - ufma(diag[j], y[i], a[i]), rcp[j]), y[i]);
+            }
+#pragma unroll
+        for (int i = 0; i < TAIL_PAIRS; ++i)
+            if ((upd >> (2 * i + c)) & 1u) {
+                x[2 * i + c] = y[i];
+                xs[c * np0 + cell[i]] = y[i];
+            }
         __syncthreads();
-    } else {
-        tail_smooth(C, T.coarsest_iters, 0, T.omega);
+    };
+    // one loop over the passes, so that each colour's code exists (and is fetched) once: red, black, ...
+    // before the coarse-grid correction, black, red, ... after it
+    const int npre = 2 * T.pre, npass = npre + 2 * T.post;
+#pragma unroll 1
+    for (int step = 0;; ++step) {
+        if (step == npre) {
+#pragma unroll
+    for (int j = 0; j < 2 * TAIL_PAIRS; ++j) {
+        if (!((fl >> j) & 1u)) continue;
+        const int i = j >> 1;
+        float v[6];
+        neighbours(i, j & 1, v);
+        rs[2 * (tid + i * TAIL_THREADS) + (odd[i] ^ (j & 1))] =
+            b[j] - (T.from_msbg ? tail_block_resid(w[j], v, diag[j], x[j]) : ufma(diag[j], x[j], tail_uniform(w[j], v)));
     }
-    for (int m = T.n - 2; m >= 0; --m) {
-        const TailLevel& L = T.lv[m];
-        const TailLevel& K = T.lv[m + 1];
-        tail_step(
-            tail_cells(L),
-            [&](int t, uint32_t* at, float* v) {
-                return dense_prolong_value(K.A.d, K.x, 0, T.F, nullptr, L.A.d, L.x, L.A.fluid, t, at, v);
-            },
-            [&](uint32_t at, float v) { L.x[at] = v; });
-        tail_smooth(L, T.sweeps, 1, T.omega);
+    __syncthreads();
+    // ---- the levels below, by the warps that cover the first of them
+    const int nt = (lattice_cells(T.lv[0].d) + 31) & ~31;
+    if (tid < nt) {
+#pragma unroll 1
+        for (int l = 0; l < T.n; ++l) {
+            const TailLow L = tail_low(T, low, l);
+            if (L.mine) {
+                const float* r = l == 0 ? rs : low + T.low[l - 1] + lattice_padded(T.lv[l - 1].d) + lattice_cells(T.lv[l - 1].d);
+                const float s = tail_restrict(r + L.child, l == 0 ? d0 : T.lv[l - 1].d);
+                L.b[tid] = L.fluid ? s : 0.f;
+            }
+            tail_bar(nt);
+            if (l + 1 == T.n) break;
+            tail_low_smooth(L, T.sweeps, 0, T.omega, nt);
+            if (L.mine) {
+                float v[6];
+                tail_nb(L.own, L.sy, L.sz, v);
+                L.r[tid] = L.fluid ? L.b[tid] - ufma(L.diag, *L.own, tail_uniform(L.w, v)) : 0.f;
+            }
+            tail_bar(nt);
+        }
+#pragma unroll 1
+        for (int l = T.n - 1; l >= 0; --l) {
+            const TailLow L = tail_low(T, low, l);
+            if (l + 1 == T.n) {  // the coarsest
+                if (T.exact) {
+                    const double* M = nex <= TAIL_INV ? inv : T.Minv;
+                    const DenseView& d = T.lv[l].d;
+                    for (int i = tid >> 5; i < nex; i += nt >> 5) {  // a warp per row
+                        double s = 0.0;
+                        for (int k = tid & 31; k < nex; k += 32) s += M[(size_t)i * nex + k] * (double)L.b[idx[k]];
+                        s = warp_sum(s);
+                        const int p = idx[i];
+                        if ((tid & 31) == 0)
+                            L.x[pad_index(d, p % d.D[0], (p / d.D[0]) % d.D[1], p / (d.D[0] * d.D[1]))] = (float)s;
+                    }
+                    tail_bar(nt);
+                } else {
+                    tail_low_smooth(L, T.coarsest_iters, 0, T.omega, nt);
+                }
+                continue;
+            }
+            if (L.fluid) *L.own += (low + T.low[l + 1])[L.parent];
+            tail_bar(nt);
+            tail_low_smooth(L, T.sweeps, 1, T.omega, nt);
+        }
     }
-    const TailLevel& L0 = T.lv[0];
-    tail_step(
-        T.from_msbg ? T.F.g.nb : T.Fd.D[0] * T.Fd.D[1] * T.Fd.D[2],
-        [&](int t, uint32_t* at, float* v) {
-            return dense_prolong_value(L0.A.d, L0.x, T.from_msbg, T.F, T.xf, T.Fd, T.xf, T.fluid_f, t, at, v);
-        },
-        [&](uint32_t at, float v) { T.xf[at] = v; });
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 2 * TAIL_PAIRS; ++j)
+        if ((fl >> j) & 1u) {
+            x[j] += (low + T.low[0])[parent[j >> 1]];
+            xs[(j & 1) * np0 + cell[j >> 1]] = x[j];
+        }
+    __syncthreads();
+        }
+        if (step == npass) break;
+        if (((step - npre) & 1) == (step < npre ? 0 : 1)) pass(0);
+        else pass(1);
+    }
+    pdl_trigger();
+#pragma unroll
+    for (int j = 0; j < 2 * TAIL_PAIRS; ++j)
+        if ((act >> j) & 1u) T.x[at[j]] = x[j];
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1705,29 +1968,28 @@ static int slots_per_cta(int r) {
 // Build the CTA batches of one block-structured level from its per-block resolutions.
 static aw_status build_batches(MGLevel& L, const Geo& geo) {
     const int nb = (int)L.h_res.size();
+    std::vector<int4> desc[3];
+    std::vector<int> blocks[3];
+    std::vector<int> by_res[3][17];
+    for (int b = 0; b < nb; ++b) {
+        const int r = L.h_res[b];
+        if (!r) continue;
+        int c[3];
+        bcoord(geo, b, c);
+        by_res[(c[0] + c[1] + c[2]) & 1][r].push_back(b);
+        by_res[2][r].push_back(b);
+    }
     for (int k = 0; k < 3; ++k) {
-        std::vector<int> by_res[17];
-        for (int b = 0; b < nb; ++b) {
-            const int r = L.h_res[b];
-            if (!r) continue;
-            if (k < 2) {
-                int c[3];
-                bcoord(geo, b, c);
-                if (((c[0] + c[1] + c[2]) & 1) != k) continue;
-            }
-            by_res[r].push_back(b);
-        }
-        std::vector<int> blocks;
-        std::vector<int4> desc;
         for (int r = 16; r >= 1; --r) {
+            const std::vector<int>& list = by_res[k][r];
             const int G = slots_per_cta(r);
-            for (size_t i = 0; i < by_res[r].size(); i += G) {
-                const int cnt = (int)std::min<size_t>(G, by_res[r].size() - i);
-                desc.push_back(make_int4((int)blocks.size(), cnt, r, 0));
-                for (int j = 0; j < cnt; ++j) blocks.push_back(by_res[r][i + j]);
+            for (size_t i = 0; i < list.size(); i += G) {
+                const int cnt = (int)std::min<size_t>(G, list.size() - i);
+                desc[k].push_back(make_int4((int)(blocks[k].size() + i), cnt, r, 0));
             }
-            if (!by_res[r].empty()) {
-                const int Gm = std::min<int>(G, (int)by_res[r].size());
+            blocks[k].insert(blocks[k].end(), list.begin(), list.end());
+            if (!list.empty()) {
+                const int Gm = std::min<int>(G, (int)list.size());
                 const size_t X3 = (size_t)(r + 2) * (r + 2) * (r + 2);
                 L.smem_smooth = std::max(L.smem_smooth, slot_image_bytes(Gm, r, sizeof(float)));
                 L.smem_x64 = std::max(L.smem_x64, slot_image_bytes(Gm, r, sizeof(double)));
@@ -1735,16 +1997,34 @@ static aw_status build_batches(MGLevel& L, const Geo& geo) {
                 L.smem_prolong = std::max(L.smem_prolong, (size_t)Gm * (X3 * 4 + NMETA * 4) + 16);
             }
         }
-        L.ndesc[k] = (int)desc.size();
-        L.h_blocks[k] = std::move(blocks);
-        if (L.ndesc[k]) {
-            AW_TRY(L.desc[k].ensure(desc.size()));
-            AW_CUDA(cudaMemcpy(L.desc[k].p, desc.data(), desc.size() * sizeof(int4), cudaMemcpyHostToDevice));
-        }
+        L.ndesc[k] = (int)desc[k].size();
+        L.nslots[k] = (int)blocks[k].size();
+    }
+    // one allocation and one copy: the descriptors, the blocks, then room for the metadata
+    size_t q[3], o = 0, host;
+    std::vector<int4> img;
+    for (int k = 0; k < 3; ++k) img.insert(img.end(), desc[k].begin(), desc[k].end());
+    for (int k = 0; k < 3; ++k) {
+        q[k] = img.size();
+        img.resize(img.size() + (blocks[k].size() + 3) / 4);
+        if (!blocks[k].empty()) memcpy(img.data() + q[k], blocks[k].data(), blocks[k].size() * sizeof(int));
+    }
+    host = img.size();
+    size_t tot = host;
+    for (int k = 0; k < 3; ++k) tot += (NMETA * blocks[k].size() + 3) / 4;
+    AW_TRY(L.batches.ensure(std::max<size_t>(tot, 1)));
+    if (host) AW_CUDA(cudaMemcpy(L.batches.p, img.data(), host * sizeof(int4), cudaMemcpyHostToDevice));
+    size_t m = host;
+    for (int k = 0; k < 3; ++k) {
+        L.desc[k] = L.batches.p + o;
+        o += desc[k].size();
+        L.blk[k] = reinterpret_cast<int*>(L.batches.p + q[k]);
+        L.meta[k] = reinterpret_cast<int*>(L.batches.p + m);
+        m += (NMETA * blocks[k].size() + 3) / 4;
     }
     return AW_OK;
 }
-static Batch batch(const MGLevel& L, int k) { return Batch{L.desc[k].p, L.meta[k].p, (int)L.h_blocks[k].size()}; }
+static Batch batch(const MGLevel& L, int k) { return Batch{L.desc[k], L.meta[k], L.nslots[k]}; }
 
 // Slot metadata of one batch of level m, laid out in batch order (field-major): block id, offsets,
 // the six face neighbours (cell offset, kind, block) and the block's cells on the adjacent levels.
@@ -1794,14 +2074,10 @@ static MetaSrc meta_src(const MGLevel* L) {
 // The slot metadata of level m's three batches, built on the device.
 static aw_status build_meta(MGLevel& L, const Geo& geo, const MGLevel* finer, const MGLevel* coarser, cudaStream_t s) {
     for (int k = 0; k < 3; ++k) {
-        const std::vector<int>& blocks = L.h_blocks[k];
-        const size_t n = blocks.size();
+        const int n = L.nslots[k];
         if (!n) continue;
-        AW_TRY(L.blk[k].ensure(n));
-        AW_CUDA(cudaMemcpyAsync(L.blk[k].p, blocks.data(), n * sizeof(int), cudaMemcpyHostToDevice, s));
-        AW_TRY(L.meta[k].ensure(NMETA * n));
-        k_build_meta<<<nblk(n), 256, 0, s>>>(geo, L.blk[k].p, (int)n, meta_src(&L), meta_src(finer), meta_src(coarser),
-                                            L.meta[k].p);
+        k_build_meta<<<nblk(n), 256, 0, s>>>(geo, L.blk[k], n, meta_src(&L), meta_src(finer), meta_src(coarser),
+                                            L.meta[k]);
         AW_LAUNCH();
     }
     return AW_OK;
@@ -1956,47 +2232,49 @@ static aw_status coarsest(aw_solver* S, int m, cudaStream_t s) {
     if (fv(S) && S->exact) {
         Uniform U = uniform_of(S, m);
         float* x = L.dense ? L.x.p : (m == 0 && S->x0 ? S->x0 : L.x.p);
-        return launch_dep(S, k_coarse_apply, 4, 128, 0, s, U, (const int*)S->ex_idx.p, (const int*)S->ex_n.p,
+        return launch_dep(S, k_coarse_apply, EXACT_CAP / 8, 256, 0, s, U, (const int*)S->ex_idx.p, (const int*)S->ex_n.p,
                           (const double*)S->Minv.p, bptr(S, m), x);
     }
     return smooth_level(S, m, S->d.coarsest_iterations, s);
 }
 
-// The uniform levels below level m (the last MSBG level or a uniform one) as one launch
-// (k_dense_tail): restriction into them, their V-cycle and the prolongation back into m.
-static aw_status dense_tail(aw_solver* S, int m, cudaStream_t s) {
-    const int last = (int)S->lv.size() - 1;
+// Levels S->tail and below as one launch (k_dense_tail), from x = 0; b of level S->tail is in place.
+static DenseTail tail_args(aw_solver* S) {
+    const int m = S->tail, last = (int)S->lv.size() - 1;
     MGLevel& F = S->lv[m];
     DenseTail T{};
-    T.n = last - m;
+    for (int a = 0; a < 3; ++a) {
+        T.top.d.D[a] = F.dense ? F.D[a] : S->g->st.geo.D[a];
+        T.top.W[a] = F.W[a].p;
+    }
+    T.top.fluid = F.fluid.p;
     T.from_msbg = F.dense ? 0 : 1;
+    if (!F.dense) T.F = lview(S, m);
+    T.x = F.x.p;
+    T.b = F.b.p;
+    T.n = last - m;
     for (int j = 0; j < T.n; ++j) {
         MGLevel& L = S->lv[m + 1 + j];
-        T.lv[j].A = DenseArgs{dview(L), {L.W[0].p, L.W[1].p, L.W[2].p}, L.fluid.p};
-        T.lv[j].x = L.x.p;
-        T.lv[j].b = L.b.p;
-        T.lv[j].r = L.r.p;
+        T.lv[j] = DenseArgs{dview(L), {L.W[0].p, L.W[1].p, L.W[2].p}, L.fluid.p};
     }
-    if (F.dense) {
-        T.Fd = dview(F);
-        T.xf = F.x.p;
-    } else {
-        T.F = lview(S, m);
-        T.xf = xstore(S, m).f;
-    }
-    T.rf = F.r.p;
-    T.fluid_f = F.fluid.p;
+    T.pre = F.dense ? S->d.dense_sweeps : S->d.pre_smooth;
+    T.post = F.dense ? S->d.dense_sweeps : S->d.post_smooth;
+    T.local = S->d.block_iterations;
     T.sweeps = S->d.dense_sweeps;
     T.coarsest_iters = S->d.coarsest_iterations;
     T.exact = S->exact ? 1 : 0;
     T.omega = S->d.omega;
     if (S->exact) {
-        T.U = uniform_of(S, last);
         T.idx = S->ex_idx.p;
         T.ex_n = S->ex_n.p;
         T.Minv = S->Minv.p;
     }
-    return launch_dep(S, k_dense_tail, 1, TAIL_THREADS, 0, s, T);
+    return T;
+}
+static aw_status dense_tail(aw_solver* S, cudaStream_t s) {
+    DenseTail T = tail_args(S);
+    const size_t smem = tail_layout(T);
+    return launch_dep(S, k_dense_tail, 1, TAIL_THREADS, smem, s, T);
 }
 
 static aw_status vcycle(aw_solver* S, int m, cudaStream_t s) {
@@ -2005,13 +2283,13 @@ static aw_status vcycle(aw_solver* S, int m, cudaStream_t s) {
     MGLevel& L = S->lv[m];
     AW_TRY(smooth_level(S, m, L.dense ? S->d.dense_sweeps : S->d.pre_smooth, s));
     AW_TRY(residual_level(S, m, nullptr, s));
-    if (S->tail && m + 1 == S->tail) {
-        AW_TRY(dense_tail(S, m, s));
-        return smooth_level(S, m, L.dense ? S->d.dense_sweeps : S->d.post_smooth, s, true);
-    }
     AW_TRY(restrict_level(S, m, s));
-    AW_TRY(zero_x(S, m + 1, s));
-    AW_TRY(vcycle(S, m + 1, s));
+    if (S->tail && m + 1 == S->tail) {
+        AW_TRY(dense_tail(S, s));
+    } else {
+        AW_TRY(zero_x(S, m + 1, s));
+        AW_TRY(vcycle(S, m + 1, s));
+    }
     AW_TRY(prolong_level(S, m, s));
     AW_TRY(smooth_level(S, m, L.dense ? S->d.dense_sweeps : S->d.post_smooth, s, true));
     return AW_OK;
@@ -2208,15 +2486,19 @@ static aw_status uni_vcycle(aw_solver* S, int m, bool zero, cudaStream_t s) {
     }
     AW_TRY(uni_residual(S, m, x, bptr(S, m), out, nullptr, s));
     int mode = UM_PLAIN;
-    if (S->tail && m + 1 == S->tail) {
-        AW_TRY(dense_tail(S, m, s));
-    } else if (K.dense) {
+    const bool tail = S->tail && m + 1 == S->tail;
+    if (K.dense) {
         AW_TRY(restrict_level(S, m, s));
-        AW_TRY(zero_x(S, m + 1, s));
-        AW_TRY(vcycle(S, m + 1, s));
+        if (tail) {
+            AW_TRY(dense_tail(S, s));
+        } else {
+            AW_TRY(zero_x(S, m + 1, s));
+            AW_TRY(vcycle(S, m + 1, s));
+        }
         AW_TRY(prolong_level(S, m, s));
     } else {
-        AW_TRY(uni_vcycle(S, m + 1, true, s));
+        if (tail) AW_TRY(dense_tail(S, s));
+        else AW_TRY(uni_vcycle(S, m + 1, true, s));
         if (x.h || S->d.post_smooth == 0) {
             const UniView V = uview(L, 2);
             if (x.h && K.half)
@@ -2354,8 +2636,7 @@ static void reset_level(MGLevel& L) {
     L.h_res.clear();
     for (int k = 0; k < 4; ++k) L.tot[k] = 0;
     for (int k = 0; k < 3; ++k) {
-        L.h_blocks[k].clear();
-        L.ndesc[k] = 0;
+        L.ndesc[k] = L.nslots[k] = 0;
     }
     L.smem_smooth = L.smem_x64 = L.smem_prolong = L.smem_meta = 0;
     L.maxres = 0;
@@ -2422,8 +2703,10 @@ static aw_status solver_build(aw_solver* S) {
             break;
         }
         AW_TRY(build_batches(L, G.geo));
-        AW_TRY(L.status[0].ensure(nb));
-        AW_TRY(L.status[1].ensure(nb));
+        if (S->d.theta >= 0.f) {  // the activation flags of smooth_level
+            AW_TRY(L.status[0].ensure(nb));
+            AW_TRY(L.status[1].ensure(nb));
+        }
         L.half = (S->d.precision == AW_PRECISION_MIXED) && m >= 1 && m < M - 1 + (ref ? 0 : 1) && L.maxres > 1;
         size_t nc = L.ncell();
         AW_TRY(L.x.ensure(nc));
@@ -2548,17 +2831,25 @@ static aw_status solver_build(aw_solver* S) {
     S->use_graph = getenv("AW_NO_GRAPH") == nullptr;
     S->use_pdl = getenv("AW_NO_PDL") == nullptr;
     S->use_devloop = getenv("AW_NO_DEVLOOP") == nullptr;
-    // the uniform tail as one launch (FV mode): the uniform levels from the first one of at most
-    // TAIL_MAX_CELLS cells down, at most TAIL_MAX of them, below a level that stores x in FP32
-    // (AW_NO_DENSE_TAIL keeps one launch per step)
+    // the tail as one launch (FV mode): from the first level of at most TAIL_TOP cells that is uniform or,
+    // where k_smooth neither tracks residuals nor deactivates blocks, the one-cell MSBG level below level 0;
+    // the uniform levels under it have at most TAIL_MAX_CELLS cells (AW_NO_DENSE_TAIL keeps one launch per
+    // step).  An 8th of 4096 cells is 512, so any level that qualifies has such levels under it.
     S->tail = 0;
     if (!ref && S->nmsbg > 0 && getenv("AW_NO_DENSE_TAIL") == nullptr) {
         const int nl = (int)S->lv.size();
         int j = S->nmsbg;
-        while (j < nl && S->lv[j].ncell() > (size_t)TAIL_MAX_CELLS) ++j;
-        bool ok = j < nl && nl - j <= TAIL_MAX && !S->lv[j - 1].half;
-        for (int k = j; ok && k < nl; ++k) ok = S->lv[k].dense && S->lv[k].ncell() <= (size_t)TAIL_MAX_CELLS;
-        if (ok) S->tail = j;
+        if (j > 1 && nb <= TAIL_TOP && S->d.theta < 0.f && !track && S->lv[j - 1].maxres == 1 && !S->lv[j - 1].half) --j;
+        else
+            while (j < nl && S->lv[j].ncell() > (size_t)TAIL_TOP) ++j;
+        bool ok = j < nl - 1 && nl - 1 - j <= TAIL_MAX;
+        for (int k = j + 1; ok && k < nl; ++k) ok = S->lv[k].dense && S->lv[k].ncell() <= (size_t)TAIL_MAX_CELLS;
+        if (ok) {
+            S->tail = j;
+            AW_CUDA(cudaFuncSetAttribute(k_dense_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+            DenseTail T = tail_args(S);
+            if (tail_layout(T) > 200 * 1024) S->tail = 0;  // a lattice so thin that its ghost layer dominates
+        }
     }
 
     AW_CUDA(cudaDeviceSynchronize());

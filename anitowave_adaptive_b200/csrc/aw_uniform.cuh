@@ -73,6 +73,14 @@ struct UG {
 __device__ __forceinline__ float ufma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double ufma(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float umul(float a, float b) { return __fmul_rn(a, b); }
+// The staged kernels divide with __fdividef, which is a multiplication by the approximate reciprocal (PTX
+// div.approx.f32) for divisors within 2^-126 .. 2^126; here a cell's divisor is fixed for a launch, so its
+// reciprocal is taken once.
+__device__ __forceinline__ float urcp(float d) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return r;
+}
 __device__ __forceinline__ double umul(double a, double b) { return __dmul_rn(a, b); }
 
 inline int uni_blocks_per_warp(int r) { return r == 8 ? 1 : (r == 4 ? 4 : (r == 2 ? 16 : 32)); }
@@ -435,7 +443,7 @@ template <int R>
 struct UCoef {
     bool one[2], edge[2];
     int src[2];
-    float cW[2], cE[2], wS, wN, diag[2][3];
+    float cW[2], cE[2], wS, wN, diag[2][3], rcp[2][3];
 };
 
 template <int R, int CLS>
@@ -457,15 +465,15 @@ __device__ __forceinline__ void uni_sweep(const ULane<R>& L, const UCoef<R>& C, 
         const float vB = z > 0 ? B[z > 0 ? z - 1 : 0] : zlo;
         const float vT = z < R - 1 ? B[z < R - 1 ? z + 1 : 0] : zhi;
         const float wB = z == 0 ? L.wz0 : L.wi, wT = z == R - 1 ? L.wz1 : L.wi;
-        const float diag = C.diag[par][z == 0 ? 0 : (z == R - 1 ? 2 : 1)];
+        const int zk = z == 0 ? 0 : (z == R - 1 ? 2 : 1);
         float Ax = ufma(C.cW[par], vW, umul(C.cE[par], vE));
         Ax = ufma(C.wS, vS, Ax);
         Ax = ufma(C.wN, vN, Ax);
         Ax = ufma(wB, vB, Ax);
         Ax = ufma(wT, vT, Ax);
-        Ax = ufma(diag, A[z], Ax);
-        const float v = ufma(omega, __fdividef(b[z] - Ax, diag), A[z]);
-        An[z] = ((fl >> (2 * z + CLS)) & 1u) && !(fabsf(diag) < 1e-9f) ? v : A[z];
+        Ax = ufma(C.diag[par][zk], A[z], Ax);
+        const float v = ufma(omega, umul(b[z] - Ax, C.rcp[par][zk]), A[z]);
+        An[z] = (fl >> (2 * z + CLS)) & 1u ? v : A[z];
     }
 #pragma unroll
     for (int z = 0; z < R; ++z) A[z] = An[z];
@@ -534,6 +542,10 @@ __device__ __forceinline__ void uni_smooth_body(const UniView& V, int warp, cons
             }
         }
     }
+    // fluid bits by class: swap the two bits of every height whose E cell is the pair's second
+    const uint32_t sw = ((L.mask & 0x5555u) << 1) | ((L.mask >> 1) & 0x5555u);
+    const uint32_t selm = q ? 0x3333u : 0xCCCCu;
+    uint32_t fl = (L.mask & ~selm) | (sw & selm);
     UCoef<R> C;
     C.wS = L.y == 0 ? L.wy0 : L.wi;
     C.wN = L.y == R - 1 ? L.wy1 : L.wi;
@@ -548,13 +560,18 @@ __device__ __forceinline__ void uni_smooth_body(const UniView& V, int warp, cons
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const float wB = k == 0 ? L.wz0 : L.wi, wT = k == 2 ? L.wz1 : L.wi;
-            C.diag[par][k] = -(C.cW[par] + C.cE[par] + C.wS + C.wN + wB + wT);
+            const float d = -(C.cW[par] + C.cE[par] + C.wS + C.wN + wB + wT);
+            C.diag[par][k] = d;
+            C.rcp[par][k] = urcp(d);
+            if (fabsf(d) < 1e-9f) {  // cut off from every neighbour: never updated
+                uint32_t bits = 0;
+#pragma unroll
+                for (int z = 0; z < R; ++z)
+                    if ((z == 0 ? 0 : (z == R - 1 ? 2 : 1)) == k) bits |= 1u << (2 * z + ((z ^ par) & 1));
+                fl &= ~bits;
+            }
         }
     }
-    // fluid bits by class: swap the two bits of every height whose E cell is the pair's second
-    const uint32_t sw = ((L.mask & 0x5555u) << 1) | ((L.mask >> 1) & 0x5555u);
-    const uint32_t selm = q ? 0x3333u : 0xCCCCu;
-    const uint32_t fl = (L.mask & ~selm) | (sw & selm);
 #pragma unroll 1
     for (int it = 0; it < iters; ++it) {
         uni_sweep<R, 0>(L, C, E, O, bE, hx, H.hy[0], H.hz[0][0], H.hz[1][0], fl, omega);
@@ -631,6 +648,7 @@ __device__ __forceinline__ void uni_smooth_one(const UniView& V, int warp, const
     else H.h[0] = H.h[1] = H.h[2] = H.h[3] = H.h[4] = H.h[5] = 0.f;
     const float(&h)[6] = H.h;
     const float diag = -(L.wx0 + L.wx1 + L.wy0 + L.wy1 + L.wz0 + L.wz1);
+    const float rcp = urcp(diag);
     if ((L.mask & 1u) && !(fabsf(diag) < 1e-9f))
 #pragma unroll 1
         for (int it = 0; it < iters; ++it) {
@@ -640,7 +658,7 @@ __device__ __forceinline__ void uni_smooth_one(const UniView& V, int warp, const
             Ax = ufma(L.wz0, h[4], Ax);
             Ax = ufma(L.wz1, h[5], Ax);
             Ax = ufma(diag, v, Ax);
-            v = ufma(omega, __fdividef(b - Ax, diag), v);
+            v = ufma(omega, umul(b - Ax, rcp), v);
         }
     pdl_trigger();
     uni_store<1, HALF>(L, x, &v, &v);
@@ -1042,12 +1060,28 @@ __device__ __forceinline__ void uni_check_body(const UniView& V, const UCheck& K
     const float* w2 = K.W.w[2] + f2;
     const float wx0 = w0[0], wx1 = w0[R], wy0 = w1[0], wy1 = w1[R * R], wz0 = w2[0], wz1 = w2[R * R * R];
     const float wi = R >= 2 ? w0[1] : wx0;
+    // UB values of each axis in flight per lane (one at a time, 54 dependent round trips of an 8^3 block took
+    // 31 us a launch)
+    constexpr int UB = 6;
     bool same = true;
-    for (int i = li; i < nf; i += G::LPB) {
-        const int fx = i % (R + 1), fy = (i / R) % (R + 1), fz = i / (R * R);
-        same = same && w0[i] == (fx == 0 ? wx0 : (fx == R ? wx1 : wi));
-        same = same && w1[i] == (fy == 0 ? wy0 : (fy == R ? wy1 : wi));
-        same = same && w2[i] == (fz == 0 ? wz0 : (fz == R ? wz1 : wi));
+#pragma unroll 1
+    for (int i0 = li; i0 < nf; i0 += UB * G::LPB) {
+        float a0[UB], a1[UB], a2[UB];
+#pragma unroll
+        for (int k = 0; k < UB; ++k) {
+            const int i = min(i0 + k * G::LPB, nf - 1);
+            a0[k] = w0[i];
+            a1[k] = w1[i];
+            a2[k] = w2[i];
+        }
+#pragma unroll
+        for (int k = 0; k < UB; ++k) {
+            const int i = min(i0 + k * G::LPB, nf - 1);
+            const int fx = i % (R + 1), fy = (i / R) % (R + 1), fz = i / (R * R);
+            same = same && a0[k] == (fx == 0 ? wx0 : (fx == R ? wx1 : wi));
+            same = same && a1[k] == (fy == 0 ? wy0 : (fy == R ? wy1 : wi));
+            same = same && a2[k] == (fz == 0 ? wz0 : (fz == R ? wz1 : wi));
+        }
     }
     int ok = same;
 #pragma unroll
