@@ -52,117 +52,263 @@ __device__ inline uint32_t particle_key(const LevelView& L, const float p[3], ui
     return L.off[0][b] + cidx(q[0], q[1], q[2], r);
 }
 
-__global__ void k_keys(LevelView L, PArr pos, int64_t n, uint32_t invalid, uint32_t* keys, uint32_t* count) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float p[3] = {pos(i, 0), pos(i, 1), pos(i, 2)};
-    uint32_t k = particle_key(L, p, invalid);
-    keys[i] = k;
-    // particles arrive mostly in last step's cell order: lanes with the same cell add once
-    const unsigned peers = __match_any_sync(__activemask(), k);
-    if ((__ffs(peers) - 1) == (int)(threadIdx.x & 31)) atomicAdd(&count[k], (uint32_t)__popc(peers));
-}
-
 // ------------------------------------------------------------------------------------------------
 // Stable LSD radix sort of (key, index) pairs, digits of up to 11 bits (as few passes as the key
 // range allows, the digit width spread evenly over them: 20-bit keys take two 10-bit passes, 22-bit
-// keys two 11-bit passes).  Each pass: per-tile digit histograms -> one exclusive scan over (digit,
-// tile) -> scatter in which one warp walks its tile in order and ranks equal digits with
-// __match_any_sync, so equal keys keep their input order.
+// keys two 11-bit passes).  The input is cut into at most SORT_MAX_TILES tiles, one CTA each.  A pass:
+// per-tile digit histograms (the first pass's by k_keys, which has the keys at hand), one scan kernel
+// (k_radix_rows) and the scatter, in which a CTA walks its tile 4096 keys at a time with all 8 warps:
+// every warp ranks its keys in order with __match_any_sync, a prefix over the warps makes the ranks the
+// tile's, and a running offset per digit carries over.  Equal keys keep their input order.
+//
+// (Before, a single warp walked 2048 keys: 41 us a pass of 4.1M keys at 14 warps per SM, 42 us even for
+// 7,680 particles, with a (digit, tile) table of 2M entries whose scan took 25 us; now 14 and 5 us.)
 // ------------------------------------------------------------------------------------------------
 constexpr int RADIX_MAX_BITS = 11, RADIX_MAX_BINS = 1 << RADIX_MAX_BITS;
+constexpr int SORT_THREADS = 256, SORT_ITEMS = 16, SORT_WARPS = SORT_THREADS / 32;
+constexpr int SORT_MAX_TILES = 592;  // 4 CTAs on each of 148 SMs; more only lengthen the histogram rows
 
-__global__ void __launch_bounds__(256) k_radix_hist(const uint32_t* __restrict__ keys, int64_t n, int shift, int bins,
-                                                    int tile, uint32_t* __restrict__ hist, uint32_t ntiles) {
-    __shared__ uint32_t h[RADIX_MAX_BINS];
-    for (int i = threadIdx.x; i < bins; i += blockDim.x) h[i] = 0;
-    __syncthreads();
-    // keys arrive nearly sorted (runs of equal digits, thousands long in crowded cells): a warp whose
-    // 32 keys share one digit adds once, so shared-memory atomics do not queue on one address
-    const int64_t base = (int64_t)blockIdx.x * tile;
-    for (int i = threadIdx.x; i < tile; i += blockDim.x) {
-        const int64_t j = base + i;
-        const bool valid = j < n;
-        const uint32_t dig = valid ? (keys[j] >> shift) & (uint32_t)(bins - 1) : 0xFFFFFFFFu;
-        const uint32_t d0 = __shfl_sync(0xffffffffu, dig, 0);
-        if (__all_sync(0xffffffffu, dig == d0)) {
-            if ((threadIdx.x & 31) == 0 && valid) atomicAdd(&h[dig], 32u);
-        } else if (valid) {
-            atomicAdd(&h[dig], 1u);
-        }
-    }
-    __syncthreads();
-    for (int d = threadIdx.x; d < bins; d += blockDim.x) hist[(size_t)d * ntiles + blockIdx.x] = h[d];
-}
-
-__global__ void __launch_bounds__(256) k_radix_scatter(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
-                                                       uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, int64_t n,
-                                                       int shift, int bins, int tile, const uint32_t* __restrict__ offs,
-                                                       uint32_t ntiles) {
-    extern __shared__ uint32_t cnt[];  // bins per warp
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t t = blockIdx.x * (blockDim.x >> 5) + w;
-    uint32_t* c = cnt + w * bins;
-    if (t >= ntiles) return;
-    for (int d = lane; d < bins; d += 32) c[d] = offs[(size_t)d * ntiles + t];
-    __syncwarp();
-    const int64_t base = (int64_t)t * tile;
-    const unsigned lt = (1u << lane) - 1u;
-    for (int ch = 0; ch < tile; ch += 32) {
-        const int64_t j = base + ch + lane;
-        const bool valid = j < n;
-        uint32_t key = 0, val = 0, dig = 0;
-        if (valid) {
-            key = kin[j];
-            val = vin ? vin[j] : (uint32_t)j;
-            dig = (key >> shift) & (uint32_t)(bins - 1);
-        }
-        const unsigned peers = __match_any_sync(0xffffffffu, valid ? dig : (uint32_t)(bins + lane));
-        const uint32_t pos = valid ? c[dig] + __popc(peers & lt) : 0u;
-        __syncwarp();
-        if (valid && (__ffs(peers) - 1) == lane) c[dig] += __popc(peers);
-        __syncwarp();
-        if (valid) {
-            kout[pos] = key;
-            vout[pos] = val;
-        }
-    }
-}
-
-static aw_status radix_sort_pairs(uint32_t* keys, uint32_t* keys2, uint32_t* vals, uint32_t* vals2, int64_t n,
-                                  uint32_t maxkey, DBuf<uint32_t>& hist, DBuf<uint32_t>& scan_out, DBuf<uint32_t>& tmp,
-                                  uint32_t** sorted_vals, cudaStream_t s) {
+struct SortPlan {
+    int passes, digit, bins;
+    int64_t tile;
+    uint32_t ntiles;
+};
+static SortPlan sort_plan(int64_t n, uint32_t maxkey) {
+    SortPlan P;
     int bits = 1;
     while (bits < 32 && (maxkey >> bits)) ++bits;
-    const int passes = (bits + RADIX_MAX_BITS - 1) / RADIX_MAX_BITS;
-    const int digit = (bits + passes - 1) / passes;
-    const int bins = 1 << digit;
-    // tiles of 2048 keys, longer for large arrays (down to about 4096 tiles, one wave of warps), so
-    // that the (digit, tile) table and its scan stay small
-    int tile = 2048;
-    while (tile < 16384 && n / (2 * (int64_t)tile) >= 4096) tile *= 2;
-    const uint32_t ntiles = (uint32_t)((n + tile - 1) / tile);
-    const size_t nh = (size_t)bins * ntiles;
-    AW_TRY(hist.ensure(nh));
-    AW_TRY(scan_out.ensure(nh + 1));
-    uint32_t *kin = keys, *kout = keys2, *vin = nullptr, *vout = vals;
-    const int wpb = 8;
-    for (int p = 0; p < passes; ++p) {
-        const int shift = p * digit;
-        k_radix_hist<<<ntiles, 256, 0, s>>>(kin, n, shift, bins, tile, hist.p, ntiles);
-        AW_LAUNCH();
-        AW_TRY(exclusive_scan_u32(hist.p, scan_out.p, nh, tmp, s));
-        const size_t ssm = (size_t)wpb * bins * sizeof(uint32_t);
-        if (ssm > 48 * 1024)
-            AW_CUDA(cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
-        k_radix_scatter<<<(ntiles + wpb - 1) / wpb, 32 * wpb, ssm, s>>>(
-            kin, vin, kout, vout, n, shift, bins, tile, scan_out.p, ntiles);
-        AW_LAUNCH();
-        std::swap(kin, kout);
-        vin = vout;
-        vout = (vout == vals) ? vals2 : vals;
+    P.passes = (bits + RADIX_MAX_BITS - 1) / RADIX_MAX_BITS;
+    P.digit = (bits + P.passes - 1) / P.passes;
+    P.bins = 1 << P.digit;
+    // tiles of 1024 keys for small inputs (many CTAs), then as long as SORT_MAX_TILES of them need
+    P.tile = std::max<int64_t>(1024, ((n + SORT_MAX_TILES - 1) / SORT_MAX_TILES + 1023) / 1024 * 1024);
+    P.ntiles = (uint32_t)((n + P.tile - 1) / P.tile);
+    return P;
+}
+
+// one digit of the warp's keys into the tile's histogram: lanes with equal digits add once
+__device__ __forceinline__ void hist_add(uint32_t* h, uint32_t dig, unsigned active) {
+    const unsigned peers = __match_any_sync(active, dig);
+    if ((__ffs(peers) - 1) == (int)(threadIdx.x & 31)) atomicAdd(&h[dig], (uint32_t)__popc(peers));
+}
+
+// keys, the particle count of every cell, and the first pass's tile histograms
+constexpr int KEYS_THREADS = 512;
+__global__ void __launch_bounds__(KEYS_THREADS) k_keys(LevelView L, PArr pos, int64_t n, uint32_t invalid, uint32_t* keys,
+                                                       uint32_t* count, int bins, int64_t tile, uint32_t* __restrict__ hist,
+                                                       uint32_t ntiles) {
+    __shared__ uint32_t h[RADIX_MAX_BINS];
+    for (int i = threadIdx.x; i < bins; i += KEYS_THREADS) h[i] = 0;
+    __syncthreads();
+    const int64_t i0 = (int64_t)blockIdx.x * tile, i1 = min(i0 + tile, n);
+    for (int64_t i = i0 + threadIdx.x; i < i1; i += KEYS_THREADS) {
+        float p[3] = {pos(i, 0), pos(i, 1), pos(i, 2)};
+        const uint32_t k = particle_key(L, p, invalid);
+        keys[i] = k;
+        // particles arrive mostly in last step's cell order: lanes with the same cell add once
+        const unsigned act = __activemask();
+        const unsigned peers = __match_any_sync(act, k);
+        if ((__ffs(peers) - 1) == (int)(threadIdx.x & 31)) {
+            atomicAdd(&count[k], (uint32_t)__popc(peers));
+            atomicAdd(&h[k & (uint32_t)(bins - 1)], (uint32_t)__popc(peers));
+        }
     }
-    *sorted_vals = vin;
+    __syncthreads();
+    for (int d = threadIdx.x; d < bins; d += KEYS_THREADS) hist[(size_t)d * ntiles + blockIdx.x] = h[d];
+}
+
+__global__ void __launch_bounds__(KEYS_THREADS) k_radix_hist(const uint32_t* __restrict__ keys, int64_t n, int shift,
+                                                             int bins, int64_t tile, uint32_t* __restrict__ hist,
+                                                             uint32_t ntiles) {
+    __shared__ uint32_t h[RADIX_MAX_BINS];
+    for (int i = threadIdx.x; i < bins; i += KEYS_THREADS) h[i] = 0;
+    __syncthreads();
+    const int64_t i0 = (int64_t)blockIdx.x * tile, i1 = min(i0 + tile, n);
+    constexpr int K = 4;  // keys in flight per thread
+    for (int64_t i = i0 + threadIdx.x; i < i1; i += K * KEYS_THREADS) {
+        uint32_t key[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) key[k] = i + k * KEYS_THREADS < i1 ? keys[i + k * KEYS_THREADS] : 0u;
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if (i + k * KEYS_THREADS < i1) hist_add(h, (key[k] >> shift) & (uint32_t)(bins - 1), __activemask());
+    }
+    __syncthreads();
+    for (int d = threadIdx.x; d < bins; d += KEYS_THREADS) hist[(size_t)d * ntiles + blockIdx.x] = h[d];
+}
+
+// Exclusive scan of every digit's row over the tiles, in place (a warp per digit), and, by the CTA that
+// finishes last, of the digits' totals into base.  tot: bins; ticket starts and ends at 0.
+__global__ void __launch_bounds__(256) k_radix_rows(uint32_t* __restrict__ hist, uint32_t ntiles, int bins,
+                                                    uint32_t* tot, uint32_t* __restrict__ base, unsigned* ticket) {
+    constexpr int NC = (SORT_MAX_TILES + 31) / 32;
+    __shared__ uint32_t part[256];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, d = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (d < bins) {
+        uint32_t* row = hist + (size_t)d * ntiles;
+        uint32_t v[NC];
+#pragma unroll
+        for (int k = 0; k < NC; ++k) {
+            const uint32_t t = k * 32 + lane;
+            v[k] = t < ntiles ? row[t] : 0u;
+        }
+        uint32_t carry = 0;
+#pragma unroll
+        for (int k = 0; k < NC; ++k) {
+            if (k * 32 >= (int)ntiles) break;
+            uint32_t x = v[k];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            const uint32_t t = k * 32 + lane;
+            if (t < ntiles) row[t] = carry + x - v[k];
+            carry += __shfl_sync(0xffffffffu, x, 31);
+        }
+        if (lane == 0) tot[d] = carry;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    constexpr int PER = RADIX_MAX_BINS / 256;
+    uint32_t v[PER], s = 0;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = threadIdx.x * PER + k;
+        v[k] = i < bins ? __ldcg(tot + i) : 0u;
+        s += v[k];
+    }
+    part[threadIdx.x] = s;
+    __syncthreads();
+    for (int o = 1; o < 256; o <<= 1) {
+        const uint32_t y = (int)threadIdx.x >= o ? part[threadIdx.x - o] : 0u;
+        __syncthreads();
+        part[threadIdx.x] += y;
+        __syncthreads();
+    }
+    uint32_t acc = part[threadIdx.x] - s;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = threadIdx.x * PER + k;
+        if (i < bins) base[i] = acc;
+        acc += v[k];
+    }
+    if (threadIdx.x == 0) *ticket = 0u;
+}
+
+// vin == nullptr: the value is the index; kout == nullptr: the keys are not needed any more
+__global__ void __launch_bounds__(SORT_THREADS) k_radix_scatter(const uint32_t* __restrict__ kin,
+                                                                const uint32_t* __restrict__ vin,
+                                                                uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
+                                                                int64_t n, int shift, int bins, int64_t tile,
+                                                                const uint32_t* __restrict__ rows,
+                                                                const uint32_t* __restrict__ base, uint32_t ntiles) {
+    extern __shared__ uint32_t sortsm[];  // running offset per digit, then the warps' counts (16 bits)
+    uint32_t* off = sortsm;
+    uint16_t* wc = reinterpret_cast<uint16_t*>(off + bins);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int d = threadIdx.x; d < bins; d += SORT_THREADS) off[d] = base[d] + rows[(size_t)d * ntiles + blockIdx.x];
+    const int64_t i0 = (int64_t)blockIdx.x * tile, i1 = min(i0 + tile, n);
+    const unsigned lt = (1u << lane) - 1u;
+    uint16_t* c = wc + w * bins;
+    for (int64_t s0 = i0; s0 < i1; s0 += SORT_THREADS * SORT_ITEMS) {
+        // the warps take consecutive runs of `items` x 32 keys
+        const int64_t left = i1 - s0;
+        const int items = (int)min((int64_t)SORT_ITEMS, (left + SORT_THREADS - 1) / SORT_THREADS);
+        const int64_t j0 = s0 + (int64_t)w * items * 32 + lane;
+        uint32_t key[SORT_ITEMS], val[SORT_ITEMS], rank[SORT_ITEMS];
+#pragma unroll
+        for (int k = 0; k < SORT_ITEMS; ++k) {
+            const int64_t j = j0 + k * 32;
+            const bool ok = k < items && j < i1;
+            key[k] = ok ? kin[j] : 0u;
+            val[k] = ok ? (vin ? vin[j] : (uint32_t)j) : 0u;
+        }
+        for (int d = threadIdx.x; d < bins * SORT_WARPS / 2; d += SORT_THREADS) reinterpret_cast<uint32_t*>(wc)[d] = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < SORT_ITEMS; ++k) {
+            if (k >= items) break;
+            const bool ok = j0 + k * 32 < i1;
+            const uint32_t dig = (key[k] >> shift) & (uint32_t)(bins - 1);
+            const unsigned peers = __match_any_sync(0xffffffffu, ok ? dig : (uint32_t)(bins + lane));
+            const uint32_t before = ok ? c[dig] : 0u;
+            rank[k] = before + __popc(peers & lt);
+            __syncwarp();
+            if (ok && (__ffs(peers) - 1) == lane) c[dig] = (uint16_t)(before + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        // counts -> exclusive prefix over the warps; the digits' totals wait in the registers of the threads
+        // that own the digits until every offset has been used
+        uint32_t total[RADIX_MAX_BINS / SORT_THREADS];
+#pragma unroll
+        for (int t = 0; t < RADIX_MAX_BINS / SORT_THREADS; ++t) {
+            const int d = threadIdx.x + t * SORT_THREADS;
+            if (d >= bins) break;
+            uint32_t v[SORT_WARPS], acc = 0;
+#pragma unroll
+            for (int q = 0; q < SORT_WARPS; ++q) v[q] = wc[q * bins + d];
+#pragma unroll
+            for (int q = 0; q < SORT_WARPS; ++q) {
+                wc[q * bins + d] = (uint16_t)acc;
+                acc += v[q];
+            }
+            total[t] = acc;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < SORT_ITEMS; ++k) {
+            if (k >= items || j0 + k * 32 >= i1) break;
+            const uint32_t dig = (key[k] >> shift) & (uint32_t)(bins - 1);
+            rank[k] += c[dig];
+            const uint32_t at = off[dig] + rank[k];
+            if (kout) kout[at] = key[k];
+            vout[at] = val[k];
+        }
+        if (s0 + SORT_THREADS * SORT_ITEMS >= i1) break;
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < RADIX_MAX_BINS / SORT_THREADS; ++t) {
+            const int d = threadIdx.x + t * SORT_THREADS;
+            if (d < bins) off[d] += total[t];
+        }
+    }
+}
+
+// The keys (already in `keys`, with the first pass's histograms in hist) sorted: *sorted_vals receives the
+// input indices in key order.  keys itself is kept.
+static aw_status radix_sort_pairs(const SortPlan& P, ParticleWork& W, int64_t n, uint32_t** sorted_vals, cudaStream_t s) {
+    const uint32_t* kin = W.keys.p;
+    const uint32_t* vin = nullptr;
+    uint32_t *kout = W.keys2.p, *vout = W.perm.p;
+    unsigned* ticket = reinterpret_cast<unsigned*>(W.hscan.p + 2 * RADIX_MAX_BINS);
+    const size_t ssm = (size_t)P.bins * (sizeof(uint32_t) + SORT_WARPS * sizeof(uint16_t));
+    AW_CUDA(cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(RADIX_MAX_BINS * (sizeof(uint32_t) + SORT_WARPS * sizeof(uint16_t)))));
+    for (int p = 0; p < P.passes; ++p) {
+        const int shift = p * P.digit;
+        if (p > 0) {
+            k_radix_hist<<<P.ntiles, KEYS_THREADS, 0, s>>>(kin, n, shift, P.bins, P.tile, W.hist.p, P.ntiles);
+            AW_LAUNCH();
+        }
+        k_radix_rows<<<(P.bins + 7) / 8, 256, 0, s>>>(W.hist.p, P.ntiles, P.bins, W.hscan.p, W.hscan.p + RADIX_MAX_BINS,
+                                                      ticket);
+        AW_LAUNCH();
+        k_radix_scatter<<<P.ntiles, SORT_THREADS, ssm, s>>>(kin, vin, p + 1 < P.passes ? kout : nullptr, vout, n, shift,
+                                                            P.bins, P.tile, W.hist.p, W.hscan.p + RADIX_MAX_BINS, P.ntiles);
+        AW_LAUNCH();
+        kin = kout;
+        kout = kout == W.keys2.p ? W.keys3.p : W.keys2.p;
+        vin = vout;
+        vout = vout == W.perm.p ? W.perm2.p : W.perm.p;
+    }
+    *sorted_vals = const_cast<uint32_t*>(vin);
     return AW_OK;
 }
 
@@ -289,20 +435,23 @@ aw_status sort_core(MsbgState& G, PArr pos, int64_t n, cudaStream_t s) {
     ParticleWork& W = G.pw;
     AW_TRY(W.ensure(n, nc));
     AW_CUDA(cudaMemsetAsync(W.cell_fill.p, 0, ((size_t)nc + 2) * sizeof(uint32_t), s));
+    const SortPlan P = sort_plan(n, nc);
     if (n > 0) {
-        k_keys<<<nblk(n), 256, 0, s>>>(G.view0(), pos, n, nc, W.keys.p, W.cell_fill.p);
+        AW_TRY(W.keys2.ensure((size_t)n));
+        if (P.passes > 2) AW_TRY(W.keys3.ensure((size_t)n));
+        AW_TRY(W.hist.ensure((size_t)P.bins * P.ntiles));
+        if (!W.hscan.p) {
+            AW_TRY(W.hscan.ensure(2 * RADIX_MAX_BINS + 1));
+            AW_CUDA(cudaMemsetAsync(W.hscan.p, 0, (2 * RADIX_MAX_BINS + 1) * sizeof(uint32_t), s));
+        }
+        k_keys<<<P.ntiles, KEYS_THREADS, 0, s>>>(G.view0(), pos, n, nc, W.keys.p, W.cell_fill.p, P.bins, P.tile, W.hist.p,
+                                                 P.ntiles);
         AW_LAUNCH();
     }
     AW_TRY(exclusive_scan_u32(W.cell_fill.p, W.cell_start.p, (size_t)nc + 1, W.tmp, s));
     W.sorted = W.perm.p;
     W.src_valid = false;  // the recorded order of aw_p2g is replaced
-    if (n > 0) {
-        // keys are consumed by the sort: keep a copy for aw_sort_particles' key output
-        AW_TRY(W.keys2.ensure((size_t)n));
-        AW_TRY(W.keys3.ensure((size_t)n));
-        AW_CUDA(cudaMemcpyAsync(W.keys3.p, W.keys.p, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-        AW_TRY(radix_sort_pairs(W.keys3.p, W.keys2.p, W.perm.p, W.perm2.p, n, nc, W.hist, W.hscan, W.tmp, &W.sorted, s));
-    }
+    if (n > 0) AW_TRY(radix_sort_pairs(P, W, n, &W.sorted, s));
     return AW_OK;
 }
 
