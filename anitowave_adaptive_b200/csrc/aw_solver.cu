@@ -55,10 +55,11 @@ struct MGLevel {
     size_t smem_smooth = 0, smem_x64 = 0, smem_prolong = 0, smem_meta = 0;
     int maxres = 0;
     // the same blocks as warps of the uniform-coefficient kernels (aw_uniform.cuh): colour 0, colour 1
-    int2* udesc = nullptr;  // these four lie in the solver's uslab
+    int2* udesc = nullptr;  // these five lie in the solver's uslab
     int4* urec = nullptr;
     float4* uwt = nullptr;
     uint16_t* umask = nullptr;
+    uint8_t* ugeneral = nullptr;
     int uwarps[2] = {0, 0};
     DBuf<float> W[3], bbar[3];
     DBuf<uint8_t> fluid;
@@ -88,9 +89,10 @@ struct aw_solver {
     // level-0 bindings for the current solve
     float* x0 = nullptr;
     const float* b0 = nullptr;
-    // the hierarchy can run the uniform-coefficient kernels (FV mode, 8^3 blocks at most, no activation
-    // or early exit), and the current solve does: every block's coefficients are uniform
-    bool uni_able = false, uni = false;
+    // the hierarchy runs the register-resident kernels of aw_uniform.cuh (FV mode, 8^3 blocks at most, no
+    // activation or early exit)
+    bool uni = false;
+    unsigned gen = 0;  // bit m: level m has blocks without a single conductance (the current solve's check)
     aw::DBuf<int4> uslab;  // slot records, weights, masks and warp descriptors of every level
     // mixed precision: FP64 vectors of the conjugate-gradient outer loop (residual, direction (two
     // buffers: the uniform form reads the old one while it writes the new), -A d), its scalars
@@ -107,13 +109,14 @@ struct aw_solver {
     cudaGraphExec_t cycle = nullptr;
     const void* cycle_x0 = nullptr;
     const void* cycle_b0 = nullptr;
-    int cycle_form = -1;  // 2 * uni + (level-0 x starts at zero)
+    unsigned cycle_form = ~0u;  // 2 * gen + (level-0 x starts at zero)
     unsigned long long cycle_kernels = 0;
+    bool vcycle_called = false;  // aw_vcycle_run ran since the solver was built
     // the mixed-precision CG iterations as one graph with a device-side while loop, per pressure
     // array; cgst = {iterations, restart flag, iteration limit}, cgprm = {||b||, tolerance}
     cudaGraphExec_t cgloop = nullptr;
     const void* cgloop_p = nullptr;
-    bool cgloop_uni = false;
+    unsigned cgloop_gen = 0;
     unsigned long long cgloop_kernels = 0;
     bool use_devloop = true;
     aw::DBuf<int> cgst;
@@ -121,7 +124,7 @@ struct aw_solver {
     bool use_graph = true;
     bool use_pdl = true;  // V-cycle kernels as programmatic dependent launches
     int tail = 0;         // first level of the uniform tail run as one k_dense_tail launch (0: none)
-    double* h_norm = nullptr;  // pinned host words: a squared norm, the count of non-uniform blocks
+    double* h_norm = nullptr;  // pinned host words: a squared norm, uniform_check's counts
     double* h_cg = nullptr;    // pinned host words of the device-loop state
     ~aw_solver() {
         if (cycle) cudaGraphExecDestroy(cycle);
@@ -2295,7 +2298,7 @@ static aw_status vcycle(aw_solver* S, int m, cudaStream_t s) {
     return AW_OK;
 }
 
-// ---- uniform coefficients: the register-resident kernels of aw_uniform.cuh -----------------------
+// ---- the register-resident kernels of aw_uniform.cuh --------------------------------------------
 // Slots, warps and slot records of every block-structured level.  All levels list their blocks in one
 // order (colour 0 then 1, native resolutions descending: a level's resolutions then descend too), in
 // one device allocation filled by one copy.
@@ -2343,12 +2346,13 @@ static aw_status build_uniform(aw_solver* S, cudaStream_t s) {
         }
     }
     auto q16 = [](size_t bytes) { return (bytes + 15) / 16; };
-    size_t tot = q16(img.size() * sizeof(int)), o_rec[UNI_MAX_LEVELS], o_wt[UNI_MAX_LEVELS], o_mask[UNI_MAX_LEVELS];
+    size_t tot = q16(img.size() * sizeof(int)), o_rec[UNI_MAX_LEVELS], o_wt[UNI_MAX_LEVELS], o_mask[UNI_MAX_LEVELS], o_gen[UNI_MAX_LEVELS];
     for (int m = 0; m < nl; ++m) {
         o_rec[m] = tot;
         o_wt[m] = o_rec[m] + n * UREC;
         o_mask[m] = o_wt[m] + 2 * n;
-        tot = o_mask[m] + q16(ndesc[m] * 32 * sizeof(uint16_t));
+        o_gen[m] = o_mask[m] + q16(ndesc[m] * 32 * sizeof(uint16_t));
+        tot = o_gen[m] + q16(ndesc[m]);
     }
     AW_TRY(S->uslab.ensure(std::max<size_t>(tot, 1)));
     if (!n) return AW_OK;
@@ -2360,6 +2364,7 @@ static aw_status build_uniform(aw_solver* S, cudaStream_t s) {
         L.urec = S->uslab.p + o_rec[m];
         L.uwt = reinterpret_cast<float4*>(S->uslab.p + o_wt[m]);
         L.umask = reinterpret_cast<uint16_t*>(S->uslab.p + o_mask[m]);
+        L.ugeneral = reinterpret_cast<uint8_t*>(S->uslab.p + o_gen[m]);
         k_build_records<<<nblk(n), 256, 0, s>>>(geo, blk, (int)n, meta_src(&L), meta_src(m + 1 < nl ? &S->lv[m + 1] : nullptr),
                                                 reinterpret_cast<int*>(L.urec));
         AW_LAUNCH();
@@ -2373,6 +2378,8 @@ static UniView uview(const MGLevel& L, int k) {  // k: colour 0, 1, or 2 for bot
     V.rec = L.urec;
     V.wt = L.uwt;
     V.mask = L.umask;
+    V.general = L.ugeneral;
+    V.W = coef(L);
     V.first = k == 1 ? L.uwarps[0] : 0;
     V.nwarp = k == 2 ? L.uwarps[0] + L.uwarps[1] : L.uwarps[k];
     return V;
@@ -2383,9 +2390,9 @@ static UX<HALF> ux(const XStore& x) {
     return UX<HALF>{x.f, x.h, x.scale};
 }
 
-// Which blocks of which levels are uniform; *S->norm[1] (as an int) receives the number of live blocks
-// that are not.  Clears x of the blocks without fluid on the levels whose x starts at zero (level 0
-// too with own_x0: then x0 is the solver's array), and both direction buffers there.
+// Weights, fluid masks and states of every block on every level.  Clears x of the blocks without fluid on
+// the levels whose x starts at zero (level 0 too with own_x0: then x0 is the solver's array), and both
+// direction buffers there.
 static aw_status uniform_check(aw_solver* S, bool own_x0, cudaStream_t s) {
     UCheckAll K{};
     unsigned grid = 1;
@@ -2393,7 +2400,6 @@ static aw_status uniform_check(aw_solver* S, bool own_x0, cudaStream_t s) {
         MGLevel& L = S->lv[m];
         K.v[m] = uview(L, 2);
         UCheck& c = K.k[m];
-        c.W = coef(L);
         c.fluid = L.fluid.p;
         if (m > 0 || own_x0) {
             c.x = L.half ? nullptr : L.x.p;
@@ -2406,10 +2412,11 @@ static aw_status uniform_check(aw_solver* S, bool own_x0, cudaStream_t s) {
         }
         c.wt = L.uwt;
         c.mask = L.umask;
-        c.counts = reinterpret_cast<int*>(S->norm.p + 1);
+        c.general = L.ugeneral;
+        c.count = reinterpret_cast<int*>(S->norm.p + 1) + m;
         grid = std::max(grid, ugrid(K.v[m]));
     }
-    AW_CUDA(cudaMemsetAsync(S->norm.p + 1, 0, sizeof(double), s));
+    AW_CUDA(cudaMemsetAsync(S->norm.p + 1, 0, UNI_MAX_LEVELS * sizeof(int), s));
     k_uni_check<<<dim3(grid, S->nmsbg), UNT, 0, s>>>(K);
     AW_LAUNCH();
     return AW_OK;
@@ -2422,8 +2429,10 @@ static aw_status uni_smooth_t(aw_solver* S, int m, int k, int rev, cudaStream_t 
     const UniView V = uview(L, k);
     if (!V.nwarp) return AW_OK;
     const bool prol = MODE == UM_PROLONG_ALL || MODE == UM_PROLONG_OWN;
-    return launch_dep(S, k_uni_smooth<HALF, MODE, HC>, ugrid(V), UNT, 0, s, V, ux<HALF>(xstore(S, m)),
-                      prol ? ux<HC>(xstore(S, m + 1)) : UX<HC>{}, bptr(S, m), S->d.omega, (int)S->d.block_iterations, rev);
+    const USmooth<HALF, HC> K{V, ux<HALF>(xstore(S, m)), prol ? ux<HC>(xstore(S, m + 1)) : UX<HC>{}, bptr(S, m),
+                              S->d.omega, (int)S->d.block_iterations, rev};
+    if ((S->gen >> m) & 1u) return launch_dep(S, k_uni_smooth<HALF, MODE, HC, true>, ugrid(V), UNT, 0, s, K);
+    return launch_dep(S, k_uni_smooth<HALF, MODE, HC, false>, ugrid(V), UNT, 0, s, K);
 }
 static aw_status uni_smooth(aw_solver* S, int m, int k, int rev, int mode, cudaStream_t s) {
     const bool half = S->lv[m].half && !(m == 0 && S->x0);
@@ -2452,14 +2461,15 @@ static aw_status uni_residual(aw_solver* S, int m, const XStore& x, const float*
                               cudaStream_t s) {
     const UniView V = uview(S->lv[m], 2);
     if (!V.nwarp) return AW_OK;
+    const bool gen = (S->gen >> m) & 1u;
     if (x.h)
-        return launch_dep(S, k_uni_residual<true>, ugrid(V), UNT, 0, s, V, ux<true>(x), b, out, S->partials.p,
-                          S->ticket.p, sum);
-    return launch_dep(S, k_uni_residual<false>, ugrid(V), UNT, 0, s, V, ux<false>(x), b, out, S->partials.p, S->ticket.p,
-                      sum);
+        return launch_dep(S, gen ? k_uni_residual<true, true> : k_uni_residual<true, false>, ugrid(V), UNT, 0, s, V,
+                          ux<true>(x), b, out, S->partials.p, S->ticket.p, sum);
+    return launch_dep(S, gen ? k_uni_residual<false, true> : k_uni_residual<false, false>, ugrid(V), UNT, 0, s, V,
+                      ux<false>(x), b, out, S->partials.p, S->ticket.p, sum);
 }
 
-// The V-cycle on a hierarchy whose live blocks are all uniform: the steps of vcycle() with the
+// The V-cycle by the register-resident kernels: the steps of vcycle() with the
 // residual restricted as it is taken, levels starting at zero without a clearing pass (zero: this
 // level does), and the correction of an FP32 level added where its first post-smoothing reads it.
 static aw_status uni_vcycle(aw_solver* S, int m, bool zero, cudaStream_t s) {
@@ -2671,6 +2681,7 @@ static aw_status solver_build(aw_solver* S) {
     if (S->cycle) cudaGraphExecDestroy(S->cycle);
     S->cycle = nullptr;
     S->cycle_x0 = S->cycle_b0 = nullptr;
+    S->vcycle_called = false;
     if (S->cgloop) cudaGraphExecDestroy(S->cgloop);
     S->cgloop = nullptr;
     S->cgloop_p = nullptr;
@@ -2734,14 +2745,13 @@ static aw_status solver_build(aw_solver* S) {
         S->smem_max = std::max({S->smem_max, L.smem_smooth, L.smem_prolong, L.smem_meta});
         S->smem_max64 = std::max(S->smem_max64, L.smem_x64);
     }
-    // the uniform-coefficient kernels take FV levels of at most 8^3 blocks without activation flags or
+    // the register-resident kernels take FV levels of at most 8^3 blocks without activation flags or
     // per-block early exit (the FV defaults; k_smooth tracks block residuals otherwise)
     const bool track = S->d.target_reduction > 0.f && (S->d.block_iterations > 2 ||
                                                       (S->d.block_iterations == 2 && S->d.target_reduction >= 1.f));
-    S->uni_able = !ref && S->d.theta < 0.f && !track && G.geo.R0 <= UNI_MAX_RES && S->nmsbg > 0 &&
-                  S->nmsbg <= UNI_MAX_LEVELS && getenv("AW_NO_UNIFORM") == nullptr;
-    S->uni = false;
-    if (S->uni_able) AW_TRY(build_uniform(S, s));
+    S->uni = !ref && S->d.theta < 0.f && !track && G.geo.R0 <= UNI_MAX_RES && S->nmsbg > 0 &&
+             S->nmsbg <= UNI_MAX_LEVELS && getenv("AW_NO_UNIFORM") == nullptr;
+    if (S->uni) AW_TRY(build_uniform(S, s));
     // uniform continuation below one cell per block (FV mode)
     size_t used = (size_t)S->nmsbg;
     if (!ref && S->nmsbg > 0 && S->lv[S->nmsbg - 1].maxres == 1) {
@@ -2825,7 +2835,7 @@ static aw_status solver_build(aw_solver* S) {
     // partial sums: one per CTA of the widest launch (batches and uniform warps hold at least one block)
     size_t nparts = (size_t)nb + 2048;
     AW_TRY(S->partials.ensure(nparts));
-    AW_TRY(S->norm.ensure(2));
+    AW_TRY(S->norm.ensure(1 + UNI_MAX_LEVELS / 2));  // a squared norm; uniform_check's count per level
     AW_TRY(S->ticket.ensure(1));
     AW_CUDA(cudaMemset(S->ticket.p, 0, sizeof(unsigned)));
     S->use_graph = getenv("AW_NO_GRAPH") == nullptr;
@@ -2986,7 +2996,7 @@ static aw_status run_vcycle(aw_solver* S, bool zero, cudaStream_t s) {
     if (!S->use_graph) return solve_vcycle(S, zero, s);
     const void* x0 = S->x0 ? (const void*)S->x0 : (const void*)S->lv[0].x.p;
     const void* b0 = S->b0 ? (const void*)S->b0 : (const void*)S->lv[0].b.p;
-    const int form = (S->uni ? 2 : 0) + (zero ? 1 : 0);
+    const unsigned form = 2 * S->gen + (zero ? 1u : 0u);
     if (!S->cycle || S->cycle_x0 != x0 || S->cycle_b0 != b0 || S->cycle_form != form) {
         if (S->cycle) {
             cudaGraphExecDestroy(S->cycle);
@@ -3026,13 +3036,24 @@ extern "C" aw_status aw_solver_coarsest_solve(aw_solver* S, aw_stream s) {
 }
 extern "C" aw_status aw_vcycle_run(aw_solver* S, aw_stream s) {
     AW_CHECK_ARG(S, "null solver");
-    return vcycle(S, 0, (cudaStream_t)s);
+    if (!S->uni) return vcycle(S, 0, (cudaStream_t)s);
+    AW_TRY(uniform_check(S, false, (cudaStream_t)s));
+    S->gen = (1u << S->nmsbg) - 1;  // no host read here: the kernels that take any block
+    // replayed from a graph (a launch each costs the host more than the kernels take) from the second call
+    // on (building it costs about one call), unless the caller is capturing this stream
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    AW_CUDA(cudaStreamIsCapturing((cudaStream_t)s, &cap));
+    if (!S->vcycle_called || cap != cudaStreamCaptureStatusNone) {
+        S->vcycle_called = true;
+        return solve_vcycle(S, false, (cudaStream_t)s);
+    }
+    return run_vcycle(S, false, (cudaStream_t)s);
 }
 
-// *out = sqrt of the sum in S->norm[0], read back (syncs); counts the non-uniform blocks too
+// *out = sqrt of the sum in S->norm[0], read back with uniform_check's counts (syncs)
 static aw_status fetch_norm(aw_solver* S, cudaStream_t s, double* out) {
-    if (!S->h_norm) AW_CUDA(cudaHostAlloc((void**)&S->h_norm, 2 * sizeof(double), cudaHostAllocDefault));
-    AW_CUDA(cudaMemcpyAsync(S->h_norm, S->norm.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
+    if (!S->h_norm) AW_CUDA(cudaHostAlloc((void**)&S->h_norm, 4 * sizeof(double), cudaHostAllocDefault));
+    AW_CUDA(cudaMemcpyAsync(S->h_norm, S->norm.p, (1 + UNI_MAX_LEVELS / 2) * sizeof(double), cudaMemcpyDeviceToHost, s));
     AW_CUDA(cudaStreamSynchronize(s));
     *out = std::sqrt(S->h_norm[0]);
     return AW_OK;
@@ -3057,7 +3078,8 @@ static aw_status true_residual(aw_solver* S, const float* p32, const double* p64
         const UniView V = uview(L0, 2);
         if (!V.nwarp) AW_CUDA(cudaMemsetAsync(S->norm.p, 0, sizeof(double), s));
         else if (p64) {
-            k_uni_residual64<<<ugrid(V), UNT, 0, s>>>(V, USrcD{p64}, b, out, S->partials.p, S->ticket.p, S->norm.p);
+            (S->gen & 1u ? k_uni_residual64<true> : k_uni_residual64<false>)<<<ugrid(V), UNT, 0, s>>>(
+                V, USrcD{p64}, b, out, S->partials.p, S->ticket.p, S->norm.p);
             AW_LAUNCH();
         } else {
             AW_TRY(uni_residual(S, 0, xp, b, out, S->norm.p, s));
@@ -3095,7 +3117,7 @@ static aw_status cg_iteration(aw_solver* S, double* p, unsigned ndot, cudaStream
         UOut out{};
         out.r64 = S->cg_q.p;
         const UniView V = uview(L0, 2);
-        AW_TRY(launch_dep(S, k_uni_apply, ugrid(V), UNT, 0, s, V, (const float*)L0.x.p, S->cg_d.p, S->cg_d2.p, out,
+        AW_TRY(launch_dep(S, S->gen & 1u ? k_uni_apply<true> : k_uni_apply<false>, ugrid(V), UNT, 0, s, V, (const float*)L0.x.p, S->cg_d.p, S->cg_d2.p, out,
                           (const double*)sc, (const int*)S->cgst.p, S->partials.p, S->ticket.p, sc + 2));
     } else {
         K.d0 = K.d1 = S->cg_d.p;
@@ -3163,7 +3185,7 @@ static bool cg_devloop_build(aw_solver* S, double* p, unsigned ndot) {
         return false;
     }
     S->cgloop_p = p;
-    S->cgloop_uni = S->uni;
+    S->cgloop_gen = S->gen;
     return true;
 }
 
@@ -3181,17 +3203,20 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
     }
     // reductions over the level-0 cells: at most 8 CTAs per SM, two cells per thread and step, grid-stride
     const unsigned ndot = (unsigned)std::max<size_t>(1, std::min<size_t>({(size_t)nsm * 8, nc / 512 + 1, S->partials.n}));
-    // ||b||, and whether the uniform-coefficient kernels apply to this solve
-    if (S->uni_able) AW_TRY(uniform_check(S, S->d.precision != AW_PRECISION_FP32, s));
+    // the blocks' coefficients and masks, ||b||
+    if (S->uni) AW_TRY(uniform_check(S, S->d.precision != AW_PRECISION_FP32, s));
     k_sumsq<<<ndot, 256, 0, s>>>(d_b, L0.fluid.p, nc, cf, S->partials.p, S->ticket.p, S->norm.p);
     AW_LAUNCH();
     double bn;
     AW_TRY(fetch_norm(S, s, &bn));
     if (!(bn == bn) || std::isinf(bn)) return set_error(AW_ERR_NAN, "right-hand side contains NaN/Inf");
     if (bn == 0.0) bn = 1.0;
-    int general = 0;
-    memcpy(&general, S->h_norm + 1, sizeof general);
-    S->uni = S->uni_able && general == 0;
+    S->gen = 0;
+    for (int m = 0; S->uni && m < S->nmsbg; ++m) {
+        int c;
+        memcpy(&c, reinterpret_cast<const char*>(S->h_norm + 1) + m * sizeof(int), sizeof c);
+        if (c) S->gen |= 1u << m;
+    }
     const int nlist = L0.ndesc[2];
     int it = 0;
     double rel = 0;
@@ -3327,7 +3352,7 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
                 st = set_error(AW_ERR_NOT_CONVERGED, "relative residual %.3e after %d iterations", rel, it);
                 break;
             }
-            if (S->use_graph && S->use_devloop && (S->cgloop_p != (const void*)p || S->cgloop_uni != S->uni) &&
+            if (S->use_graph && S->use_devloop && (S->cgloop_p != (const void*)p || S->cgloop_gen != S->gen) &&
                 !cg_devloop_build(S, p, ndot))
                 S->use_devloop = false;  // no such graph on this device: the host loop below
             if (restart) {

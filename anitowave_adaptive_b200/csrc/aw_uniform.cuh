@@ -1,15 +1,15 @@
-// aw_uniform.cuh — register-resident multigrid kernels for blocks with uniform coefficients.
+// aw_uniform.cuh — register-resident multigrid kernels of the finite-volume V-cycle.
 //
-// With one density (beta = 1/rho constant over a block) the finite-volume conductances of a block are
-// seven numbers: one for every face between two of its cells and one per side of the block (wall,
-// same, coarser, finer or absent neighbour).  k_uni_check establishes this from the coefficient
-// arrays themselves at the start of every solve, block by block; nothing is remembered from an
-// earlier call.  The kernels here then hold a block in the registers of a group of lanes:
+// A block of R^3 cells takes R * R/2 lanes: a lane holds the x pair (2 xp, 2 xp + 1) of one y for every z,
+// so z neighbours are the lane's own registers, x and y neighbours come by warp shuffles and only the
+// block's halo comes from memory.  A warp serves one 8^3, 4 4^3, 16 2^3 or 32 1^3 blocks, without shared
+// memory and without a CTA barrier.
 //
-//   a block of R^3 cells takes R * R/2 lanes; a lane holds the x pair (2 xp, 2 xp + 1) of one y for
-//   every z, so z neighbours are the lane's own registers, x and y neighbours come by warp shuffles
-//   and only the block's halo comes from memory.  A warp serves one 8^3, 4 4^3, 16 2^3 or 32 1^3
-//   blocks, without shared memory and without a CTA barrier.
+// With one density (beta = 1/rho constant over a block) the conductances of a block are seven numbers: one
+// for every face between two of its cells and one per side of the block (wall, same, coarser, finer or
+// absent neighbour).  k_uni_check establishes this from the coefficient arrays themselves at the start of
+// every solve, block by block; nothing is remembered from an earlier call.  Blocks that are not uniform
+// (a two-phase interface) read each cell's six conductances where they need them.
 //
 // What bounded the staged form (one CTA per 8^3 block: block, halo and the three coefficient arrays
 // in shared memory) was instruction issue: index splits of the staging loops, six shared-memory
@@ -42,7 +42,7 @@ constexpr int UWARPS = UNT / 32;
 constexpr int UREC = 8;               // int4 words of a slot record
 constexpr int UNI_MAX_RES = 8;        // 16^3 blocks would take 128 cells per lane: they keep the staged form
 
-// state of a slot, set by k_uni_check
+// state of a slot, set by k_uni_check: no fluid cell (nothing to do), one conductance, several
 enum { US_AIR = 0, US_UNIFORM = 1, US_GENERAL = 2 };
 
 // One block-structured level as the kernels below see it.  Slots: the level's active blocks, colour 0
@@ -58,6 +58,8 @@ struct UniView {
     const int4* rec;
     const float4* wt;
     const uint16_t* mask;
+    const uint8_t* general;  // per warp: some block of it is not uniform
+    Coef3 W;           // the level's conductances (blocks that are not uniform)
     int first, nwarp;  // the warps of this launch
 };
 
@@ -140,7 +142,7 @@ template <int R>
 struct ULane {
     using G = UG<R>;
     int lane, y, xp;
-    bool live;
+    bool live, general;  // holds fluid; has no single conductance
     uint32_t off;      // cell offset of the block
     uint32_t at;       // ... of the lane's pair at z = 0
     bool even;         // pairs start at even indices
@@ -169,7 +171,8 @@ struct ULane {
         wy1 = wb.x;
         wz0 = wb.y;
         wz1 = wb.z;
-        live = s < cnt && __float_as_int(wb.w) == US_UNIFORM;
+        live = s < cnt && __float_as_int(wb.w) != US_AIR;
+        general = live && __float_as_int(wb.w) == US_GENERAL;
         off = (uint32_t)r0.x;
         block = r0.y;
         kinds = r0.z;
@@ -177,6 +180,19 @@ struct ULane {
         at = off + (uint32_t)(G::NI * xp + R * y);
         even = (off & 1u) == 0;
         return __any_sync(0xffffffffu, live);
+    }
+    // the six conductances {W, E, S, N, B, T} of cell (2 xp + i, y, z)
+    __device__ __forceinline__ void weights(const Coef3& W, int i, int z, float (&w)[6]) const {
+        const int x = G::NI * xp + i;
+        const float* a = W.w[0] + foff(0) + (x + (R + 1) * (y + R * z));
+        const float* b = W.w[1] + foff(1) + (x + R * (y + (R + 1) * z));
+        const float* c = W.w[2] + foff(2) + (x + R * (y + R * z));
+        w[0] = a[0];
+        w[1] = a[1];
+        w[2] = b[0];
+        w[3] = b[R];
+        w[4] = c[0];
+        w[5] = c[R * R];
     }
     __device__ __forceinline__ int word(int k) const { return reinterpret_cast<const int*>(rec)[k]; }
     __device__ __forceinline__ int kind(int f) const { return (kinds >> (4 * f)) & 15; }
@@ -441,12 +457,13 @@ enum { UM_PLAIN = 0, UM_ZERO_ALL = 1, UM_ZERO_OWN = 2, UM_PROLONG_ALL = 3, UM_PR
 // next lane on its side.
 template <int R>
 struct UCoef {
+    const float* face[3];  // the first faces of the pair's first cell at z = 0 (general blocks)
     bool one[2], edge[2];
     int src[2];
     float cW[2], cE[2], wS, wN, diag[2][3], rcp[2][3];
 };
 
-template <int R, int CLS>
+template <int R, int CLS, bool GEN>
 __device__ __forceinline__ void uni_sweep(const ULane<R>& L, const UCoef<R>& C, float (&A)[R], const float (&B)[R],
                                           const float (&b)[R], const float* hx, const float (&hy)[R], float zlo, float zhi,
                                           uint32_t fl, float omega) {
@@ -464,25 +481,55 @@ __device__ __forceinline__ void uni_sweep(const ULane<R>& L, const UCoef<R>& C, 
         const float vW = C.one[par] ? B[z] : outer, vE = C.one[par] ? outer : B[z];
         const float vB = z > 0 ? B[z > 0 ? z - 1 : 0] : zlo;
         const float vT = z < R - 1 ? B[z < R - 1 ? z + 1 : 0] : zhi;
-        const float wB = z == 0 ? L.wz0 : L.wi, wT = z == R - 1 ? L.wz1 : L.wi;
         const int zk = z == 0 ? 0 : (z == R - 1 ? 2 : 1);
-        float Ax = ufma(C.cW[par], vW, umul(C.cE[par], vE));
-        Ax = ufma(C.wS, vS, Ax);
-        Ax = ufma(C.wN, vN, Ax);
-        Ax = ufma(wB, vB, Ax);
-        Ax = ufma(wT, vT, Ax);
-        Ax = ufma(C.diag[par][zk], A[z], Ax);
-        const float v = ufma(omega, umul(b[z] - Ax, C.rcp[par][zk]), A[z]);
-        An[z] = (fl >> (2 * z + CLS)) & 1u ? v : A[z];
+        float w[6] = {C.cW[par], C.cE[par], C.wS, C.wN, z == 0 ? L.wz0 : L.wi, z == R - 1 ? L.wz1 : L.wi};
+        float diag = C.diag[par][zk], rcp = C.rcp[par][zk];
+        bool on = (fl >> (2 * z + CLS)) & 1u;
+        if (GEN) {
+            asm volatile("" ::: "memory");  // one height's weights at a time: all at once would spill
+            const float *fx = C.face[0] + C.one[par], *fy = C.face[1] + C.one[par], *fz = C.face[2] + C.one[par];
+            w[0] = fx[(R + 1) * R * z];
+            w[1] = fx[(R + 1) * R * z + 1];
+            w[2] = fy[R * (R + 1) * z];
+            w[3] = fy[R * (R + 1) * z + R];
+            w[4] = fz[R * R * z];
+            w[5] = fz[R * R * z + R * R];
+            diag = -(w[0] + w[1] + w[2] + w[3] + w[4] + w[5]);
+            rcp = urcp(diag);
+            on = on && !(fabsf(diag) < 1e-9f);
+        }
+        float Ax = ufma(w[0], vW, umul(w[1], vE));
+        Ax = ufma(w[2], vS, Ax);
+        Ax = ufma(w[3], vN, Ax);
+        Ax = ufma(w[4], vB, Ax);
+        Ax = ufma(w[5], vT, Ax);
+        Ax = ufma(diag, A[z], Ax);
+        const float v = ufma(omega, umul(b[z] - Ax, rcp), A[z]);
+        An[z] = on ? v : A[z];
     }
 #pragma unroll
     for (int z = 0; z < R; ++z) A[z] = An[z];
 }
 
-template <int R, bool HALF, int MODE, bool HC>
-__device__ __forceinline__ void uni_smooth_body(const UniView& V, int warp, const UX<HALF>& x, const UX<HC>& xc,
-                                                const float* __restrict__ bvec, float omega, int iters, int rev) {
+// the arguments of a smoothing launch
+template <bool HALF, bool HC>
+struct USmooth {
+    UniView V;
+    UX<HALF> x;
+    UX<HC> xc;
+    const float* b;
+    float omega;
+    int iters, rev;
+};
+template <int R, bool HALF, int MODE, bool HC, bool GEN>
+__device__ __forceinline__ void uni_smooth_body(const USmooth<HALF, HC>& K, int warp) {
     using G = UG<R>;
+    const UniView& V = K.V;
+    const UX<HALF> x = K.x;
+    const UX<HC> xc = K.xc;
+    const float* __restrict__ bvec = K.b;
+    const float omega = K.omega;
+    const int iters = K.iters, rev = K.rev;
     constexpr bool PO = MODE == UM_PROLONG_ALL || MODE == UM_PROLONG_OWN, PH = MODE == UM_PROLONG_ALL;
     constexpr bool ZO = MODE == UM_ZERO_ALL || MODE == UM_ZERO_OWN, ZH = MODE == UM_ZERO_ALL;
     using S = USrcX<HALF, HC>;
@@ -563,7 +610,7 @@ __device__ __forceinline__ void uni_smooth_body(const UniView& V, int warp, cons
             const float d = -(C.cW[par] + C.cE[par] + C.wS + C.wN + wB + wT);
             C.diag[par][k] = d;
             C.rcp[par][k] = urcp(d);
-            if (fabsf(d) < 1e-9f) {  // cut off from every neighbour: never updated
+            if (!L.general && fabsf(d) < 1e-9f) {  // cut off from every neighbour: never updated
                 uint32_t bits = 0;
 #pragma unroll
                 for (int z = 0; z < R; ++z)
@@ -572,10 +619,21 @@ __device__ __forceinline__ void uni_smooth_body(const UniView& V, int warp, cons
             }
         }
     }
+    if (GEN && V.general[warp]) {
+        C.face[0] = V.W.w[0] + L.foff(0) + (2 * L.xp + (R + 1) * L.y);
+        C.face[1] = V.W.w[1] + L.foff(1) + (2 * L.xp + R * L.y);
+        C.face[2] = V.W.w[2] + L.foff(2) + (2 * L.xp + R * L.y);
 #pragma unroll 1
-    for (int it = 0; it < iters; ++it) {
-        uni_sweep<R, 0>(L, C, E, O, bE, hx, H.hy[0], H.hz[0][0], H.hz[1][0], fl, omega);
-        uni_sweep<R, 1>(L, C, O, E, bO, hx, H.hy[1], H.hz[0][1], H.hz[1][1], fl, omega);
+        for (int it = 0; it < iters; ++it) {
+            uni_sweep<R, 0, GEN>(L, C, E, O, bE, hx, H.hy[0], H.hz[0][0], H.hz[1][0], fl, omega);
+            uni_sweep<R, 1, GEN>(L, C, O, E, bO, hx, H.hy[1], H.hz[0][1], H.hz[1][1], fl, omega);
+        }
+    } else {
+#pragma unroll 1
+        for (int it = 0; it < iters; ++it) {
+            uni_sweep<R, 0, false>(L, C, E, O, bE, hx, H.hy[0], H.hz[0][0], H.hz[1][0], fl, omega);
+            uni_sweep<R, 1, false>(L, C, O, E, bO, hx, H.hy[1], H.hz[0][1], H.hz[1][1], fl, omega);
+        }
     }
     pdl_trigger();
     float v0[R], v1[R];
@@ -626,8 +684,13 @@ struct UHaloOne {
 // Blocks of one cell: a lane per block, six halo values.  The cell is black or red by its parity 0, so
 // every sweep updates it once.
 template <bool HALF, int MODE, bool HC>
-__device__ __forceinline__ void uni_smooth_one(const UniView& V, int warp, const UX<HALF>& x, const UX<HC>& xc,
-                                               const float* __restrict__ bvec, float omega, int iters) {
+__device__ __forceinline__ void uni_smooth_one(const USmooth<HALF, HC>& K, int warp) {
+    const UniView& V = K.V;
+    const UX<HALF> x = K.x;
+    const UX<HC> xc = K.xc;
+    const float* __restrict__ bvec = K.b;
+    const float omega = K.omega;
+    const int iters = K.iters;
     constexpr bool PO = MODE == UM_PROLONG_ALL || MODE == UM_PROLONG_OWN, PH = MODE == UM_PROLONG_ALL;
     constexpr bool ZO = MODE == UM_ZERO_ALL || MODE == UM_ZERO_OWN, ZH = MODE == UM_ZERO_ALL;
     using S = USrcX<HALF, HC>;
@@ -672,21 +735,23 @@ __device__ __forceinline__ void uni_smooth_one(const UniView& V, int warp, const
         default: ONE; break;        \
     }
 
-// One block colour of the block red-black smoother (the arithmetic of k_smooth) for uniform blocks.
+// One block colour of the block red-black smoother (the arithmetic of k_smooth).
+// GEN: the level has blocks that are not uniform; their warps (and the uniform blocks these share) read
+// every weight from memory.  An instance of its own: in one kernel the second body's addresses and weights
+// cost the common path registers (dam_drop_128 step 1.86 to 1.94 ms inlined, 1.92 ms as a call).
 // 4 CTAs per SM (128 registers a thread): the 8^3 body holds 16 cells, 16 right-hand sides and 28 halo
 // values per lane, and spills at 5 (96 registers; small-level launches 10 to 11 instead of 7.5 to 9.5 us).
-template <bool HALF, int MODE, bool HC>
-__global__ void __launch_bounds__(UNT, 4) k_uni_smooth(UniView V, UX<HALF> x, UX<HC> xc, const float* __restrict__ b,
-                                                       float omega, int iters, int rev) {
+template <bool HALF, int MODE, bool HC, bool GEN>
+__global__ void __launch_bounds__(UNT, 4) k_uni_smooth(const __grid_constant__ USmooth<HALF, HC> K) {
     const int w = blockIdx.x * UWARPS + (threadIdx.x >> 5);
-    if (w >= V.nwarp) {
+    if (w >= K.V.nwarp) {
         pdl_wait();
         return;
     }
-    const int warp = V.first + w;
-    const int r = V.desc[warp].y >> 8;
-#define AW_UB(R) uni_smooth_body<R, HALF, MODE, HC>(V, warp, x, xc, b, omega, iters, rev)
-    AW_UNI_RES(r, AW_UB, (uni_smooth_one<HALF, MODE, HC>(V, warp, x, xc, b, omega, iters)))
+    const int warp = K.V.first + w;
+    const int r = K.V.desc[warp].y >> 8;
+#define AW_UB(R) uni_smooth_body<R, HALF, MODE, HC, GEN>(K, warp)
+    AW_UNI_RES(r, AW_UB, (uni_smooth_one<HALF, MODE, HC>(K, warp)))
 #undef AW_UB
 }
 
@@ -753,9 +818,9 @@ __device__ __forceinline__ T uni_Ax(T diag, T v, T w0, T x0, T w1, T x1, T w2, T
 
 // r = b - A x of the lane's cells (bvec == nullptr: b = 0), 0 on air cells.  Returns the lane's partial
 // sum.
-template <int R, class S, bool DOT>
-__device__ __forceinline__ double uni_residual_body(const ULane<R>& L, UHalos<R, S, false>& H, const S& src,
-                                                    const float* __restrict__ bvec, const UOut& out, float sc) {
+template <int R, class S, bool DOT, bool GEN>
+__device__ __forceinline__ double uni_residual_body(const ULane<R>& L, const Coef3& W, bool general,
+                                                    UHalos<R, S, false>& H, const S& src, const float* __restrict__ bvec, const UOut& out, float sc) {
     using G = UG<R>;
     using T = typename S::T;
     double acc = 0.0;
@@ -810,13 +875,23 @@ __device__ __forceinline__ double uni_residual_body(const ULane<R>& L, UHalos<R,
         const T wB = z == 0 ? (T)L.wz0 : wi, wT = z == R - 1 ? (T)L.wz1 : wi;
         const float bv0 = bb0[z], bv1 = bb1[z];
         T r0 = T(0), r1 = T(0);
+        T w0[6] = {cW, wi, wS, wN, wB, wT}, w1[6] = {wi, cE, wS, wN, wB, wT};
+        if (GEN && general) {
+            float g[6];
+            L.weights(W, 0, z, g);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) w0[k] = g[k];
+            L.weights(W, 1, z, g);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) w1[k] = g[k];
+        }
         if ((L.mask >> (2 * z)) & 1u) {
-            const T diag = -(cW + wi + wS + wN + wB + wT);
-            r0 = (T)bv0 - uni_Ax(diag, v0[z], cW, xm, wi, v1[z], wS, s0, wN, n0, wB, b0, wT, t0);
+            const T diag = -(w0[0] + w0[1] + w0[2] + w0[3] + w0[4] + w0[5]);
+            r0 = (T)bv0 - uni_Ax(diag, v0[z], w0[0], xm, w0[1], v1[z], w0[2], s0, w0[3], n0, w0[4], b0, w0[5], t0);
         }
         if ((L.mask >> (2 * z + 1)) & 1u) {
-            const T diag = -(wi + cE + wS + wN + wB + wT);
-            r1 = (T)bv1 - uni_Ax(diag, v1[z], wi, v0[z], cE, xq, wS, s1, wN, n1, wB, b1, wT, t1);
+            const T diag = -(w1[0] + w1[1] + w1[2] + w1[3] + w1[4] + w1[5]);
+            r1 = (T)bv1 - uni_Ax(diag, v1[z], w1[0], v0[z], w1[1], xq, w1[2], s1, w1[3], n1, w1[4], b1, w1[5], t1);
         }
         if (L.live) {
             if (out.r) ustore2(out.r, i, L.even, (float)r0, (float)r1);
@@ -906,8 +981,9 @@ __device__ __forceinline__ void last_cta_sum(double v, double* part, unsigned* t
 
 // r = b - A x on a V-cycle level (FP32 or FP16 x): to r, or restricted into the coarse right-hand side,
 // with an optional sum of r^2 into *sum.
-template <bool HALF>
-__global__ void __launch_bounds__(UNT, 4) k_uni_residual(UniView V, UX<HALF> x, const float* __restrict__ b, UOut out,
+template <bool HALF, bool GEN>
+__global__ void __launch_bounds__(UNT, 4) k_uni_residual(const __grid_constant__ UniView V, UX<HALF> x,
+                                                         const float* __restrict__ b, const __grid_constant__ UOut out,
                                                          double* part, unsigned* ticket, double* sum) {
     const int w = blockIdx.x * UWARPS + (threadIdx.x >> 5);
     double acc = 0.0;
@@ -925,7 +1001,8 @@ __global__ void __launch_bounds__(UNT, 4) k_uni_residual(UniView V, UX<HALF> x, 
         H.init(L);                                                                                    \
         pdl_wait();                                                                                   \
         waited = true;                                                                                \
-        if (any) acc = uni_residual_body<R, S, false>(L, H, src, b, out, x.sc(L.block));              \
+        if (any)                                                                                      \
+            acc = uni_residual_body<R, S, false, GEN>(L, V.W, GEN && V.general[warp], H, src, b, out, x.sc(L.block)); \
     }
 #define AW_UB1                                                                     \
     {                                                                              \
@@ -950,7 +1027,7 @@ __global__ void __launch_bounds__(UNT, 4) k_uni_residual(UniView V, UX<HALF> x, 
 // gradients: q = -A d with d = z + beta d_old formed where it is read (own cells and halo), stored as the
 // new direction, and d . q (k_uni_apply).  The direction alternates between two buffers, since a
 // neighbour's halo still reads the old one.
-template <class S, bool DOT, class F>
+template <class S, bool DOT, bool GEN, class F>
 __device__ __forceinline__ double uni_residual64(const UniView& V, S& src, const float* b, UOut& out, F begin) {
     const int w = blockIdx.x * UWARPS + (threadIdx.x >> 5);
     double acc = 0.0;
@@ -968,7 +1045,8 @@ __device__ __forceinline__ double uni_residual64(const UniView& V, S& src, const
         H.init(L);                                                        \
         pdl_wait();                                                       \
         begin();                                                          \
-        if (any) acc = uni_residual_body<R, S, DOT>(L, H, src, b, out, 1.f); \
+        if (any)                                                          \
+            acc = uni_residual_body<R, S, DOT, GEN>(L, V.W, GEN && V.general[warp], H, src, b, out, 1.f); \
     }
 #define AW_UB1                                                            \
     {                                                                     \
@@ -985,17 +1063,20 @@ __device__ __forceinline__ double uni_residual64(const UniView& V, S& src, const
 #undef AW_UB1
     return acc;
 }
-__global__ void __launch_bounds__(UNT, 3) k_uni_residual64(UniView V, USrcD src, const float* __restrict__ b, UOut out,
+template <bool GEN>
+__global__ void __launch_bounds__(UNT, 3) k_uni_residual64(const __grid_constant__ UniView V, USrcD src,
+                                                           const float* __restrict__ b, UOut out,
                                                            double* part, unsigned* ticket, double* sum) {
-    const double acc = uni_residual64<USrcD, false>(V, src, b, out, []() {});
+    const double acc = uni_residual64<USrcD, false, GEN>(V, src, b, out, []() {});
     last_cta_sum(acc, part, ticket, [&](double t) { *sum = t; });
 }
 // sc = {rho, rho_old}, st = {iterations, restart}: d1 becomes the direction in even iterations, d0 in odd
-__global__ void __launch_bounds__(UNT, 3) k_uni_apply(UniView V, const float* __restrict__ z, double* d0, double* d1,
+template <bool GEN>
+__global__ void __launch_bounds__(UNT, 3) k_uni_apply(const __grid_constant__ UniView V, const float* __restrict__ z, double* d0, double* d1,
                                                       UOut out, const double* __restrict__ sc, const int* __restrict__ st,
                                                       double* part, unsigned* ticket, double* sum) {
     USrcDir src{z, d0, 0.0, true};
-    const double acc = uni_residual64<USrcDir, true>(V, src, nullptr, out, [&]() {
+    const double acc = uni_residual64<USrcDir, true, GEN>(V, src, nullptr, out, [&]() {
         const bool odd = (st[0] & 1) != 0;
         src.first = st[1] != 0;
         src.beta = src.first ? 0.0 : sc[0] / sc[1];
@@ -1011,9 +1092,8 @@ __global__ void __launch_bounds__(UNT, 3) k_uni_apply(UniView V, const float* __
 // ------------------------------------------------------------------------------------------------
 // A block is uniform when every face between two of its cells has one conductance and every side of
 // the block has one; a block without fluid takes no part (its x is set to 0, which its neighbours
-// read).  counts[0] += blocks that are neither.
+// read).
 struct UCheck {
-    Coef3 W;
     const uint8_t* fluid;
     float* x;       // FP32 storage of the level's x to clear in air blocks (nullptr: keep)
     __half* xh;     // FP16 storage
@@ -1021,7 +1101,8 @@ struct UCheck {
     double *d0, *d1;  // FP64 vectors to clear there too
     float4* wt;
     uint16_t* mask;
-    int* counts;
+    uint8_t* general;
+    int* count;     // += blocks that are not uniform
 };
 constexpr int UNI_MAX_LEVELS = 4;  // 8^3 blocks halve to one cell in three steps
 struct UCheckAll {
@@ -1055,9 +1136,9 @@ __device__ __forceinline__ void uni_check_body(const UniView& V, const UCheck& K
     // weights
     constexpr int nf = (R + 1) * R * R;
     const uint32_t f0 = (uint32_t)rec[22], f1 = (uint32_t)rec[23], f2 = (uint32_t)rec[24];
-    const float* w0 = K.W.w[0] + f0;
-    const float* w1 = K.W.w[1] + f1;
-    const float* w2 = K.W.w[2] + f2;
+    const float* w0 = V.W.w[0] + f0;
+    const float* w1 = V.W.w[1] + f1;
+    const float* w2 = V.W.w[2] + f2;
     const float wx0 = w0[0], wx1 = w0[R], wy0 = w1[0], wy1 = w1[R * R], wz0 = w2[0], wz1 = w2[R * R * R];
     const float wi = R >= 2 ? w0[1] : wx0;
     // UB values of each axis in flight per lane (one at a time, 54 dependent round trips of an 8^3 block took
@@ -1097,12 +1178,16 @@ __device__ __forceinline__ void uni_check_body(const UniView& V, const UCheck& K
             }
         if (K.xh && li == 0) K.scale[rec[1]] = 0.f;
     }
+    // (the six faces of one cell are its six sides)
+    const unsigned gen = __ballot_sync(0xffffffffu, R > 1 && valid && li == 0 && state == US_GENERAL);
+    if (lane == 0) {
+        K.general[warp] = gen != 0;
+        if (gen) atomicAdd(K.count, __popc(gen));
+    }
     if (valid && li == 0) {
         K.wt[2 * (size_t)slot] = make_float4(wi, wx0, wx1, wy0);
         K.wt[2 * (size_t)slot + 1] = make_float4(wy1, wz0, wz1, __int_as_float(state));
     }
-    const unsigned gen = __ballot_sync(0xffffffffu, valid && li == 0 && state == US_GENERAL);
-    if (lane == 0 && gen) atomicAdd(K.counts, __popc(gen));
 }
 // level = blockIdx.y
 __global__ void __launch_bounds__(UNT) k_uni_check(const __grid_constant__ UCheckAll A) {

@@ -145,3 +145,67 @@ def test_fluid_flags_change_between_solves():
         assert not p[fluid == 0].any()
     sv.close()
     g.close()
+
+
+@pytest.mark.parametrize("name", ["row", "odd", "hole"])
+@pytest.mark.parametrize("precision", [aw.PRECISION_FP32, aw.PRECISION_FP32_PCG])
+def test_varying_coefficients(name, precision):
+    """Every face its own 1/rho (a stirred two-phase interface): every block reads its weights."""
+    dims, lv = MAPS[name]
+    g = _grid(dims, lv)
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    n = g.totals()[0]
+    for a in range(3):
+        beta = g.channel(aw.BETA_COEFF_X + a)
+        beta.copy_(0.3 + 0.7 * torch.rand(beta.numel(), generator=gen, device="cuda"))
+    fluid = (g.face_positions(3)[:, 0] < 0.7 * dims[0]).to(torch.uint8)
+    b = torch.randn(n, generator=gen, device="cuda") * fluid
+    a = _solve(g, True, precision, fluid, b, 1e-30, max_cycles=2)
+    s = _solve(g, False, precision, fluid, b, 1e-30, max_cycles=2)
+    assert all(_same(x[2], y[2]) for x, y in zip(a, s))
+    g.close()
+
+
+@pytest.mark.parametrize("precision", [aw.PRECISION_FP32, aw.PRECISION_MIXED])
+def test_vcycle_call(precision):
+    """aw_vcycle_run from a given x: register-resident against staged, launched, replayed and captured."""
+    dims, lv = MAPS["odd"]
+    g = _grid(dims, lv)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    n = g.totals()[0]
+    fluid = (g.face_positions(3)[:, 1] < 2.2).to(torch.uint8)
+    b = torch.randn(n, generator=gen, device="cuda") * fluid
+    x0 = torch.randn(n, generator=gen, device="cuda")  # air cells too: their values are the neighbours' ghosts
+
+    def cycles(uniform, capture):
+        sv = _solver(g, uniform, precision=precision)
+        sv.setup(fluid)
+        x, bb = sv.level_array(0, 0), sv.level_array(0, 1)
+        x.copy_(x0)
+        bb.copy_(b)
+        torch.cuda.synchronize()
+        if capture:
+            s = torch.cuda.Stream()
+            with torch.cuda.stream(s):
+                sv.vcycle()
+                s.synchronize()
+                x.copy_(x0)
+                G = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(G, stream=s):
+                    sv.vcycle(stream=torch.cuda.current_stream().cuda_stream)
+                G.replay()
+                G.replay()
+                s.synchronize()
+            del G
+        else:
+            sv.vcycle()
+            sv.vcycle()
+        torch.cuda.synchronize()
+        out = x.cpu().clone()
+        sv.close()
+        return out
+
+    ref = cycles(False, False)
+    assert torch.equal(cycles(True, False), ref)
+    assert torch.equal(cycles(True, True), ref)
+    g.close()
