@@ -145,14 +145,6 @@ __global__ void k_wall_bc(LevelView L, float* u0, float* u1, float* u2) {
     }
 }
 
-__global__ void k_fluid_from_count(const uint32_t* __restrict__ cstart, uint32_t nc, uint8_t* fluid, float* count) {
-    uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nc) return;
-    uint32_t k = cstart[c + 1] - cstart[c];
-    fluid[c] = k > 0;
-    if (count) count[c] = (float)k;
-}
-
 __device__ inline void atomic_max_pos(float* addr, float v) {
     atomicMax((int*)addr, __float_as_int(v));  // v >= 0
 }
@@ -646,10 +638,9 @@ aw_status flip_step_soa(MsbgState& G, aw_solver* solver, const aw_flip_desc& d, 
             pin.beta[a] = G.ch[AW_BETA_COEFF_X + a];
         }
     }
-    AW_TRY(p2g_sorted(G, soa_out, n, G.pw.cell_start.p, U, Mm, nomom, nullptr, s, fp ? &pin : nullptr));
+    AW_TRY(p2g_sorted(G, soa_out, n, G.pw.cell_start.p, U, Mm, nomom, G.ch[AW_CELL_TYPE], s, fp ? &pin : nullptr,
+                      B.fluid.p));
     if (ev) AW_CUDA(cudaEventRecord(ev[2], s));
-    k_fluid_from_count<<<nblk(G.tot[0]), 256, 0, s>>>(G.pw.cell_start.p, G.tot[0], B.fluid.p, G.ch[AW_CELL_TYPE]);
-    AW_LAUNCH();
     if (fluid_in) AW_TRY(copy_d2d(B.fluid.p, fluid_in, G.tot[0], s));
     if (rec) {
         for (int a = 0; a < 3; ++a) {

@@ -113,6 +113,46 @@ aw_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, DBuf<u
     return AW_OK;
 }
 
+aw_status clear_faces(const MsbgState& G, float* const* arrays, int triplets, cudaStream_t s) {
+    const float *lo = G.slab.p, *hi = G.slab.p + G.slab.n;
+    float* at = nullptr;
+    float* end = nullptr;  // the run [at, end) still to clear
+    auto flush = [&]() -> aw_status {
+        if (end > at) AW_CUDA(cudaMemsetAsync(at, 0, (size_t)(end - at) * sizeof(float), s));
+        return AW_OK;
+    };
+    for (int k = 0; k < 3 * triplets; ++k) {
+        float* p = arrays[k];
+        const uint32_t n = G.tot[1 + k % 3];
+        if (!n) continue;
+        // the next channel of the slab: the padding between is the slab's own
+        if (at && p >= end && p < end + 64 && at >= lo && p + n <= hi) {
+            end = p + n;
+            continue;
+        }
+        AW_TRY(flush());
+        at = p;
+        end = p + n;
+    }
+    return flush();
+}
+aw_status copy_faces(const MsbgState& G, float* const dst[3], float* const src[3], cudaStream_t s) {
+    const float *lo = G.slab.p, *hi = G.slab.p + G.slab.n;
+    const bool one = G.tot[1] && G.tot[2] && G.tot[3] && src[0] >= lo && dst[0] >= lo && src[2] + G.tot[3] <= hi &&
+                     dst[2] + G.tot[3] <= hi && src[2] > src[1] && src[1] > src[0] &&
+                     src[1] - src[0] == dst[1] - dst[0] && src[2] - src[0] == dst[2] - dst[0] &&
+                     src[1] - src[0] < (ptrdiff_t)G.tot[1] + 64 && src[2] - src[1] < (ptrdiff_t)G.tot[2] + 64;
+    if (one) {
+        AW_CUDA(cudaMemcpyAsync(dst[0], src[0], ((size_t)(src[2] - src[0]) + G.tot[3]) * sizeof(float),
+                                cudaMemcpyDeviceToDevice, s));
+        return AW_OK;
+    }
+    for (int a = 0; a < 3; ++a)
+        if (G.tot[1 + a])
+            AW_CUDA(cudaMemcpyAsync(dst[a], src[a], G.tot[1 + a] * sizeof(float), cudaMemcpyDeviceToDevice, s));
+    return AW_OK;
+}
+
 // ------------------------------------------------------------------------------------------------
 // Level map kernels
 // ------------------------------------------------------------------------------------------------

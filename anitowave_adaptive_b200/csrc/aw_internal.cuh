@@ -186,7 +186,7 @@ struct ParticleWork {
     // The particle arrays the last aw_p2g sorted (caller pointers and count) and 64-bit hashes of
     // their contents then: hash[0] positions, hash[1] velocities; hash[2..3] receive the hashes of
     // the arrays at a later drop-in G2P or advection, which reuses this sort when they match;
-    // hash[4..] holds the partial sums of the hashing kernels.
+    // hash[4..] holds the partial sums of the hashing kernels and their CTA ticket (0 between them).
     const float* src_pos = nullptr;
     const float* src_vel = nullptr;
     int64_t src_n = -1;
@@ -235,7 +235,7 @@ struct MsbgState {
     bool blk_order_on = false;  // blk_order holds this step's order (small grids only)
     DBuf<float> tiles_bar_new, tiles_bar_old;  // adjoint tiles (VJP kernels)
     DBuf<float> adj_u[3], adj_m[3];             // forward P2G recomputed by aw_vjp_p2g
-    DBuf<float> p2g_P[3];                       // P2G momentum accumulator when MOMENTUM_* is not asked for
+    DBuf<float> p2g_P;                          // P2G momentum accumulators (x, y, z) when MOMENTUM_* is not asked for
     DBuf<float> p2g_Phi[3];                     // P2G phase accumulator (two-phase P2G)
     DBuf<int> lattice_tab;                      // per-axis lookup tables of aw_resample_cells
     FlipBufs proj;                              // aw_project / aw_vjp_project work buffers
@@ -268,6 +268,11 @@ aw_status relevel_on_device(MsbgState& G, const float* d_pos, int64_t si, int64_
 // the storage it already holds where the new levels fit, and sets it up with every cell fluid.
 aw_status solver_relayout(aw_solver* S);
 
+// Clears / copies a face-channel triplet (tot[1 + a] floats each) in as few calls as it has contiguous
+// runs: the channels of the grid's slab follow one another (padded to 64 floats), so a triplet is one.
+aw_status clear_faces(const MsbgState& G, float* const* arrays, int triplets, cudaStream_t s);
+aw_status copy_faces(const MsbgState& G, float* const dst[3], float* const src[3], cudaStream_t s);
+
 // Exclusive scan of n u32 values into out[0..n] (out[n] = total).  tmp: scan scratch.
 aw_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, DBuf<uint32_t>& tmp, cudaStream_t s);
 
@@ -285,7 +290,8 @@ struct PhaseIn {
     float* beta[3];
 };
 aw_status p2g_sorted(MsbgState& G, const float* soa, int64_t n, const uint32_t* cell_start, float* u[3], float* m[3],
-                     float* mom[3], float* cell_count, cudaStream_t s, const PhaseIn* ph = nullptr);
+                     float* mom[3], float* cell_count, cudaStream_t s, const PhaseIn* ph = nullptr,
+                     uint8_t* fluid = nullptr);  // fluid: 1 where a cell holds a particle
 // beta at T-junctions: the coarse face and the 4 fine faces it covers all take the mean of the
 // 4 fine values, which keeps the finite-volume operator symmetric for variable coefficients
 aw_status beta_sync(MsbgState& G, float* beta[3], cudaStream_t s);
