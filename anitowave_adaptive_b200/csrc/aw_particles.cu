@@ -2281,8 +2281,8 @@ aw_status advect_sorted(MsbgState& G, float* soa, int64_t n, const uint32_t* cs,
     int maxres = 0;
     for (int r : G.h_res) maxres = std::max(maxres, r);
     const size_t smem = (size_t)tile_block(maxres) * sizeof(float);
-    if (smem > 48 * 1024)
-        AW_CUDA(cudaFuncSetAttribute(k_advect_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // (always set: a grid of smaller blocks may have lowered it)
+    AW_CUDA(cudaFuncSetAttribute(k_advect_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_advect_tile<<<G.nb, 256, smem, s>>>(G.view0(), soa, n, cs, dt, G.tile_off.p, G.tiles_new.p, G.err.p + 1,
                                           DropIn{nullptr, nullptr, nullptr}, G.blk_busy.p ? G.tile_ok.p : nullptr,
                                           Field3{{un[0], un[1], un[2]}}, G.blk_order_on ? G.blk_order.p : nullptr);

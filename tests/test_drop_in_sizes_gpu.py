@@ -64,3 +64,29 @@ def test_drop_in_calls(n, off, change):
     tol = 8 * EPS + dt * 3 * 108 * EPS * umax * (1 + 2 * dt * umax / h) ** 2
     assert float((pos - pos2).abs().max()) <= tol
     g.close()
+
+
+def test_small_blocks_do_not_change_later_steps():
+    """A FLIP step on 8-cell blocks after an advection of a grid of 4-cell blocks (smaller shared tiles)."""
+    def step():
+        g = _grid((2, 2, 2), 8, 1)
+        g.set_refinement_map(np.zeros(8, np.uint32))
+        g.allocate()
+        gen = torch.Generator(device="cuda").manual_seed(1)
+        pos = torch.rand((2000, 3), generator=gen, device="cuda") * torch.tensor([0.9, 0.4, 0.9], device="cuda") + 0.02
+        vel = torch.randn((2000, 3), generator=gen, device="cuda") * 0.1
+        sim = aw.Flip(g, pos.cpu().numpy(), vel.cpu().numpy(), 0.01)
+        sim.step()
+        out = sim.particles()[0]
+        sim.close()
+        g.close()
+        return out
+
+    h = _grid((2, 2, 2), 4, 1)
+    p = torch.rand((100, 3), device="cuda")
+    v = torch.zeros_like(p)
+    h.p2g(p, v)
+    h.advect(p, 0.01)
+    h.close()
+    out = step()
+    assert bool(np.isfinite(np.asarray(out)).all())
