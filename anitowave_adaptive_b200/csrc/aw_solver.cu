@@ -123,6 +123,7 @@ struct aw_solver {
     aw::DBuf<double> cgprm;
     bool use_graph = true;
     bool use_pdl = true;  // V-cycle kernels as programmatic dependent launches
+    int low = 1 << 30;    // first level of those that k_uni_low walks
     int tail = 0;         // first level of the uniform tail run as one k_dense_tail launch (0: none)
     double* h_norm = nullptr;  // pinned host words: a squared norm, uniform_check's counts
     double* h_cg = nullptr;    // pinned host words of the device-loop state
@@ -2369,6 +2370,10 @@ static aw_status build_uniform(aw_solver* S, cudaStream_t s) {
                                                 reinterpret_cast<int*>(L.urec));
         AW_LAUNCH();
     }
+    // the levels that k_uni_low walks (AW_NO_UNIFORM_LOW keeps a launch per step)
+    S->low = nl - 1;
+    if (getenv("AW_NO_UNIFORM_LOW") == nullptr)
+        while (S->low > 0 && S->lv[S->low - 1].uwarps[0] + S->lv[S->low - 1].uwarps[1] <= ULOW_WARPS) --S->low;
     return AW_OK;
 }
 
@@ -2469,6 +2474,49 @@ static aw_status uni_residual(aw_solver* S, int m, const XStore& x, const float*
                       ux<false>(x), b, out, S->partials.p, S->ticket.p, sum);
 }
 
+// Levels m .. and below as one launch of k_uni_low (or two around the coarser part); S->low <= m.
+static aw_status uni_vcycle(aw_solver* S, int m, bool zero, cudaStream_t s);
+static aw_status uni_low(aw_solver* S, int m, bool zero, cudaStream_t s) {
+    const int end = S->nmsbg - 1;  // the level below the walk
+    ULow K{};
+    bool gen = false;
+    for (int k = m; k <= end; ++k) {
+        MGLevel& L = S->lv[k];
+        const XStore x = xstore(S, k);
+        K.lv[k] = ULowLevel{uview(L, 2), L.uwarps[0], x.f, x.h, x.scale, bptr(S, k), UOut{}};
+        if (k < end) {
+            K.lv[k].out.bc = S->lv[k + 1].b.p;
+            K.lv[k].out.fluid_c = S->lv[k + 1].fluid.p;
+            gen = gen || ((S->gen >> k) & 1u);
+        }
+    }
+    K.first = m;
+    K.last = end - 1;
+    K.pre = S->d.pre_smooth;
+    K.post = S->d.post_smooth;
+    K.iters = (int)S->d.block_iterations;
+    K.omega = S->d.omega;
+    K.zero = zero;
+    K.exact = S->exact && end == (int)S->lv.size() - 1 && S->lv[end].ncell() <= (size_t)ULOW_EXACT && S->lv[end].maxres == 1;
+    if (K.exact) {
+        K.idx = S->ex_idx.p;
+        K.ex_n = S->ex_n.p;
+        K.Minv = S->Minv.p;
+        K.cell = S->lv[end].off[0].p;
+        K.xb = S->lv[end].b.p;
+    }
+    auto launch = [&](bool down, bool up) {
+        K.down = down;
+        K.up = up;
+        return launch_dep(S, gen ? k_uni_low<true> : k_uni_low<false>, 1, ULOW_THREADS, 0, s, K);
+    };
+    if (K.exact) return launch(true, true);
+    AW_TRY(launch(true, false));
+    if (S->tail && end == S->tail) AW_TRY(dense_tail(S, s));
+    else AW_TRY(uni_vcycle(S, end, true, s));
+    return launch(false, true);
+}
+
 // The V-cycle by the register-resident kernels: the steps of vcycle() with the
 // residual restricted as it is taken, levels starting at zero without a clearing pass (zero: this
 // level does), and the correction of an FP32 level added where its first post-smoothing reads it.
@@ -2479,6 +2527,7 @@ static aw_status uni_vcycle(aw_solver* S, int m, bool zero, cudaStream_t s) {
         if (zero) AW_TRY(zero_x(S, m, s));
         return vcycle(S, m, s);
     }
+    if (m >= S->low && m < S->nmsbg - 1) return uni_low(S, m, zero, s);
     if (zero && S->d.pre_smooth == 0) AW_TRY(zero_x(S, m, s));
     for (int it = 0; it < S->d.pre_smooth; ++it)
         for (int k = 0; k < 2; ++k) {

@@ -402,8 +402,8 @@ struct USrcDir {
 };
 
 // Store the block: FP32, or FP16 with a fresh per-block scale.  v0/v1: the pair at every z.
-template <int R, bool HALF>
-__device__ __forceinline__ void uni_store(const ULane<R>& L, const UX<HALF>& x, const float* v0, const float* v1) {
+template <int R, bool HALF, bool KEEP = false>  // KEEP: v0, v1 become the values as read back
+__device__ __forceinline__ void uni_store(const ULane<R>& L, const UX<HALF>& x, float* v0, float* v1) {
     using G = UG<R>;
     if (!HALF) {
         if (!L.live) return;
@@ -423,23 +423,25 @@ __device__ __forceinline__ void uni_store(const ULane<R>& L, const UX<HALF>& x, 
 #pragma unroll
     for (int o = 1; o < G::LPB; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if (!L.live) return;
-    const float inv = m > 0.f ? 32768.f / m : 0.f;
+    const float inv = m > 0.f ? 32768.f / m : 0.f, scale = m > 0.f ? m * (1.f / 32768.f) : 0.f;
 #pragma unroll
     for (int z = 0; z < R; ++z) {
         const uint32_t i = L.at + (uint32_t)(R * R * z);
         const __half a = __float2half_rn(v0[z] * inv);
+        if (KEEP) v0[z] = umul(__half2float(a), scale);
         if (G::NI == 1) {
             x.h[i] = a;
             continue;
         }
         const __half b = __float2half_rn(v1[z] * inv);
+        if (KEEP) v1[z] = umul(__half2float(b), scale);
         if (L.even) *reinterpret_cast<__half2*>(x.h + i) = __halves2half2(a, b);
         else {
             x.h[i] = a;
             x.h[i + 1] = b;
         }
     }
-    if (L.lane % G::LPB == 0) x.scale[L.block] = m > 0.f ? m * (1.f / 32768.f) : 0.f;
+    if (L.lane % G::LPB == 0) x.scale[L.block] = scale;
 }
 
 // How a smoothing launch meets its input:
@@ -511,6 +513,84 @@ __device__ __forceinline__ void uni_sweep(const ULane<R>& L, const UCoef<R>& C, 
     for (int z = 0; z < R; ++z) A[z] = An[z];
 }
 
+// The halo of a block by colour class: hx by height (R = 2: by height and class, the pair being the whole
+// row), hy and hz by class.
+template <int R, class HS, class S>
+__device__ __forceinline__ void uni_halo(const ULane<R>& L, HS& H, const S& src, int q, float (&hx)[R == 2 ? 4 : R]) {
+    // R - 1 is odd, so the classes of the plane above the block are swapped
+    H.load(L, src, [&](int k, int z) { return 2 * L.xp + ((q ^ z ^ k) & 1); },
+           [&](int side, int k) { return 2 * L.xp + ((q ^ k ^ side) & 1); });
+#pragma unroll
+    for (int z = 0; z < R; ++z) {
+        if (R == 2) {
+            const bool one = ((q ^ z) & 1) != 0;
+            const float lo = H.hx[z], hi = H.hx[R == 2 ? R + z : z];
+            hx[R == 2 ? 2 * z : z] = one ? hi : lo;
+            hx[R == 2 ? 2 * z + 1 : z] = one ? lo : hi;
+        } else {
+            hx[z] = H.hx[z];
+        }
+    }
+}
+// The lane's weights and the fluid bits by class (those of cells cut off from every neighbour cleared).
+template <int R>
+__device__ __forceinline__ void uni_coef(const ULane<R>& L, int q, UCoef<R>& C, uint32_t& fl) {
+    using G = UG<R>;
+    // swap the two bits of every height whose E cell is the pair's second
+    const uint32_t sw = ((L.mask & 0x5555u) << 1) | ((L.mask >> 1) & 0x5555u);
+    const uint32_t selm = q ? 0x3333u : 0xCCCCu;
+    fl = (L.mask & ~selm) | (sw & selm);
+    C.wS = L.y == 0 ? L.wy0 : L.wi;
+    C.wN = L.y == R - 1 ? L.wy1 : L.wi;
+#pragma unroll
+    for (int par = 0; par < 2; ++par) {
+        const bool one = ((q ^ par) & 1) != 0;
+        C.one[par] = one;
+        C.edge[par] = one ? L.xp == G::XP - 1 : L.xp == 0;
+        C.src[par] = one ? L.lane + 1 : L.lane - 1;
+        C.cW[par] = !one && L.xp == 0 ? L.wx0 : L.wi;
+        C.cE[par] = one && L.xp == G::XP - 1 ? L.wx1 : L.wi;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float wB = k == 0 ? L.wz0 : L.wi, wT = k == 2 ? L.wz1 : L.wi;
+            const float d = -(C.cW[par] + C.cE[par] + C.wS + C.wN + wB + wT);
+            C.diag[par][k] = d;
+            C.rcp[par][k] = urcp(d);
+            if (!L.general && fabsf(d) < 1e-9f) {  // never updated
+                uint32_t bits = 0;
+#pragma unroll
+                for (int z = 0; z < R; ++z)
+                    if ((z == 0 ? 0 : (z == R - 1 ? 2 : 1)) == k) bits |= 1u << (2 * z + ((z ^ par) & 1));
+                fl &= ~bits;
+            }
+        }
+    }
+}
+template <int R>
+__device__ __forceinline__ void uni_faces(const ULane<R>& L, const Coef3& W, UCoef<R>& C) {
+    C.face[0] = W.w[0] + L.foff(0) + (2 * L.xp + (R + 1) * L.y);
+    C.face[1] = W.w[1] + L.foff(1) + (2 * L.xp + R * L.y);
+    C.face[2] = W.w[2] + L.foff(2) + (2 * L.xp + R * L.y);
+}
+template <int R, bool GEN, class HS>
+__device__ __forceinline__ void uni_iterate(const ULane<R>& L, const UCoef<R>& C, float (&E)[R], float (&O)[R],
+                                            const float (&bE)[R], const float (&bO)[R], const float (&hx)[R == 2 ? 4 : R],
+                                            const HS& H, uint32_t fl, float omega, int iters, bool general) {
+    if (GEN && general) {
+#pragma unroll 1
+        for (int it = 0; it < iters; ++it) {
+            uni_sweep<R, 0, GEN>(L, C, E, O, bE, hx, H.hy[0], H.hz[0][0], H.hz[1][0], fl, omega);
+            uni_sweep<R, 1, GEN>(L, C, O, E, bO, hx, H.hy[1], H.hz[0][1], H.hz[1][1], fl, omega);
+        }
+    } else {
+#pragma unroll 1
+        for (int it = 0; it < iters; ++it) {
+            uni_sweep<R, 0, false>(L, C, E, O, bE, hx, H.hy[0], H.hz[0][0], H.hz[1][0], fl, omega);
+            uni_sweep<R, 1, false>(L, C, O, E, bO, hx, H.hy[1], H.hz[0][1], H.hz[1][1], fl, omega);
+        }
+    }
+}
+
 // the arguments of a smoothing launch
 template <bool HALF, bool HC>
 struct USmooth {
@@ -527,7 +607,7 @@ __device__ __forceinline__ void uni_smooth_body(const USmooth<HALF, HC>& K, int 
     const UniView& V = K.V;
     const UX<HALF> x = K.x;
     const UX<HC> xc = K.xc;
-    const float* __restrict__ bvec = K.b;
+    const float* bvec = K.b;
     const float omega = K.omega;
     const int iters = K.iters, rev = K.rev;
     constexpr bool PO = MODE == UM_PROLONG_ALL || MODE == UM_PROLONG_OWN, PH = MODE == UM_PROLONG_ALL;
@@ -566,7 +646,6 @@ __device__ __forceinline__ void uni_smooth_body(const USmooth<HALF, HC>& K, int 
         bE[z] = one ? bv.y : bv.x;
         bO[z] = one ? bv.x : bv.y;
     }
-    // halo: hx by height (R = 2: by height and class, the pair being the whole row), hy and hz by class
     float hx[R == 2 ? 4 : R];
     if (ZH) {
 #pragma unroll
@@ -574,67 +653,14 @@ __device__ __forceinline__ void uni_smooth_body(const USmooth<HALF, HC>& K, int 
         if (R == 2) hx[R == 2 ? 2 : 0] = hx[R == 2 ? 3 : 0] = 0.f;
         H.hz[0][0] = H.hz[0][1] = H.hz[1][0] = H.hz[1][1] = 0.f;
     } else {
-        // R - 1 is odd, so the classes of the plane above the block are swapped
-        H.load(L, src, [&](int k, int z) { return 2 * L.xp + ((q ^ z ^ k) & 1); },
-               [&](int side, int k) { return 2 * L.xp + ((q ^ k ^ side) & 1); });
-#pragma unroll
-        for (int z = 0; z < R; ++z) {
-            if (R == 2) {
-                const bool one = ((q ^ z) & 1) != 0;
-                const float lo = H.hx[z], hi = H.hx[R == 2 ? R + z : z];
-                hx[R == 2 ? 2 * z : z] = one ? hi : lo;
-                hx[R == 2 ? 2 * z + 1 : z] = one ? lo : hi;
-            } else {
-                hx[z] = H.hx[z];
-            }
-        }
+        uni_halo<R>(L, H, src, q, hx);
     }
-    // fluid bits by class: swap the two bits of every height whose E cell is the pair's second
-    const uint32_t sw = ((L.mask & 0x5555u) << 1) | ((L.mask >> 1) & 0x5555u);
-    const uint32_t selm = q ? 0x3333u : 0xCCCCu;
-    uint32_t fl = (L.mask & ~selm) | (sw & selm);
+    uint32_t fl;
     UCoef<R> C;
-    C.wS = L.y == 0 ? L.wy0 : L.wi;
-    C.wN = L.y == R - 1 ? L.wy1 : L.wi;
-#pragma unroll
-    for (int par = 0; par < 2; ++par) {
-        const bool one = ((q ^ par) & 1) != 0;
-        C.one[par] = one;
-        C.edge[par] = one ? L.xp == G::XP - 1 : L.xp == 0;
-        C.src[par] = one ? L.lane + 1 : L.lane - 1;
-        C.cW[par] = !one && L.xp == 0 ? L.wx0 : L.wi;
-        C.cE[par] = one && L.xp == G::XP - 1 ? L.wx1 : L.wi;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float wB = k == 0 ? L.wz0 : L.wi, wT = k == 2 ? L.wz1 : L.wi;
-            const float d = -(C.cW[par] + C.cE[par] + C.wS + C.wN + wB + wT);
-            C.diag[par][k] = d;
-            C.rcp[par][k] = urcp(d);
-            if (!L.general && fabsf(d) < 1e-9f) {  // cut off from every neighbour: never updated
-                uint32_t bits = 0;
-#pragma unroll
-                for (int z = 0; z < R; ++z)
-                    if ((z == 0 ? 0 : (z == R - 1 ? 2 : 1)) == k) bits |= 1u << (2 * z + ((z ^ par) & 1));
-                fl &= ~bits;
-            }
-        }
-    }
-    if (GEN && V.general[warp]) {
-        C.face[0] = V.W.w[0] + L.foff(0) + (2 * L.xp + (R + 1) * L.y);
-        C.face[1] = V.W.w[1] + L.foff(1) + (2 * L.xp + R * L.y);
-        C.face[2] = V.W.w[2] + L.foff(2) + (2 * L.xp + R * L.y);
-#pragma unroll 1
-        for (int it = 0; it < iters; ++it) {
-            uni_sweep<R, 0, GEN>(L, C, E, O, bE, hx, H.hy[0], H.hz[0][0], H.hz[1][0], fl, omega);
-            uni_sweep<R, 1, GEN>(L, C, O, E, bO, hx, H.hy[1], H.hz[0][1], H.hz[1][1], fl, omega);
-        }
-    } else {
-#pragma unroll 1
-        for (int it = 0; it < iters; ++it) {
-            uni_sweep<R, 0, false>(L, C, E, O, bE, hx, H.hy[0], H.hz[0][0], H.hz[1][0], fl, omega);
-            uni_sweep<R, 1, false>(L, C, O, E, bO, hx, H.hy[1], H.hz[0][1], H.hz[1][1], fl, omega);
-        }
-    }
+    uni_coef<R>(L, q, C, fl);
+    const bool general = GEN && V.general[warp];
+    if (general) uni_faces<R>(L, V.W, C);
+    uni_iterate<R, GEN>(L, C, E, O, bE, bO, hx, H, fl, omega, iters, general);
     pdl_trigger();
     float v0[R], v1[R];
 #pragma unroll
@@ -688,7 +714,7 @@ __device__ __forceinline__ void uni_smooth_one(const USmooth<HALF, HC>& K, int w
     const UniView& V = K.V;
     const UX<HALF> x = K.x;
     const UX<HC> xc = K.xc;
-    const float* __restrict__ bvec = K.b;
+    const float* bvec = K.b;
     const float omega = K.omega;
     const int iters = K.iters;
     constexpr bool PO = MODE == UM_PROLONG_ALL || MODE == UM_PROLONG_OWN, PH = MODE == UM_PROLONG_ALL;
@@ -820,7 +846,7 @@ __device__ __forceinline__ T uni_Ax(T diag, T v, T w0, T x0, T w1, T x1, T w2, T
 // sum.
 template <int R, class S, bool DOT, bool GEN>
 __device__ __forceinline__ double uni_residual_body(const ULane<R>& L, const Coef3& W, bool general,
-                                                    UHalos<R, S, false>& H, const S& src, const float* __restrict__ bvec, const UOut& out, float sc) {
+                                                    UHalos<R, S, false>& H, const S& src, const float* bvec, const UOut& out, float sc) {
     using G = UG<R>;
     using T = typename S::T;
     double acc = 0.0;
@@ -925,7 +951,7 @@ __device__ __forceinline__ double uni_residual_body(const ULane<R>& L, const Coe
 }
 template <class S, bool DOT>
 __device__ __forceinline__ double uni_residual_one(const ULane<1>& L, UHaloOne<S, false>& H, const S& src,
-                                                   const float* __restrict__ bvec, const UOut& out) {
+                                                   const float* bvec, const UOut& out) {
     using T = typename S::T;
     const T v = src.get(L.at, src.ctx(L.block));
     H.load(src);
@@ -1023,6 +1049,216 @@ __global__ void __launch_bounds__(UNT, 4) k_uni_residual(const __grid_constant__
     if (sum) last_cta_sum(acc, part, ticket, [&](double t) { *sum = t; });
 }
 
+// The V-cycle's small block-structured levels as one launch: one CTA walks levels first .. last down
+// (smoothing, restricted residual), applies the inverse of the coarsest operator where that is the next
+// level and small, and walks back up (prolongation, smoothing).  down / up alone: the legs around a coarser
+// part with launches of its own.  A warp keeps its blocks' cells, weights and addresses in registers for a
+// leg of a level and meets the others at CTA barriers; a colour's step then reads the halo, updates and
+// stores.  Every cell's arithmetic is that of the separate launches, bit for bit.
+// A level of at most ULOW_WARPS warps leaves most of the chip idle either way, and as launches its steps were
+// latency alone, 3.5 to 4 us a colour of 32 4^3 blocks, most of it the record, weight and halo-address chain
+// and the fetch of straight-line code that runs once: @.
+constexpr int UNI_MAX_LEVELS = 4;  // 8^3 blocks halve to one cell in three steps
+constexpr int ULOW_THREADS = 512;
+constexpr int ULOW_WARPS = ULOW_THREADS / 32;
+constexpr int ULOW_EXACT = 128;  // cells of a coarsest level taken along (its inverse comes from L2: 128 KB)
+struct ULowLevel {
+    UniView v;   // both colours
+    int n0;      // warps of colour 0
+    float* xf;
+    __half* xh;  // nullptr: FP32 storage
+    float* scale;
+    const float* b;
+    UOut out;    // restricted residual
+};
+struct ULow {
+    ULowLevel lv[UNI_MAX_LEVELS];  // lv[last + 1]: x of the level below
+    int first, last, pre, post, iters;
+    bool zero, down, up, exact;        // zero: level `first` starts from zero
+    float omega;
+    const int* idx;                    // the coarsest level's inverse
+    const int* ex_n;
+    const double* Minv;
+    const uint32_t* cell;              // cell offset of a block of the coarsest level
+    const float* xb;
+};
+// one warp's smoothing of one leg: 1 + ns barriers
+template <int R, bool HALF, bool GEN>
+__device__ __forceinline__ void uni_low_smooth(const ULow& K, const ULowLevel& l, const ULowLevel& c, int warp, int leg, bool zero) {
+    const int k = warp >= l.n0, ns = 2 * (leg ? K.post : K.pre);
+    const UX<HALF> x{l.xf, l.xh, l.scale};
+    using S = USrcX<HALF, false>;
+    const S src{x, UX<false>{nullptr, nullptr, nullptr}, false};
+    ULane<R> L;
+    UHalos<R, S, false> H;
+    const bool any = L.init(l.v, warp);
+    H.init(L);
+    const int q = (L.y & 1) ^ leg;
+    float E[R], O[R], bE[R], bO[R];
+    {
+        float v0[R], v1[R];
+        const bool moved = zero || leg;  // x changes before the first step
+        const float sc = zero || !L.live ? 1.f : x.sc(L.block);
+        const float scc = leg && c.xh && L.live ? c.scale[L.block] : 1.f;
+#pragma unroll
+        for (int z = 0; z < R; ++z) {
+            float2 v = make_float2(0.f, 0.f), bv = make_float2(0.f, 0.f);
+            if (L.live) {
+                const uint32_t i = L.at + (uint32_t)(R * R * z);
+                if (!zero) v = x.get2(i, sc, L.even);
+                uload2(l.b, i, L.even, bv.x, bv.y);
+                if (leg) {
+                    const uint32_t ci = L.coff + (uint32_t)(L.xp + (R / 2) * ((L.y >> 1) + (R / 2) * (z >> 1)));
+                    const float d = c.xh ? umul(__half2float(c.xh[ci]), scc) : c.xf[ci];
+                    if ((L.mask >> (2 * z)) & 1u) v.x += d;
+                    if ((L.mask >> (2 * z + 1)) & 1u) v.y += d;
+                }
+            }
+            v0[z] = v.x;
+            v1[z] = v.y;
+            const bool one = ((q ^ z) & 1) != 0;
+            bE[z] = one ? bv.y : bv.x;
+            bO[z] = one ? bv.x : bv.y;
+        }
+        if (moved && any) uni_store<R, HALF, true>(L, x, v0, v1);
+#pragma unroll
+        for (int z = 0; z < R; ++z) {
+            const bool one = ((q ^ z) & 1) != 0;
+            E[z] = one ? v1[z] : v0[z];
+            O[z] = one ? v0[z] : v1[z];
+        }
+    }
+    uint32_t fl;
+    UCoef<R> C;
+    uni_coef<R>(L, q, C, fl);
+    const bool general = GEN && l.v.general[warp];
+    if (general) uni_faces<R>(L, l.v.W, C);
+    __syncthreads();
+#pragma unroll 1
+    for (int st = 0; st < ns; ++st) {
+        if (((st ^ leg) & 1) == k && any) {
+            float hx[R == 2 ? 4 : R], v0[R], v1[R];
+            uni_halo<R>(L, H, src, q, hx);
+            uni_iterate<R, GEN>(L, C, E, O, bE, bO, hx, H, fl, K.omega, K.iters, general);
+#pragma unroll
+            for (int z = 0; z < R; ++z) {
+                const bool one = ((q ^ z) & 1) != 0;
+                v0[z] = one ? O[z] : E[z];
+                v1[z] = one ? E[z] : O[z];
+            }
+            uni_store<R, HALF, true>(L, x, v0, v1);
+            if (HALF) {
+#pragma unroll
+                for (int z = 0; z < R; ++z) {
+                    const bool one = ((q ^ z) & 1) != 0;
+                    E[z] = one ? v1[z] : v0[z];
+                    O[z] = one ? v0[z] : v1[z];
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+template <bool HALF>
+__device__ __forceinline__ void uni_low_smooth_one(const ULow& K, const ULowLevel& l, const ULowLevel& c, int warp, int leg, bool zero) {
+    const int k = warp >= l.n0, ns = 2 * (leg ? K.post : K.pre);
+    const UX<HALF> x{l.xf, l.xh, l.scale};
+    using S = USrcX<HALF, false>;
+    const S src{x, UX<false>{nullptr, nullptr, nullptr}, false};
+    ULane<1> L;
+    UHaloOne<S, false> H;
+    const bool any = L.init(l.v, warp);
+    H.init(L);
+    float v = 0.f, b = 0.f;
+    if (L.live) {
+        if (!zero) v = x.get(L.at, x.sc(L.block));
+        b = l.b[L.at];
+        if (leg && (L.mask & 1u)) v += c.xh ? umul(__half2float(c.xh[L.coff]), c.scale[L.block]) : c.xf[L.coff];
+    }
+    if ((zero || leg) && any) uni_store<1, HALF, true>(L, x, &v, &v);
+    const float diag = -(L.wx0 + L.wx1 + L.wy0 + L.wy1 + L.wz0 + L.wz1);
+    const float rcp = urcp(diag);
+    const bool on = (L.mask & 1u) && !(fabsf(diag) < 1e-9f);
+    __syncthreads();
+#pragma unroll 1
+    for (int st = 0; st < ns; ++st) {
+        if (((st ^ leg) & 1) == k && any) {
+            H.load(src);
+            const float(&h)[6] = H.h;
+            if (on)
+#pragma unroll 1
+                for (int it = 0; it < K.iters; ++it) {
+                    float Ax = ufma(L.wx0, h[0], umul(L.wx1, h[1]));
+                    Ax = ufma(L.wy0, h[2], Ax);
+                    Ax = ufma(L.wy1, h[3], Ax);
+                    Ax = ufma(L.wz0, h[4], Ax);
+                    Ax = ufma(L.wz1, h[5], Ax);
+                    Ax = ufma(diag, v, Ax);
+                    v = ufma(K.omega, umul(b - Ax, rcp), v);
+                }
+            uni_store<1, HALF, true>(L, x, &v, &v);
+        }
+        __syncthreads();
+    }
+}
+template <bool GEN>
+__global__ void __launch_bounds__(ULOW_THREADS, 1) k_uni_low(const __grid_constant__ ULow K) {
+    const int wid = threadIdx.x >> 5;
+    pdl_wait();
+#pragma unroll 1
+    for (int leg = K.down ? 0 : 1; leg < (K.up ? 2 : 1); ++leg) {
+#pragma unroll 1
+        for (int i = 0; i <= K.last - K.first; ++i) {
+            const int m = leg ? K.last - i : K.first + i;
+            const ULowLevel& l = K.lv[m];
+            const ULowLevel& c = K.lv[m + 1];
+            const bool zero = leg == 0 && (m > K.first || K.zero);
+            const bool has = wid < l.v.nwarp;  // a warp per descriptor
+            const int r = has ? l.v.desc[wid].y >> 8 : 0;
+#define AW_UB(R) uni_low_smooth<R, false, GEN>(K, l, c, wid, leg, zero)
+            if (!has) {
+                for (int st = 0; st <= 2 * (leg ? K.post : K.pre); ++st) __syncthreads();
+            } else if (l.xh) {
+                if (r == 4) uni_low_smooth<4, true, GEN>(K, l, c, wid, leg, zero);
+                else if (r == 2) uni_low_smooth<2, true, GEN>(K, l, c, wid, leg, zero);
+                else uni_low_smooth_one<true>(K, l, c, wid, leg, zero);
+            } else {
+                AW_UNI_RES(r, AW_UB, (uni_low_smooth_one<false>(K, l, c, wid, leg, zero)))
+            }
+#undef AW_UB
+            if (leg == 0) {
+                if (has) {
+#define AW_UB(R, H)                                                                                    {                                                                                                      const USrcX<H, false> src{UX<H>{l.xf, l.xh, l.scale}, UX<false>{}, false};                          ULane<R> L;                                                                                        UHalos<R, USrcX<H, false>, false> E;                                                               const bool any = L.init(l.v, wid);                                                                 E.init(L);                                                                                         if (any)                                                                                               uni_residual_body<R, USrcX<H, false>, false, GEN>(L, l.v.W, GEN && l.v.general[wid], E,                                                               src, l.b, l.out, src.x.sc(L.block));      }
+#define AW_UB1(H)                                                                     {                                                                                     const USrcX<H, false> src{UX<H>{l.xf, l.xh, l.scale}, UX<false>{}, false};         ULane<1> L;                                                                       UHaloOne<USrcX<H, false>, false> E;                                               const bool any = L.init(l.v, wid);                                                E.init(L);                                                                        if (any) uni_residual_one<USrcX<H, false>, false>(L, E, src, l.b, l.out);     }
+#define AW_UBF(R) AW_UB(R, false)
+                    if (l.xh) {
+                        if (r == 4) AW_UB(4, true)
+                        else if (r == 2) AW_UB(2, true)
+                        else AW_UB1(true)
+                    } else {
+                        AW_UNI_RES(r, AW_UBF, AW_UB1(false))
+                    }
+#undef AW_UB
+#undef AW_UBF
+#undef AW_UB1
+                }
+                __syncthreads();
+            }
+        }
+        if (leg == 0 && K.exact) {  // x = Minv b, as k_coarse_apply
+            const int n = K.ex_n[0], lane = threadIdx.x & 31;
+            for (int i = wid; i < n; i += ULOW_WARPS) {
+                double t = 0.0;
+                for (int j = lane; j < n; j += 32) t += K.Minv[(size_t)i * n + j] * (double)K.xb[K.cell[K.idx[j]]];
+                t = warp_sum(t);
+                if (lane == 0) K.lv[K.last + 1].xf[K.cell[K.idx[i]]] = (float)t;
+            }
+            __syncthreads();
+        }
+    }
+    pdl_trigger();
+}
+
 // FP64: r64 = b - A p with its FP32 copy r and |r|^2 (k_uni_residual64), or one step of the conjugate
 // gradients: q = -A d with d = z + beta d_old formed where it is read (own cells and halo), stored as the
 // new direction, and d . q (k_uni_apply).  The direction alternates between two buffers, since a
@@ -1104,7 +1340,6 @@ struct UCheck {
     uint8_t* general;
     int* count;     // += blocks that are not uniform
 };
-constexpr int UNI_MAX_LEVELS = 4;  // 8^3 blocks halve to one cell in three steps
 struct UCheckAll {
     UniView v[UNI_MAX_LEVELS];
     UCheck k[UNI_MAX_LEVELS];

@@ -209,3 +209,33 @@ def test_vcycle_call(precision):
     assert torch.equal(cycles(True, False), ref)
     assert torch.equal(cycles(True, True), ref)
     g.close()
+
+
+# block grids around the limits of the one-launch form: 16 and more warps a colour (levels with launches of
+# their own above it), 128 and more coarsest cells (two legs around the coarsest solve)
+@pytest.mark.parametrize("dims", [(2, 1, 1), (2, 2, 2), (4, 4, 2), (5, 7, 1), (8, 4, 4), (43, 3, 1), (8, 8, 2), (8, 8, 8)])
+@pytest.mark.parametrize("spread", [1, 4])
+@pytest.mark.parametrize("precision", [aw.PRECISION_FP32, aw.PRECISION_MIXED])
+def test_small_levels_in_one_launch(dims, spread, precision):
+    """The same bodies in one launch and in a launch per step: equal bits, the mixed form's FP64 sums too."""
+    nb = int(np.prod(dims))
+    lv = np.arange(nb) * 7919 % spread
+    g = _grid(dims, lv)
+    gen = torch.Generator(device="cuda").manual_seed(nb)
+    n = g.totals()[0]
+    X = g.face_positions(3)
+    fluid = (X[:, 0] + 0.4 * X[:, 1] < 0.8 * dims[0]).to(torch.uint8)
+    b = torch.randn(n, generator=gen, device="cuda") * fluid
+    for varying in (False, True):
+        if varying:
+            beta = g.channel(aw.BETA_COEFF_Y)
+            beta.copy_(0.3 + 0.7 * torch.rand(beta.numel(), generator=gen, device="cuda"))
+        a = _solve(g, True, precision, fluid, b, 1e-30, max_cycles=4)
+        os.environ["AW_NO_UNIFORM_LOW"] = "1"
+        try:
+            s = _solve(g, True, precision, fluid, b, 1e-30, max_cycles=4)
+        finally:
+            os.environ.pop("AW_NO_UNIFORM_LOW", None)
+        for (c1, r1, p1), (c0, r0, q0) in zip(a, s):
+            assert c1 == c0 and _same(p1, q0) and (r1 == r0 or r0 != r0)
+    g.close()
