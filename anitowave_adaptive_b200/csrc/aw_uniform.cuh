@@ -1053,7 +1053,8 @@ __global__ void __launch_bounds__(UNT, 4) k_uni_residual(const __grid_constant__
 // (smoothing, restricted residual), applies the inverse of the coarsest operator where that is the next
 // level and small, and walks back up (prolongation, smoothing).  down / up alone: the legs around a coarser
 // part with launches of its own.  A warp keeps its blocks' cells, weights and addresses in registers for a
-// leg of a level and meets the others at CTA barriers; a colour's step then reads the halo, updates and
+// leg of a level, keeps x in shared memory too (halos read from L1 or L2 after another warp's store took
+// 0.5 us of a step), and meets the others at CTA barriers; a colour's step then reads the halo, updates and
 // stores.  Every cell's arithmetic is that of the separate launches, bit for bit.
 // A level of at most ULOW_WARPS warps leaves most of the chip idle either way, and as launches its steps were
 // latency alone, 3.5 to 4 us a colour of 32 4^3 blocks, most of it the record, weight and halo-address chain
@@ -1061,6 +1062,7 @@ __global__ void __launch_bounds__(UNT, 4) k_uni_residual(const __grid_constant__
 constexpr int UNI_MAX_LEVELS = 4;  // 8^3 blocks halve to one cell in three steps
 constexpr int ULOW_THREADS = 512;
 constexpr int ULOW_WARPS = ULOW_THREADS / 32;
+constexpr int ULOW_CELLS = 512 * ULOW_WARPS;  // an 8^3 block a warp at most
 constexpr int ULOW_EXACT = 128;  // cells of a coarsest level taken along (its inverse comes from L2: 128 KB)
 struct ULowLevel {
     UniView v;   // both colours
@@ -1082,30 +1084,56 @@ struct ULow {
     const uint32_t* cell;              // cell offset of a block of the coarsest level
     const float* xb;
 };
+// x of the walk's current level in shared memory, as the kernels read it back from its storage
+struct UXS {
+    float* s;
+    __device__ __forceinline__ float2 get2(uint32_t i, float, bool even) const {
+        if (even) return *reinterpret_cast<const float2*>(s + i);
+        return make_float2(s[i], s[i + 1]);
+    }
+};
+struct USrcS {
+    using T = float;
+    struct Ctx {};
+    UXS x;
+    __device__ __forceinline__ Ctx ctx(int) const { return Ctx{}; }
+    __device__ __forceinline__ float get(uint32_t i, const Ctx&) const { return x.s[i]; }
+    __device__ __forceinline__ float coarse(uint32_t, const Ctx&) const { return 0.f; }
+};
+// the block to shared memory (v0, v1 as stored)
+template <int R>
+__device__ __forceinline__ void uni_low_put(const ULane<R>& L, float* xs, const float* v0, const float* v1) {
+#pragma unroll
+    for (int z = 0; z < R; ++z) {
+        if (R == 1) xs[L.at] = v0[z];
+        else ustore2(xs, L.at + (uint32_t)(R * R * z), L.even, v0[z], v1[z]);
+    }
+}
 // one warp's smoothing of one leg: 1 + ns barriers
 template <int R, bool HALF, bool GEN>
-__device__ __forceinline__ void uni_low_smooth(const ULow& K, const ULowLevel& l, const ULowLevel& c, int warp, int leg, bool zero) {
+__device__ __forceinline__ void uni_low_smooth(const ULow& K, const ULowLevel& l, const ULowLevel& c, int warp, int leg, bool zero, float* xs) {
     const int k = warp >= l.n0, ns = 2 * (leg ? K.post : K.pre);
     const UX<HALF> x{l.xf, l.xh, l.scale};
-    using S = USrcX<HALF, false>;
-    const S src{x, UX<false>{nullptr, nullptr, nullptr}, false};
+    using S = USrcS;
+    const S src{UXS{xs}};
     ULane<R> L;
     UHalos<R, S, false> H;
     const bool any = L.init(l.v, warp);
+    const bool in = L.lane / UG<R>::LPB < (l.v.desc[warp].y & 0xFF);  // a block's lane; air blocks are read too
     H.init(L);
     const int q = (L.y & 1) ^ leg;
     float E[R], O[R], bE[R], bO[R];
     {
         float v0[R], v1[R];
         const bool moved = zero || leg;  // x changes before the first step
-        const float sc = zero || !L.live ? 1.f : x.sc(L.block);
+        const float sc = zero || !in ? 1.f : x.sc(L.block);
         const float scc = leg && c.xh && L.live ? c.scale[L.block] : 1.f;
 #pragma unroll
         for (int z = 0; z < R; ++z) {
             float2 v = make_float2(0.f, 0.f), bv = make_float2(0.f, 0.f);
+            const uint32_t i = L.at + (uint32_t)(R * R * z);
+            if (in && !zero) v = x.get2(i, sc, L.even);
             if (L.live) {
-                const uint32_t i = L.at + (uint32_t)(R * R * z);
-                if (!zero) v = x.get2(i, sc, L.even);
                 uload2(l.b, i, L.even, bv.x, bv.y);
                 if (leg) {
                     const uint32_t ci = L.coff + (uint32_t)(L.xp + (R / 2) * ((L.y >> 1) + (R / 2) * (z >> 1)));
@@ -1121,6 +1149,7 @@ __device__ __forceinline__ void uni_low_smooth(const ULow& K, const ULowLevel& l
             bO[z] = one ? bv.x : bv.y;
         }
         if (moved && any) uni_store<R, HALF, true>(L, x, v0, v1);
+        if (in) uni_low_put<R>(L, xs, v0, v1);
 #pragma unroll
         for (int z = 0; z < R; ++z) {
             const bool one = ((q ^ z) & 1) != 0;
@@ -1147,6 +1176,7 @@ __device__ __forceinline__ void uni_low_smooth(const ULow& K, const ULowLevel& l
                 v1[z] = one ? E[z] : O[z];
             }
             uni_store<R, HALF, true>(L, x, v0, v1);
+            if (L.live) uni_low_put<R>(L, xs, v0, v1);
             if (HALF) {
 #pragma unroll
                 for (int z = 0; z < R; ++z) {
@@ -1160,22 +1190,24 @@ __device__ __forceinline__ void uni_low_smooth(const ULow& K, const ULowLevel& l
     }
 }
 template <bool HALF>
-__device__ __forceinline__ void uni_low_smooth_one(const ULow& K, const ULowLevel& l, const ULowLevel& c, int warp, int leg, bool zero) {
+__device__ __forceinline__ void uni_low_smooth_one(const ULow& K, const ULowLevel& l, const ULowLevel& c, int warp, int leg, bool zero, float* xs) {
     const int k = warp >= l.n0, ns = 2 * (leg ? K.post : K.pre);
     const UX<HALF> x{l.xf, l.xh, l.scale};
-    using S = USrcX<HALF, false>;
-    const S src{x, UX<false>{nullptr, nullptr, nullptr}, false};
+    using S = USrcS;
+    const S src{UXS{xs}};
     ULane<1> L;
     UHaloOne<S, false> H;
     const bool any = L.init(l.v, warp);
+    const bool in = L.lane < (l.v.desc[warp].y & 0xFF);
     H.init(L);
     float v = 0.f, b = 0.f;
+    if (in && !zero) v = x.get(L.at, x.sc(L.block));
     if (L.live) {
-        if (!zero) v = x.get(L.at, x.sc(L.block));
         b = l.b[L.at];
         if (leg && (L.mask & 1u)) v += c.xh ? umul(__half2float(c.xh[L.coff]), c.scale[L.block]) : c.xf[L.coff];
     }
     if ((zero || leg) && any) uni_store<1, HALF, true>(L, x, &v, &v);
+    if (in) xs[L.at] = v;
     const float diag = -(L.wx0 + L.wx1 + L.wy0 + L.wy1 + L.wz0 + L.wz1);
     const float rcp = urcp(diag);
     const bool on = (L.mask & 1u) && !(fabsf(diag) < 1e-9f);
@@ -1197,12 +1229,14 @@ __device__ __forceinline__ void uni_low_smooth_one(const ULow& K, const ULowLeve
                     v = ufma(K.omega, umul(b - Ax, rcp), v);
                 }
             uni_store<1, HALF, true>(L, x, &v, &v);
+            if (L.live) xs[L.at] = v;
         }
         __syncthreads();
     }
 }
 template <bool GEN>
 __global__ void __launch_bounds__(ULOW_THREADS, 1) k_uni_low(const __grid_constant__ ULow K) {
+    __shared__ __align__(16) float xs[ULOW_CELLS];
     const int wid = threadIdx.x >> 5;
     pdl_wait();
 #pragma unroll 1
@@ -1215,31 +1249,39 @@ __global__ void __launch_bounds__(ULOW_THREADS, 1) k_uni_low(const __grid_consta
             const bool zero = leg == 0 && (m > K.first || K.zero);
             const bool has = wid < l.v.nwarp;  // a warp per descriptor
             const int r = has ? l.v.desc[wid].y >> 8 : 0;
-#define AW_UB(R) uni_low_smooth<R, false, GEN>(K, l, c, wid, leg, zero)
+#define AW_UB(R) uni_low_smooth<R, false, GEN>(K, l, c, wid, leg, zero, xs)
             if (!has) {
                 for (int st = 0; st <= 2 * (leg ? K.post : K.pre); ++st) __syncthreads();
             } else if (l.xh) {
-                if (r == 4) uni_low_smooth<4, true, GEN>(K, l, c, wid, leg, zero);
-                else if (r == 2) uni_low_smooth<2, true, GEN>(K, l, c, wid, leg, zero);
-                else uni_low_smooth_one<true>(K, l, c, wid, leg, zero);
+                if (r == 4) uni_low_smooth<4, true, GEN>(K, l, c, wid, leg, zero, xs);
+                else if (r == 2) uni_low_smooth<2, true, GEN>(K, l, c, wid, leg, zero, xs);
+                else uni_low_smooth_one<true>(K, l, c, wid, leg, zero, xs);
             } else {
-                AW_UNI_RES(r, AW_UB, (uni_low_smooth_one<false>(K, l, c, wid, leg, zero)))
+                AW_UNI_RES(r, AW_UB, (uni_low_smooth_one<false>(K, l, c, wid, leg, zero, xs)))
             }
 #undef AW_UB
             if (leg == 0) {
                 if (has) {
-#define AW_UB(R, H)                                                                                    {                                                                                                      const USrcX<H, false> src{UX<H>{l.xf, l.xh, l.scale}, UX<false>{}, false};                          ULane<R> L;                                                                                        UHalos<R, USrcX<H, false>, false> E;                                                               const bool any = L.init(l.v, wid);                                                                 E.init(L);                                                                                         if (any)                                                                                               uni_residual_body<R, USrcX<H, false>, false, GEN>(L, l.v.W, GEN && l.v.general[wid], E,                                                               src, l.b, l.out, src.x.sc(L.block));      }
-#define AW_UB1(H)                                                                     {                                                                                     const USrcX<H, false> src{UX<H>{l.xf, l.xh, l.scale}, UX<false>{}, false};         ULane<1> L;                                                                       UHaloOne<USrcX<H, false>, false> E;                                               const bool any = L.init(l.v, wid);                                                E.init(L);                                                                        if (any) uni_residual_one<USrcX<H, false>, false>(L, E, src, l.b, l.out);     }
-#define AW_UBF(R) AW_UB(R, false)
-                    if (l.xh) {
-                        if (r == 4) AW_UB(4, true)
-                        else if (r == 2) AW_UB(2, true)
-                        else AW_UB1(true)
-                    } else {
-                        AW_UNI_RES(r, AW_UBF, AW_UB1(false))
-                    }
+                    const USrcS src{UXS{xs}};
+#define AW_UB(R)                                                                                                    \
+    {                                                                                                               \
+        ULane<R> L;                                                                                                 \
+        UHalos<R, USrcS, false> E;                                                                                  \
+        const bool any = L.init(l.v, wid);                                                                          \
+        E.init(L);                                                                                                  \
+        if (any)                                                                                                    \
+            uni_residual_body<R, USrcS, false, GEN>(L, l.v.W, GEN && l.v.general[wid], E, src, l.b, l.out, 1.f);     \
+    }
+#define AW_UB1                                                         \
+    {                                                                  \
+        ULane<1> L;                                                    \
+        UHaloOne<USrcS, false> E;                                      \
+        const bool any = L.init(l.v, wid);                             \
+        E.init(L);                                                     \
+        if (any) uni_residual_one<USrcS, false>(L, E, src, l.b, l.out); \
+    }
+                    AW_UNI_RES(r, AW_UB, AW_UB1)
 #undef AW_UB
-#undef AW_UBF
 #undef AW_UB1
                 }
                 __syncthreads();

@@ -211,9 +211,9 @@ def test_vcycle_call(precision):
     g.close()
 
 
-# block grids around the limits of the one-launch form: 16 and more warps a colour (levels with launches of
-# their own above it), 128 and more coarsest cells (two legs around the coarsest solve)
-@pytest.mark.parametrize("dims", [(2, 1, 1), (2, 2, 2), (4, 4, 2), (5, 7, 1), (8, 4, 4), (43, 3, 1), (8, 8, 2), (8, 8, 8)])
+# block grids around the limits of the one-launch form: a CTA (16 warps), clusters of 2 to 8 CTAs, and more (levels
+# with launches of their own), 128 and more coarsest cells (two legs around the coarsest solve)
+@pytest.mark.parametrize("dims", [(2, 1, 1), (2, 2, 2), (4, 4, 2), (5, 7, 1), (8, 4, 4), (43, 3, 1), (8, 8, 2), (3, 3, 3), (5, 5, 5), (8, 8, 8), (13, 11, 8)])
 @pytest.mark.parametrize("spread", [1, 4])
 @pytest.mark.parametrize("precision", [aw.PRECISION_FP32, aw.PRECISION_MIXED])
 def test_small_levels_in_one_launch(dims, spread, precision):
