@@ -619,6 +619,7 @@ __device__ __forceinline__ void p2g_cross(const CrossNb& N, int rn, const float 
 constexpr int P2G_THREADS = 512;  // the most threads a P2G CTA is launched with
 constexpr int P2G_XQ = 96;  // per-warp queue of cross-resolution pairs: < 32 waiting + 2 per lane
 constexpr int P2G_SLICE = 16;  // particles of one cell per register-accumulation task
+constexpr int P2G_BINS = 64;   // counts told apart when a block's cells are ordered
 constexpr int P2G_MAX_SLICES = 1 << 19;  // 6 * 8^3 * this stays below 2^31
 constexpr int P2G_MAX_CELLS = 16 * 16 * 16;  // cells of the largest block (base resolution <= 16)
 constexpr int P2G_NEAR_CELLS = 8 * 8 * 8;    // blocks up to this size list their near cells
@@ -702,6 +703,7 @@ __global__ void __launch_bounds__(P2G_THREADS, 2) k_p2g_own(LevelView L, const f
     __shared__ int ccount[P2G_MAX_CELLS / 32], cocount[P2G_MAX_CELLS / 32];
     __shared__ uint16_t clist[P2G_MAX_CELLS], colist[P2G_MAX_CELLS];
     __shared__ int nonempty, nnear, ncoarse;
+    __shared__ int hist[P2G_BINS];  // cells by particle count, then where a count's cells go in clist
     __shared__ int tctr[2];  // next own / coarse task to hand out
     // near-cell list of the cross-resolution pass (blocks of at most P2G_NEAR_CELLS cells)
     __shared__ uint16_t nl_cell[P2G_NEAR_CELLS];
@@ -753,6 +755,7 @@ __global__ void __launch_bounds__(P2G_THREADS, 2) k_p2g_own(LevelView L, const f
     float* cpw = cmw + 3 * TAc;
     float* cqw = cmw + 6 * TAc;
     for (int i = threadIdx.x; i < ntile; i += blockDim.x) sm[i] = 0.f;
+    if (threadIdx.x < P2G_BINS) hist[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         cross = 0;
         coarse = 0;
@@ -796,8 +799,11 @@ __global__ void __launch_bounds__(P2G_THREADS, 2) k_p2g_own(LevelView L, const f
     // over the particles whose phase is not 0 (the others add nothing).  Slices hold P2G_SLICE
     // particles unless a crowded cell would push the task count past 6 * 512 * P2G_MAX_SLICES.
     const int nc3 = r * r * r;
-    // The block's non-empty cells, in cell order: tasks run over these only, so that lanes do not
-    // idle on the air cells of a surface block.
+    // The block's non-empty cells, fullest first: tasks run over these only, so that lanes do not idle on the
+    // air cells of a surface block, and the lanes of a warp take cells of one count (in cell order a warp ran
+    // as long as its fullest cell, 13 steps for a mean of 8, and a second slice took a pass over all cells:
+    // with the loads below 243 to 207 us at 4.1M particles).  Counts of P2G_BINS - 1 and more are not told
+    // apart.
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     // A cell is listed for the coarse tile too when it lies within two of b's cells (one coarse
     // cell, the reach there) of a side towards a coarser neighbour, on every axis that neighbour's
@@ -824,36 +830,38 @@ __global__ void __launch_bounds__(P2G_THREADS, 2) k_p2g_own(LevelView L, const f
             if (c == nc3 - 1) cst[nc3] = a1;
             cnt = a1 - a0;
         }
-        if (cnt > 0) atomicMax(&maxcnt, cnt);
-        const unsigned m = __ballot_sync(0xffffffffu, cnt > 0);
-        const unsigned mc = __ballot_sync(0xffffffffu, cnt > 0 && cmask && coarse_near(c));
-        if (lane == 0) {
-            ccount[ch] = __popc(m);
-            cocount[ch] = __popc(mc);
+        if (cnt > 0) {
+            atomicMax(&maxcnt, cnt);
+            atomicAdd(&hist[min(cnt, (uint32_t)(P2G_BINS - 1))], 1);
         }
+        const unsigned mc = __ballot_sync(0xffffffffu, cnt > 0 && cmask && coarse_near(c));
+        if (lane == 0) cocount[ch] = __popc(mc);
     }
     __syncthreads();
-    if (wid == 0) {  // exclusive scans of the per-chunk counts
+    if (wid == 0) {  // exclusive scans: the bins from the fullest down, the chunks' counts of coarse-near cells
         int carry = 0, carry2 = 0;
-        for (int base = 0; base < nchunk; base += 32) {
-            const int ch = base + lane;
-            const int v = ch < nchunk ? ccount[ch] : 0;
-            const int v2 = ch < nchunk ? cocount[ch] : 0;
-            int incl = v, incl2 = v2;
+        for (int base = 0; base < P2G_BINS; base += 32) {
+            const int k = P2G_BINS - 1 - base - lane;
+            const int v = hist[k];
+            int incl = v;
 #pragma unroll
             for (int sh = 1; sh < 32; sh <<= 1) {
                 const int y = __shfl_up_sync(0xffffffffu, incl, sh);
-                const int y2 = __shfl_up_sync(0xffffffffu, incl2, sh);
-                if (lane >= sh) {
-                    incl += y;
-                    incl2 += y2;
-                }
+                if (lane >= sh) incl += y;
             }
-            if (ch < nchunk) {
-                ccount[ch] = carry + incl - v;
-                cocount[ch] = carry2 + incl2 - v2;
-            }
+            hist[k] = carry + incl - v;
             carry += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        for (int base = 0; base < nchunk; base += 32) {
+            const int ch = base + lane;
+            const int v2 = ch < nchunk ? cocount[ch] : 0;
+            int incl2 = v2;
+#pragma unroll
+            for (int sh = 1; sh < 32; sh <<= 1) {
+                const int y2 = __shfl_up_sync(0xffffffffu, incl2, sh);
+                if (lane >= sh) incl2 += y2;
+            }
+            if (ch < nchunk) cocount[ch] = carry2 + incl2 - v2;
             carry2 += __shfl_sync(0xffffffffu, incl2, 31);
         }
         if (lane == 0) {
@@ -866,9 +874,8 @@ __global__ void __launch_bounds__(P2G_THREADS, 2) k_p2g_own(LevelView L, const f
         const int c = ch * 32 + lane;
         const bool ne = c < nc3 && cst[c + 1] > cst[c];
         const bool cn = ne && cmask && coarse_near(c);
-        const unsigned m = __ballot_sync(0xffffffffu, ne);
         const unsigned mc = __ballot_sync(0xffffffffu, cn);
-        if (ne) clist[ccount[ch] + __popc(m & ((1u << lane) - 1u))] = (uint16_t)c;
+        if (ne) clist[atomicAdd(&hist[min(cst[c + 1] - cst[c], (uint32_t)(P2G_BINS - 1))], 1)] = (uint16_t)c;
         if (cn) colist[cocount[ch] + __popc(mc & ((1u << lane) - 1u))] = (uint16_t)c;
     }
     __syncthreads();
@@ -1006,9 +1013,12 @@ __global__ void __launch_bounds__(P2G_THREADS, 2) k_p2g_own(LevelView L, const f
             } else {
                 val = soa[(int64_t)(3 + a) * n + i];
             }
-            const float qa = (soa[(int64_t)a * n + i] - oa) * invh;
-            const float q1 = (soa[(int64_t)t1 * n + i] - o1) * invh;
-            const float q2 = (soa[(int64_t)t2 * n + i] - o2) * invh;
+            // the kinds' lanes of a cell read one address each time and turn the axes in registers (reading axis
+            // a, t1, t2 first touched 32 sectors a load, and L1 wavefronts bounded the kernel)
+            const float px = soa[i], py = soa[n + i], pz = soa[2 * n + i];
+            const float qa = ((a == 0 ? px : (a == 1 ? py : pz)) - oa) * invh;
+            const float q1 = ((a == 0 ? py : (a == 1 ? pz : px)) - o1) * invh;
+            const float q2 = ((a == 0 ? pz : (a == 1 ? px : py)) - o2) * invh;
             // Along a: faces ka and ka + 1.  Across: of the three face rows k - 1, k, k + 1 (centres at
             // k - 0.5, k + 0.5, k + 1.5 in cell units) a particle reaches the centre row k and the side
             // row on its own side of the cell centre; the third is more than one cell away, so its

@@ -1058,7 +1058,10 @@ __global__ void __launch_bounds__(UNT, 4) k_uni_residual(const __grid_constant__
 // stores.  Every cell's arithmetic is that of the separate launches, bit for bit.
 // A level of at most ULOW_WARPS warps leaves most of the chip idle either way, and as launches its steps were
 // latency alone, 3.5 to 4 us a colour of 32 4^3 blocks, most of it the record, weight and halo-address chain
-// and the fetch of straight-line code that runs once: @.
+// and the fetch of straight-line code that runs once: the 64-block levels under a 32^3 grid and their coarsest
+// solve took 79 us a cycle, 34.5 in this launch; the 16^3 FLIP step 982, now 831 us.  (A cluster of 2 to 8 CTAs
+// for levels of 17 to 128 warps lost: 64^3 V-cycle 170 to 182 us, its barrier and halos through L2.)  What
+// bounds it is the latency of one colour's update.
 constexpr int UNI_MAX_LEVELS = 4;  // 8^3 blocks halve to one cell in three steps
 constexpr int ULOW_THREADS = 512;
 constexpr int ULOW_WARPS = ULOW_THREADS / 32;
