@@ -70,7 +70,7 @@ __device__ inline uint32_t particle_key(const LevelView& L, const float p[3], ui
 // tile's, and a running offset per digit carries over.  Equal keys keep their input order.
 //
 // (Before, a single warp walked 2048 keys: 41 us a pass of 4.1M keys at 14 warps per SM, 42 us even for
-// 7,680 particles, with a (digit, tile) table of 2M entries whose scan took 25 us; now 14 and 5 us.)
+// 7,680 particles, with a (digit, tile) table of 2M entries whose scan took 25 us; now 20 to 23 us a pass and 7 for its rows.)
 // ------------------------------------------------------------------------------------------------
 constexpr int RADIX_MAX_BITS = 11, RADIX_MAX_BINS = 1 << RADIX_MAX_BITS;
 constexpr int SORT_THREADS = 256, SORT_ITEMS = 16, SORT_WARPS = SORT_THREADS / 32;
@@ -415,8 +415,8 @@ __global__ void k_gather(const uint32_t* __restrict__ src, int64_t n, PArr pos, 
 }
 
 // Content hashes of AoS positions and, when given, velocities into hash[2], hash[3].  Four particles per
-// thread and step, read as three 16-byte words where the array allows it (12-byte particles read float by
-// float kept the load unit busy: 26 us for 4.1M particles, 17 now).
+// thread and step, read as three 16-byte words where the array allows it (of 4.1M particles' positions: 26 us
+// float by float, 17 now; positions and velocities 28).  Bound by memory traffic.
 __device__ __forceinline__ void hash_load4(const float* __restrict__ p, int64_t q, bool wide, float v[12]) {
     if (wide) {
         const float4* f = reinterpret_cast<const float4*>(p) + 3 * q;
@@ -1293,7 +1293,7 @@ __global__ void __launch_bounds__(1024) k_block_order(LevelView L, const uint32_
     __shared__ int hist[NBK], base[NBK];
     if (threadIdx.x < NBK) hist[threadIdx.x] = 0;
     // every load of a step for all of the thread's blocks before the first is used (block by block, the
-    // three dependent loads took 14 us for 4096 blocks)
+    // three dependent loads took 14 us for 4096 blocks, 8 now)
     int r[K], bk[K];
     uint32_t c0[K], p0[K], p1[K];
 #pragma unroll

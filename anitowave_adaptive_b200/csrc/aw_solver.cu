@@ -10,10 +10,13 @@
 //   MultigridTransfer.cuh:9-102 restriction (8-child sum) / prolongation (injection add)
 //   VCycle.cuh:177-304    init (coarse offsets, Galerkin) and recursive runCycle
 //
-// B200 design: every block-structured kernel is one CTA per block with the block and a one-cell
-// halo staged in shared memory; the smoother runs all its block-local sweeps out of shared
-// memory and touches HBM once per launch.  Uniform coarse levels continue below one cell per
-// block and end in an FP64 dense solve (Cholesky inverse built on the device each setup).
+// B200 design: finite-volume solves on blocks of up to 8^3 cells run out of registers, a group of lanes per
+// block (aw_uniform.cuh), the smallest block-structured levels in one CTA (k_uni_low).  The staged kernels
+// here serve the rest (larger blocks, residual tracking, deactivation, the reference's operator, the level
+// calls): a CTA per batch of blocks with the blocks and a one-cell halo in shared memory; the smoother runs
+// all its block-local sweeps there and touches HBM once per launch.  Uniform coarse levels continue below one
+// cell per block (k_dense_tail from 4096 cells on) and end in an FP64 dense solve (Cholesky inverse built on
+// the device each setup).
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>

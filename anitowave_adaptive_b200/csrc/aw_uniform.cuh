@@ -14,9 +14,9 @@
 // What bounded the staged form (one CTA per 8^3 block: block, halo and the three coefficient arrays
 // in shared memory) was instruction issue: index splits of the staging loops, six shared-memory
 // weight loads per update, and a CTA barrier per colour: 45.7M warp instructions and 60 us per colour
-// of the 4.7M-cell poisson_256 level at 13% of the HBM rate.  Here the same launch takes 19.5 us (ncu,
-// cold), the solve to 1e-6 2.69 instead of 5.92 ms; the small levels' launches 5 to 10 instead of 10 to 13
-// us, and the dam_drop_128 step 2.05 instead of 2.68 ms.  What bounds it now is the latency of a launch's
+// of the 4.7M-cell poisson_256 level at 13% of the HBM rate.  Here the same launch takes 27 us (ncu,
+// cold), the solve to 1e-6 2.71 instead of 5.92 ms; the small levels' launches 5 to 10 instead of 10 to 13
+// us, and the dam_drop_128 step's solve 1.06 instead of 1.71 ms.  What bounds it now is the latency of a launch's
 // loads (slot record, then cells and halo).  The arithmetic of a cell is that of the staged kernels,
 // operation by operation, so both forms agree bit for bit.
 #pragma once
