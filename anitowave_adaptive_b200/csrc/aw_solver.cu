@@ -101,6 +101,9 @@ struct aw_solver {
     // buffers: the uniform form reads the old one while it writes the new), -A d), its scalars
     // {rho, rho_old, d.(-A d)} and a zero right-hand side for applying A
     aw::DBuf<double> cg_r, cg_d, cg_d2, cg_q, cg_sc;
+    // aligned copies of a caller's b and p that do not start on 16 bytes (aw_solve)
+    aw::DBuf<float> b_copy;
+    aw::DBuf<double> p_copy;
     aw::DBuf<unsigned> ticket;  // last_cta_sum: finished CTAs of the running launch (0 between launches)
     aw::DBuf<float> cg_zero;
     // FP32 conjugate gradients: direction, -A d, scalars {rho, rho_old, d.(-A d)}, partial sums
@@ -896,7 +899,6 @@ __global__ void k_cg_direction(double* __restrict__ d, const float* __restrict__
 // 32 bytes read and 20 written per cell; two cells per thread and step.
 struct CgVec {
     double* p;
-    int p_pairs;  // p is 16-byte aligned
     double* r;
     float* rf;
     const double *d0, *d1, *qn;
@@ -921,7 +923,7 @@ __global__ void __launch_bounds__(256) k_cg_update(CgVec K, double* part, unsign
         if (!(f.x | f.y)) continue;
         const double2 dv = reinterpret_cast<const double2*>(d)[i], qv = reinterpret_cast<const double2*>(K.qn)[i];
         double2 rv = reinterpret_cast<const double2*>(K.r)[i];
-        double2 pv = K.p_pairs ? reinterpret_cast<const double2*>(K.p)[i] : make_double2(K.p[2 * i], K.p[2 * i + 1]);
+        double2 pv = reinterpret_cast<const double2*>(K.p)[i];
         if (f.x) {
             pv.x += alpha * dv.x;
             rv.x = rv.x + alpha * qv.x;
@@ -932,12 +934,7 @@ __global__ void __launch_bounds__(256) k_cg_update(CgVec K, double* part, unsign
             rv.y = rv.y + alpha * qv.y;
             acc += rv.y * rv.y;
         }
-        if (K.p_pairs) {
-            reinterpret_cast<double2*>(K.p)[i] = pv;
-        } else {
-            K.p[2 * i] = pv.x;
-            K.p[2 * i + 1] = pv.y;
-        }
+        reinterpret_cast<double2*>(K.p)[i] = pv;
         reinterpret_cast<double2*>(K.r)[i] = rv;
         reinterpret_cast<float2*>(K.rf)[i] = make_float2((float)rv.x, (float)rv.y);
     }
@@ -3180,7 +3177,6 @@ static aw_status cg_iteration(aw_solver* S, double* p, unsigned ndot, cudaStream
         AW_TRY(launch_dep(S, k_reduce_sum, 1, 256, 0, s, S->partials.p, L0.ndesc[2], sc + 2));
     }
     K.p = p;
-    K.p_pairs = ((uintptr_t)p & 15u) == 0;
     K.r = S->cg_r.p;
     K.rf = L0.b.p;
     K.qn = S->cg_q.p;
@@ -3241,10 +3237,9 @@ static bool cg_devloop_build(aw_solver* S, double* p, unsigned ndot) {
     return true;
 }
 
-extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t* cycles, double* final_rel,
-                              aw_stream s_) {
-    AW_CHECK_ARG(S && d_b && d_p, "null argument");
-    cudaStream_t s = (cudaStream_t)s_;
+// aw_solve on arrays that start on 16 bytes: the kernels take two cells of a level array at a time
+static aw_status solve_aligned(aw_solver* S, const float* d_b, void* d_p, int32_t* cycles, double* final_rel,
+                               cudaStream_t s) {
     MGLevel& L0 = S->lv[0];
     const int cf = fv(S) ? 1 : 0;
     const size_t nc = L0.ncell();
@@ -3438,5 +3433,34 @@ extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t
     }
     if (cycles) *cycles = it;
     if (final_rel) *final_rel = rel;
+    return st;
+}
+
+// The caller's arrays may start at any element (a view): one that is not on 16 bytes is solved in an aligned
+// copy, 0.2 GB of traffic at 4.7M cells beside the solve's own, and p is copied back whatever the status.
+extern "C" aw_status aw_solve(aw_solver* S, const float* d_b, void* d_p, int32_t* cycles, double* final_rel,
+                              aw_stream s_) {
+    AW_CHECK_ARG(S && d_b && d_p, "null argument");
+    cudaStream_t s = (cudaStream_t)s_;
+    const size_t nc = S->lv[0].ncell();
+    const size_t pbytes = nc * (S->d.precision == AW_PRECISION_MIXED ? sizeof(double) : sizeof(float));
+    auto aligned = [](const void* q) { return ((uintptr_t)q & 15u) == 0; };
+    const float* b = d_b;
+    void* p = d_p;
+    if (!aligned(d_b)) {
+        AW_TRY(S->b_copy.ensure(std::max<size_t>(nc, 1)));
+        AW_CUDA(cudaMemcpyAsync(S->b_copy.p, d_b, nc * sizeof(float), cudaMemcpyDeviceToDevice, s));
+        b = S->b_copy.p;
+    }
+    if (!aligned(d_p)) {
+        AW_TRY(S->p_copy.ensure(std::max<size_t>((pbytes + 7) / 8, 1)));
+        AW_CUDA(cudaMemcpyAsync(S->p_copy.p, d_p, pbytes, cudaMemcpyDeviceToDevice, s));
+        p = S->p_copy.p;
+    }
+    const aw_status st = solve_aligned(S, b, p, cycles, final_rel, s);
+    if (p != d_p && st != AW_ERR_CUDA) {
+        AW_CUDA(cudaMemcpyAsync(d_p, p, pbytes, cudaMemcpyDeviceToDevice, s));
+        AW_CUDA(cudaStreamSynchronize(s));
+    }
     return st;
 }

@@ -45,6 +45,8 @@ constexpr int UNI_MAX_RES = 8;        // 16^3 blocks would take 128 cells per la
 // state of a slot, set by k_uni_check: no fluid cell (nothing to do), one conductance, several
 enum { US_AIR = 0, US_UNIFORM = 1, US_GENERAL = 2 };
 
+// The arrays of a level start on 16 bytes (the solver's own do, aw_solve sees to the caller's): a pair of cells
+// at an even index is one access.
 // One block-structured level as the kernels below see it.  Slots: the level's active blocks, colour 0
 // then colour 1, resolutions descending.  Warp w serves desc[w] = {first slot, count | res << 8}.
 //   rec: {cell offset, block, kinds, coarse cell offset}, neighbour cell offsets (6), neighbour blocks

@@ -252,6 +252,8 @@ aw_status aw_vcycle_run(aw_solver* sv, aw_stream s);
 /* Solve A p = b on level 0 to desc.tolerance.  FP32 precision: p is float*, V-cycles in place.
  * Mixed precision: p is double*, outer defect correction with the FP64 residual, FP64
  * accumulation and FP64 coarsest solve; V-cycle in FP32 with FP16 coarse corrections.
+ * d_b and d_p may start at any element; 16-byte aligned arrays are used in place, others through
+ * a copy that the solver keeps.
  * syncs (one residual norm read per cycle).  Returns AW_ERR_NOT_CONVERGED if max_cycles ran out. */
 aw_status aw_solve(aw_solver* sv, const float* d_b, void* d_p, int32_t* cycles, double* final_rel, aw_stream s);
 /* pressure-gradient update of VELOCITY_*: u -= dt (W/area) (p_high - p_low) on faces with a fluid

@@ -1,0 +1,54 @@
+"""Which arrays the solver takes and what it leaves in its own."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import anitowave_adaptive_b200 as aw  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+ALL = (aw.PRECISION_FP32, aw.PRECISION_MIXED, aw.PRECISION_FP32_PCG)
+
+
+def _grid(R0=8, dims=(5, 3, 3)):
+    """Blocks of every size beside one another, an inactive one among them."""
+    lv = [min(3, abs(x - 2) + (y == 2)) for z in range(dims[2]) for y in range(dims[1]) for x in range(dims[0])]
+    lv[-1] = 4
+    g = aw.MSBG(dims, 1.0, (0.0, 0.0, 0.0), R0, 4)
+    g.set_refinement_map(np.asarray(lv, np.uint32))
+    g.enforce_grading()
+    g.allocate()
+    return g
+
+
+def _problem(g, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    n = g.totals()[0]
+    fluid = (g.face_positions(3)[:, 0] < 3.3).to(torch.uint8)  # full, cut and empty blocks
+    return n, fluid, torch.randn(n, generator=gen, device="cuda") * fluid
+
+
+@pytest.mark.parametrize("precision", ALL)
+@pytest.mark.parametrize("R0", [8, 16])
+def test_arrays_that_start_at_any_element(R0, precision):
+    """Views at odd elements of b and p give the bits of arrays of their own, and nothing beside them is touched."""
+    g = _grid(R0)
+    n, fluid, b0 = _problem(g, 1)
+    dt = torch.float64 if precision == aw.PRECISION_MIXED else torch.float32
+    sv = aw.Solver(g, precision=precision, tolerance=1e-30, max_cycles=3)
+    sv.setup(fluid)
+    ref = torch.zeros(n, dtype=dt, device="cuda")
+    cyc, rel, st = sv.solve(b0, ref, raise_on_error=False)
+    for ob, op in [(1, 0), (0, 1), (1, 1), (2, 3), (3, 2), (4, 4)]:
+        bb = torch.full((n + 8,), 7.0, device="cuda")
+        pp = torch.full((n + 8,), 7.0, dtype=dt, device="cuda")
+        b, p = bb[ob:ob + n], pp[op:op + n]
+        b.copy_(b0)
+        p.zero_()
+        torch.cuda.synchronize()
+        assert sv.solve(b, p, raise_on_error=False) == (cyc, rel, st)
+        assert torch.equal(p, ref) and torch.equal(b, b0)
+        assert (pp[:op] == 7).all() and (pp[op + n:] == 7).all()
+    sv.close()
+    g.close()
