@@ -129,6 +129,7 @@ struct aw_solver {
     aw::DBuf<double> cgprm;
     bool use_graph = true;
     bool use_pdl = true;  // V-cycle kernels as programmatic dependent launches
+    bool full_next = false;  // the next of them starts after its predecessor has ended (launch_dep)
     int low = 1 << 30;    // first level of those that k_uni_low walks
     int tail = 0;         // first level of the uniform tail run as one k_dense_tail launch (0: none)
     double* h_norm = nullptr;  // pinned host words: a squared norm, uniform_check's counts
@@ -2107,9 +2108,10 @@ static Uniform uniform_of(aw_solver* S, int m) {
 }
 
 // A V-cycle kernel launch, as a programmatic dependent of the kernel before it in the stream (the
-// kernels call pdl_wait before reading what it wrote).
+// kernels call pdl_wait before reading what it wrote).  After uniform_check the first one is an ordinary
+// launch: the records' weights and masks, read before the wait, are what that launch's predecessor wrote.
 template <typename... KArgs, typename... Args>
-static aw_status launch_dep(const aw_solver* S, void (*k)(KArgs...), unsigned grid, unsigned block, size_t smem,
+static aw_status launch_dep(aw_solver* S, void (*k)(KArgs...), unsigned grid, unsigned block, size_t smem,
                             cudaStream_t s, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -2120,7 +2122,8 @@ static aw_status launch_dep(const aw_solver* S, void (*k)(KArgs...), unsigned gr
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = S->use_pdl ? 1 : 0;
+    cfg.numAttrs = S->use_pdl && !S->full_next ? 1 : 0;
+    S->full_next = false;
     AW_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...));
     AW_LAUNCH();
     return AW_OK;
@@ -2424,6 +2427,7 @@ static aw_status uniform_check(aw_solver* S, bool own_x0, cudaStream_t s) {
     AW_CUDA(cudaMemsetAsync(S->norm.p + 1, 0, UNI_MAX_LEVELS * sizeof(int), s));
     k_uni_check<<<dim3(grid, S->nmsbg), UNT, 0, s>>>(K);
     AW_LAUNCH();
+    S->full_next = true;
     return AW_OK;
 }
 

@@ -33,7 +33,8 @@ struct Coef3 {
 // predecessor drains.  A kernel reads what its predecessor wrote only after pdl_wait() (which returns
 // once the predecessor grid has completed and its memory is visible; at once for a kernel launched
 // without the attribute), and lets its successor start with pdl_trigger() once its own main work is
-// issued.  Descriptors and slot metadata (fixed at solver build) are staged before the wait.
+// issued.  Descriptors and slot metadata (fixed at solver build) are staged before the wait, and so are
+// k_uni_check's weights and masks: the launch after it is an ordinary one (launch_dep).
 __device__ inline void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ inline void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" :::); }
 
@@ -153,7 +154,8 @@ struct ULane {
     float wi, wx0, wx1, wy0, wy1, wz0, wz1;
     uint32_t mask;
     const int4* rec;
-    // the record, weights and mask are fixed before the launch's predecessors: read before the wait
+    // read before the wait: the record is fixed at solver build, and k_uni_check, which writes weights and mask,
+    // has ended before the first launch after it begins
     __device__ __forceinline__ bool init(const UniView& V, int warp) {
         lane = threadIdx.x & 31;
         const int li = lane % G::LPB, s = lane / G::LPB;

@@ -1,4 +1,6 @@
 """Which arrays the solver takes and what it leaves in its own."""
+import os
+
 import numpy as np
 import pytest
 
@@ -51,4 +53,59 @@ def test_arrays_that_start_at_any_element(R0, precision):
         assert torch.equal(p, ref) and torch.equal(b, b0)
         assert (pp[:op] == 7).all() and (pp[op + n:] == 7).all()
     sv.close()
+    g.close()
+
+
+def _solver(g, env=(), **kw):
+    for k in env:
+        os.environ[k] = "1"
+    try:
+        return aw.Solver(g, **kw)
+    finally:
+        for k in env:
+            os.environ.pop(k, None)
+
+
+@pytest.mark.parametrize("pre", [2, 0])
+@pytest.mark.parametrize("form", ["launched", "replayed", "captured"])
+def test_vcycle_sees_the_flags_and_coefficients_of_its_call(form, pre):
+    """Fluid flags and 1/rho change between two V-cycles: the kernels right behind the check of the blocks read
+    the new weights and masks, launched one by one, from the solver's graph and in a graph of the caller's."""
+    g = _grid()
+    n, _, b0 = _problem(g, 2)
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    X = g.face_positions(3)
+    steps = []
+    for k in range(6):
+        fluid = (X[:, k % 3] + 0.3 * X[:, (k + 1) % 3] < (3.0, 1.6, 2.5)[k % 3]).to(torch.uint8)
+        steps.append((fluid, None if k % 2 else 0.3 + 0.7 * torch.rand(g.channel(aw.BETA_COEFF_Y).numel(), generator=gen,
+                                                                      device="cuda")))
+    env = {"launched": ("AW_NO_GRAPH",), "staged": ("AW_NO_UNIFORM",)}
+
+    def run(form):
+        sv = _solver(g, env.get(form, ()), pre_smooth=pre)
+        x, b = sv.level_array(0, 0), sv.level_array(0, 1)
+        out, G = [], None
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            if form == "captured":
+                G = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(G, stream=s):
+                    sv.vcycle(stream=s.cuda_stream)
+            for fluid, beta in steps:
+                ch = g.channel(aw.BETA_COEFF_Y)
+                ch.fill_(1.0) if beta is None else ch.copy_(beta)
+                sv.update_coefficients(stream=s.cuda_stream)
+                sv.setup(fluid, stream=s.cuda_stream)
+                x.zero_()
+                b.copy_(b0 * fluid)
+                G.replay() if G else sv.vcycle(stream=s.cuda_stream)
+                out.append(x.clone())
+            s.synchronize()
+        del G
+        sv.close()
+        return out
+
+    for a, r in zip(run(form), run("staged")):
+        assert torch.equal(a, r)
     g.close()
