@@ -96,6 +96,7 @@ struct aw_solver {
     // activation or early exit)
     bool uni = false;
     unsigned gen = 0;  // bit m: level m has blocks without a single conductance (the current solve's check)
+    bool keep_r = true;  // the cycles store every level's residual (not those that precondition a CG solve)
     aw::DBuf<int4> uslab;  // slot records, weights, masks and warp descriptors of every level
     // mixed precision: FP64 vectors of the conjugate-gradient outer loop (residual, direction (two
     // buffers: the uniform form reads the old one while it writes the new), -A d), its scalars
@@ -937,7 +938,7 @@ __global__ void __launch_bounds__(256) k_cg_update(CgVec K, double* part, unsign
         }
         reinterpret_cast<double2*>(K.p)[i] = pv;
         reinterpret_cast<double2*>(K.r)[i] = rv;
-        reinterpret_cast<float2*>(K.rf)[i] = make_float2((float)rv.x, (float)rv.y);
+        reinterpret_cast<float2*>(K.rf)[i] = make_float2(f.x ? (float)rv.x : 0.f, f.y ? (float)rv.y : 0.f);
     }
     if (t0 == 0 && (K.n & 1) && K.fluid[K.n - 1]) {
         const size_t i = K.n - 1;
@@ -1550,7 +1551,9 @@ struct DenseTail {
     LevelView F;
     float* x;
     const float* b;
+    float* r;                 // nullptr: residuals are not stored
     DenseArgs lv[TAIL_MAX];   // uniform levels below, lv[n - 1] the coarsest
+    float *lx[TAIL_MAX], *lb[TAIL_MAX], *lr[TAIL_MAX];  // their x, b and r (the coarsest has none), stored on the way
     int low[TAIL_MAX];        // their places in shared memory, in floats behind the top's arrays
     int n;
     int pre, post, local;     // smoothing of the top: sweeps, updates of a cell per colour (MSBG)
@@ -1850,12 +1853,15 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) k_dense_tail(const __grid_con
         if (step == npre) {
 #pragma unroll
     for (int j = 0; j < 2 * TAIL_PAIRS; ++j) {
-        if (!((fl >> j) & 1u)) continue;
         const int i = j >> 1;
-        float v[6];
-        neighbours(i, j & 1, v);
-        rs[2 * (tid + i * TAIL_THREADS) + (odd[i] ^ (j & 1))] =
-            b[j] - (T.from_msbg ? tail_block_resid(w[j], v, diag[j], x[j]) : ufma(diag[j], x[j], tail_uniform(w[j], v)));
+        float r = 0.f;
+        if ((fl >> j) & 1u) {
+            float v[6];
+            neighbours(i, j & 1, v);
+            r = b[j] - (T.from_msbg ? tail_block_resid(w[j], v, diag[j], x[j]) : ufma(diag[j], x[j], tail_uniform(w[j], v)));
+            rs[2 * (tid + i * TAIL_THREADS) + (odd[i] ^ (j & 1))] = r;
+        }
+        if (T.r && ((act >> j) & 1u)) T.r[at[j]] = r;
     }
     __syncthreads();
     // ---- the levels below, by the warps that cover the first of them
@@ -1867,7 +1873,9 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) k_dense_tail(const __grid_con
             if (L.mine) {
                 const float* r = l == 0 ? rs : low + T.low[l - 1] + lattice_padded(T.lv[l - 1].d) + lattice_cells(T.lv[l - 1].d);
                 const float s = tail_restrict(r + L.child, l == 0 ? d0 : T.lv[l - 1].d);
-                L.b[tid] = L.fluid ? s : 0.f;
+                const float b = L.fluid ? s : 0.f;
+                L.b[tid] = b;
+                T.lb[l][tid] = b;
             }
             tail_bar(nt);
             if (l + 1 == T.n) break;
@@ -1875,7 +1883,9 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) k_dense_tail(const __grid_con
             if (L.mine) {
                 float v[6];
                 tail_nb(L.own, L.sy, L.sz, v);
-                L.r[tid] = L.fluid ? L.b[tid] - ufma(L.diag, *L.own, tail_uniform(L.w, v)) : 0.f;
+                const float r = L.fluid ? L.b[tid] - ufma(L.diag, *L.own, tail_uniform(L.w, v)) : 0.f;
+                L.r[tid] = r;
+                if (T.r) T.lr[l][tid] = r;
             }
             tail_bar(nt);
         }
@@ -1898,11 +1908,13 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) k_dense_tail(const __grid_con
                 } else {
                     tail_low_smooth(L, T.coarsest_iters, 0, T.omega, nt);
                 }
+                if (L.mine) T.lx[l][tid] = *L.own;
                 continue;
             }
             if (L.fluid) *L.own += (low + T.low[l + 1])[L.parent];
             tail_bar(nt);
             tail_low_smooth(L, T.sweeps, 1, T.omega, nt);
+            if (L.mine) T.lx[l][tid] = *L.own;
         }
     }
     __syncthreads();
@@ -2259,10 +2271,14 @@ static DenseTail tail_args(aw_solver* S) {
     if (!F.dense) T.F = lview(S, m);
     T.x = F.x.p;
     T.b = F.b.p;
+    T.r = S->keep_r ? F.r.p : nullptr;
     T.n = last - m;
     for (int j = 0; j < T.n; ++j) {
         MGLevel& L = S->lv[m + 1 + j];
         T.lv[j] = DenseArgs{dview(L), {L.W[0].p, L.W[1].p, L.W[2].p}, L.fluid.p};
+        T.lx[j] = L.x.p;
+        T.lb[j] = L.b.p;
+        T.lr[j] = L.r.p;
     }
     T.pre = F.dense ? S->d.dense_sweeps : S->d.pre_smooth;
     T.post = F.dense ? S->d.dense_sweeps : S->d.post_smooth;
@@ -2398,9 +2414,10 @@ static UX<HALF> ux(const XStore& x) {
     return UX<HALF>{x.f, x.h, x.scale};
 }
 
-// Weights, fluid masks and states of every block on every level.  Clears x of the blocks without fluid on
-// the levels whose x starts at zero (level 0 too with own_x0: then x0 is the solver's array), and both
-// direction buffers there.
+// Weights, fluid masks and states of every block on every level.  In the blocks without fluid, which the
+// kernels leave out, it clears r, and x and b where they are the solver's to write: on every level but the
+// finest, and there too with own_x0 (the preconditioner of a CG solve), with the vectors whose old
+// values a later kernel would read or add there: the directions, or the FP32 form's -A d.
 static aw_status uniform_check(aw_solver* S, bool own_x0, cudaStream_t s) {
     UCheckAll K{};
     unsigned grid = 1;
@@ -2409,7 +2426,9 @@ static aw_status uniform_check(aw_solver* S, bool own_x0, cudaStream_t s) {
         K.v[m] = uview(L, 2);
         UCheck& c = K.k[m];
         c.fluid = L.fluid.p;
+        c.r = L.r.p;
         if (m > 0 || own_x0) {
+            c.b = L.b.p;
             c.x = L.half ? nullptr : L.x.p;
             c.xh = L.half ? L.xh.p : nullptr;
             c.scale = L.xscale.p;
@@ -2418,6 +2437,7 @@ static aw_status uniform_check(aw_solver* S, bool own_x0, cudaStream_t s) {
             c.d0 = S->cg_d.p;
             c.d1 = S->cg_d2.p;
         }
+        if (m == 0 && own_x0 && S->d.precision == AW_PRECISION_FP32_PCG) c.q = S->cg32_q.p;
         c.wt = L.uwt;
         c.mask = L.umask;
         c.general = L.ugeneral;
@@ -2489,6 +2509,7 @@ static aw_status uni_low(aw_solver* S, int m, bool zero, cudaStream_t s) {
         const XStore x = xstore(S, k);
         K.lv[k] = ULowLevel{uview(L, 2), L.uwarps[0], x.f, x.h, x.scale, bptr(S, k), UOut{}};
         if (k < end) {
+            K.lv[k].out.r = S->keep_r ? L.r.p : nullptr;
             K.lv[k].out.bc = S->lv[k + 1].b.p;
             K.lv[k].out.fluid_c = S->lv[k + 1].fluid.p;
             gen = gen || ((S->gen >> k) & 1u);
@@ -2524,6 +2545,7 @@ static aw_status uni_low(aw_solver* S, int m, bool zero, cudaStream_t s) {
 // The V-cycle by the register-resident kernels: the steps of vcycle() with the
 // residual restricted as it is taken, levels starting at zero without a clearing pass (zero: this
 // level does), and the correction of an FP32 level added where its first post-smoothing reads it.
+// Every level's x and b, and with keep_r its r, hold afterwards what vcycle() leaves there.
 static aw_status uni_vcycle(aw_solver* S, int m, bool zero, cudaStream_t s) {
     const int last = (int)S->lv.size() - 1;
     MGLevel& L = S->lv[m];
@@ -2541,9 +2563,8 @@ static aw_status uni_vcycle(aw_solver* S, int m, bool zero, cudaStream_t s) {
     MGLevel& K = S->lv[m + 1];
     const XStore x = xstore(S, m);
     UOut out{};
-    if (K.dense) {
-        out.r = L.r.p;
-    } else {
+    if (S->keep_r || K.dense) out.r = L.r.p;
+    if (!K.dense) {
         out.bc = K.b.p;
         out.fluid_c = K.fluid.p;
     }
@@ -3091,6 +3112,7 @@ extern "C" aw_status aw_vcycle_run(aw_solver* S, aw_stream s) {
     AW_CHECK_ARG(S, "null solver");
     if (!S->uni) return vcycle(S, 0, (cudaStream_t)s);
     AW_TRY(uniform_check(S, false, (cudaStream_t)s));
+    S->keep_r = true;
     S->gen = (1u << S->nmsbg) - 1;  // no host read here: the kernels that take any block
     // replayed from a graph (a launch each costs the host more than the kernels take) from the second call
     // on (building it costs about one call), unless the caller is capturing this stream
@@ -3254,6 +3276,8 @@ static aw_status solve_aligned(aw_solver* S, const float* d_b, void* d_p, int32_
     }
     // reductions over the level-0 cells: at most 8 CTAs per SM, two cells per thread and step, grid-stride
     const unsigned ndot = (unsigned)std::max<size_t>(1, std::min<size_t>({(size_t)nsm * 8, nc / 512 + 1, S->partials.n}));
+    // (19 MB a cycle at poisson_256's size: 2860 to 2910 us a solve when the mixed form stored it)
+    S->keep_r = S->d.precision == AW_PRECISION_FP32;
     // the blocks' coefficients and masks, ||b||
     if (S->uni) AW_TRY(uniform_check(S, S->d.precision != AW_PRECISION_FP32, s));
     k_sumsq<<<ndot, 256, 0, s>>>(d_b, L0.fluid.p, nc, cf, S->partials.p, S->ticket.p, S->norm.p);

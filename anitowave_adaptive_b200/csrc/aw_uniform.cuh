@@ -826,7 +826,7 @@ __global__ void __launch_bounds__(UNT) k_uni_prolong(UniView V, UX<HALF> x, UX<H
 #undef AW_UB
 }
 
-// Where a residual goes: r (FP32) and / or r64, or, restricted (8-child sum on the coarse level's fluid
+// Where a residual goes: r (FP32), r64 and, restricted (8-child sum on the coarse level's fluid
 // cells), the coarse right-hand side.  dsum: partial sums of r^2, or of d . r for DOT.
 struct UOut {
     float* r;
@@ -1377,12 +1377,13 @@ __global__ void __launch_bounds__(UNT, 3) k_uni_apply(const __grid_constant__ Un
 // ------------------------------------------------------------------------------------------------
 // A block is uniform when every face between two of its cells has one conductance and every side of
 // the block has one; a block without fluid takes no part (its x is set to 0, which its neighbours
-// read).
+// read, and so are its b and r, as the staged kernels leave them).
 struct UCheck {
     const uint8_t* fluid;
     float* x;       // FP32 storage of the level's x to clear in air blocks (nullptr: keep)
     __half* xh;     // FP16 storage
     float* scale;
+    float *b, *r, *q;  // cleared there too (nullptr: keep)
     double *d0, *d1;  // FP64 vectors to clear there too
     float4* wt;
     uint16_t* mask;
@@ -1458,6 +1459,9 @@ __device__ __forceinline__ void uni_check_body(const UniView& V, const UCheck& K
                 const uint32_t c = off + (uint32_t)(G::NI * xp + i + R * (y + R * z));
                 if (K.x) K.x[c] = 0.f;
                 if (K.xh) K.xh[c] = __float2half_rn(0.f);
+                if (K.b) K.b[c] = 0.f;
+                K.r[c] = 0.f;
+                if (K.q) K.q[c] = 0.f;
                 if (K.d0) K.d0[c] = K.d1[c] = 0.0;
             }
         if (K.xh && li == 0) K.scale[rec[1]] = 0.f;

@@ -247,13 +247,17 @@ aw_status aw_mg_prolongate(aw_solver* sv, int32_t level, aw_stream s);
 /* coarsest-level solve (VCycle.cuh:252-256): FP64 dense solve of the uniform coarsest level in FV
  * mode, coarsest_iterations smoother iterations in reference mode */
 aw_status aw_solver_coarsest_solve(aw_solver* sv, aw_stream s);
-/* VCycleSolver::runCycle(mg, 0) (VCycle.cuh:251-304) on the level-0 arrays x, b */
+/* VCycleSolver::runCycle(mg, 0) (VCycle.cuh:251-304) on the level-0 arrays x, b.  Afterwards every level
+ * holds the cycle's x, b and r (r: the residual that was restricted; the coarsest level has none). */
 aw_status aw_vcycle_run(aw_solver* sv, aw_stream s);
 /* Solve A p = b on level 0 to desc.tolerance.  FP32 precision: p is float*, V-cycles in place.
  * Mixed precision: p is double*, outer defect correction with the FP64 residual, FP64
  * accumulation and FP64 coarsest solve; V-cycle in FP32 with FP16 coarse corrections.
  * d_b and d_p may start at any element; 16-byte aligned arrays are used in place, others through
  * a copy that the solver keeps.
+ * The level arrays are the cycles' work space: afterwards they hold the last cycle's x, b and r, but r only
+ * with FP32 precision (level 0: the final b - A p); the cycles that precondition _MIXED and _FP32_PCG restrict
+ * a residual without storing it.
  * syncs (one residual norm read per cycle).  Returns AW_ERR_NOT_CONVERGED if max_cycles ran out. */
 aw_status aw_solve(aw_solver* sv, const float* d_b, void* d_p, int32_t* cycles, double* final_rel, aw_stream s);
 /* pressure-gradient update of VELOCITY_*: u -= dt (W/area) (p_high - p_low) on faces with a fluid

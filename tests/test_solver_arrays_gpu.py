@@ -1,4 +1,5 @@
 """Which arrays the solver takes and what it leaves in its own."""
+import ctypes as C
 import os
 
 import numpy as np
@@ -108,4 +109,107 @@ def test_vcycle_sees_the_flags_and_coefficients_of_its_call(form, pre):
 
     for a, r in zip(run(form), run("staged")):
         assert torch.equal(a, r)
+    g.close()
+
+
+STAGED = ("AW_NO_UNIFORM", "AW_NO_UNIFORM_LOW", "AW_NO_DENSE_TAIL")
+GRIDS = {  # one-cell blocks: 45 (odd), 256 (the tail's top), 32768 (uniform levels of 4096 cells and below)
+    "odd": lambda: _grid(),
+    "tail": lambda: _grid(8, (8, 8, 4)),
+    "uniform": lambda: _even(2, (32, 32, 32)),
+}
+
+
+def _even(R0, dims):
+    g = aw.MSBG(dims, 1.0, (0.0, 0.0, 0.0), R0, 2)
+    g.set_refinement_map(np.asarray([(i // 7) % 2 for i in range(int(np.prod(dims)))], np.uint32))
+    g.enforce_grading()
+    g.allocate()
+    return g
+
+
+def _levels(sv, precision):
+    """x, b, r and fluid flags of every level (r not on the coarsest; FP16 x without its scales)."""
+    out, nl = {}, sv.num_levels()
+    for m in range(nl):
+        try:
+            res = int(sv.level_array(m, 11).max())
+        except aw.AWError:  # a uniform level
+            res = 1
+        for which in (0, 1, 2, 6):
+            if which == 2 and m + 1 == nl:
+                continue
+            if which == 0 and precision == aw.PRECISION_MIXED and m > 0 and res > 1:
+                p, n = C.c_void_p(), C.c_uint32()
+                aw.check(aw.lib().aw_solver_level_array(sv.h, m, 0, C.byref(p), C.byref(n)))
+                out[m, which] = aw._tensor_from_ptr(p.value, n.value, torch.float16).clone()
+            else:
+                out[m, which] = sv.level_array(m, which).clone()
+    torch.cuda.synchronize()
+    return out
+
+
+def _cut(X, cut):
+    return (X[:, 0] + 0.3 * X[:, 1] < cut * float(X[:, 0].max())).to(torch.uint8)
+
+
+@pytest.mark.parametrize("name", list(GRIDS))
+@pytest.mark.parametrize("precision", [aw.PRECISION_FP32, aw.PRECISION_MIXED])
+def test_vcycle_leaves_every_levels_arrays(name, precision):
+    """x, b and r of all levels after aw_vcycle_run: the register-resident, one-launch forms leave the bits of the
+    staged ones, in blocks that lose their fluid from one call to the next too."""
+    g = GRIDS[name]()
+    n, _, b0 = _problem(g, 3)
+    X = g.face_positions(3)
+    got = []
+    for env in (), STAGED:
+        sv = _solver(g, env, precision=precision)
+        x, b = sv.level_array(0, 0), sv.level_array(0, 1)
+        for cut in (0.9, 0.6, 0.25):
+            fluid = _cut(X, cut)
+            sv.setup(fluid)
+            x.zero_()
+            b.copy_(b0 * fluid)
+            torch.cuda.synchronize()
+            sv.vcycle()
+            torch.cuda.synchronize()
+            got.append(_levels(sv, precision))
+        sv.close()
+    for a, r in zip(got[:3], got[3:]):
+        assert a.keys() == r.keys()
+        for k in a:
+            assert torch.equal(a[k], r[k]), k
+    g.close()
+
+
+@pytest.mark.parametrize("name", list(GRIDS))
+@pytest.mark.parametrize("precision", ALL)
+def test_solve_leaves_every_levels_arrays(name, precision):
+    """... and after aw_solve those of its last cycle, r in the FP32 form.  The mixed form's FP64 sums have another order: a relative
+    change of some 1e-16 a scalar, at most an FP32 rounding here (bar 1e-5 of an array's largest value, FP16 x left
+    out), and exact zeros without fluid."""
+    g = GRIDS[name]()
+    n, _, b0 = _problem(g, 4)
+    X = g.face_positions(3)
+    got = []
+    for env in (), STAGED:
+        sv = _solver(g, env, precision=precision, tolerance=1e-30, max_cycles=2)
+        for cut in (0.9, 0.4):
+            fluid = _cut(X, cut)
+            sv.setup(fluid)
+            p = torch.zeros(n, dtype=torch.float64 if precision == aw.PRECISION_MIXED else torch.float32, device="cuda")
+            sv.solve(b0 * fluid, p, raise_on_error=False)
+            got.append(_levels(sv, precision))
+        sv.close()
+    for a, r in zip(got[:2], got[2:]):
+        for k in a:
+            if precision != aw.PRECISION_FP32 and k[1] == 2:
+                continue
+            if precision != aw.PRECISION_MIXED or k[1] == 6:
+                assert torch.equal(a[k], r[k]), k
+            elif a[k].dtype == torch.float32:
+                d = (a[k] - r[k]).abs().max()
+                assert d <= 1e-5 * r[k].abs().max(), (k, d)
+                air = a[k[0], 6] == 0
+                assert not a[k][air].any() and not r[k][air].any(), k
     g.close()
