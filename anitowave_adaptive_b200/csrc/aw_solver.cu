@@ -3110,9 +3110,9 @@ extern "C" aw_status aw_solver_coarsest_solve(aw_solver* S, aw_stream s) {
 }
 extern "C" aw_status aw_vcycle_run(aw_solver* S, aw_stream s) {
     AW_CHECK_ARG(S, "null solver");
+    S->keep_r = true;
     if (!S->uni) return vcycle(S, 0, (cudaStream_t)s);
     AW_TRY(uniform_check(S, false, (cudaStream_t)s));
-    S->keep_r = true;
     S->gen = (1u << S->nmsbg) - 1;  // no host read here: the kernels that take any block
     // replayed from a graph (a launch each costs the host more than the kernels take) from the second call
     // on (building it costs about one call), unless the caller is capturing this stream

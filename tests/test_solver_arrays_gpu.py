@@ -213,3 +213,24 @@ def test_solve_leaves_every_levels_arrays(name, precision):
                 air = a[k[0], 6] == 0
                 assert not a[k][air].any() and not r[k][air].any(), k
     g.close()
+
+
+@pytest.mark.parametrize("env", [(), ("AW_NO_UNIFORM",)])
+def test_vcycle_after_a_solve_leaves_every_levels_arrays(env):
+    """A mixed solve's cycles do not store r; a call after it does, in the tail's levels too."""
+    g = GRIDS["tail"]()
+    n, fluid, b0 = _problem(g, 5)
+    got = []
+    for e in env, STAGED:
+        sv = _solver(g, e, precision=aw.PRECISION_MIXED, tolerance=1e-30, max_cycles=1)
+        sv.setup(fluid)
+        sv.solve(b0, torch.zeros(n, dtype=torch.float64, device="cuda"), raise_on_error=False)
+        sv.level_array(0, 0).zero_()
+        sv.level_array(0, 1).copy_(b0)
+        torch.cuda.synchronize()
+        sv.vcycle()
+        torch.cuda.synchronize()
+        got.append(_levels(sv, aw.PRECISION_MIXED))
+        sv.close()
+    assert all(torch.equal(got[0][k], got[1][k]) for k in got[1])
+    g.close()
