@@ -295,7 +295,6 @@ static aw_status radix_sort_pairs(const SortPlan& P, ParticleWork& W, int64_t n,
     const uint32_t* kin = W.keys.p;
     const uint32_t* vin = nullptr;
     uint32_t *kout = W.keys2.p, *vout = W.perm.p;
-    unsigned* ticket = reinterpret_cast<unsigned*>(W.hscan.p + 2 * RADIX_MAX_BINS);
     const size_t ssm = (size_t)P.bins * (sizeof(uint32_t) + SORT_WARPS * sizeof(uint16_t));
     AW_CUDA(cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(RADIX_MAX_BINS * (sizeof(uint32_t) + SORT_WARPS * sizeof(uint16_t)))));
@@ -306,7 +305,7 @@ static aw_status radix_sort_pairs(const SortPlan& P, ParticleWork& W, int64_t n,
             AW_LAUNCH();
         }
         k_radix_rows<<<(P.bins + 7) / 8, 256, 0, s>>>(W.hist.p, P.ntiles, P.bins, W.hscan.p, W.hscan.p + RADIX_MAX_BINS,
-                                                      ticket);
+                                                      W.ticket);
         AW_LAUNCH();
         k_radix_scatter<<<P.ntiles, SORT_THREADS, ssm, s>>>(kin, vin, p + 1 < P.passes ? kout : nullptr, vout, n, shift,
                                                             P.bins, P.tile, W.hist.p, W.hscan.p + RADIX_MAX_BINS, P.ntiles);
@@ -387,11 +386,11 @@ __device__ inline void hash_block_add(unsigned long long hp, unsigned long long 
 }
 
 // gather pos/vel into SoA sorted order, carry the original ids; with hash, the content hashes of the
-// input positions and velocities into hash[0], hash[1] (partial sums behind hash[4])
+// input positions and velocities into hash[0], hash[1] (partial sums in part)
 __global__ void k_gather(const uint32_t* __restrict__ src, int64_t n, PArr pos, PArr vel, float* __restrict__ soa,
                          const uint32_t* __restrict__ ids_in, uint32_t* __restrict__ ids_out,
                          const uint32_t* __restrict__ keys, uint32_t* __restrict__ keys_sorted,
-                         unsigned long long* hash = nullptr) {
+                         unsigned long long* hash = nullptr, unsigned long long* part = nullptr) {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long hp = 0, hv = 0;
     if (j < n) {
@@ -411,7 +410,7 @@ __global__ void k_gather(const uint32_t* __restrict__ src, int64_t n, PArr pos, 
         if (ids_out) ids_out[j] = ids_in ? ids_in[i] : i;
         if (keys_sorted) keys_sorted[j] = keys[i];
     }
-    if (hash) hash_block_add(hp, hv, hash + 4, hash);  // uniform across the CTA
+    if (hash) hash_block_add(hp, hv, part, hash);  // uniform across the CTA
 }
 
 // Content hashes of AoS positions and, when given, velocities into hash[2], hash[3].  Four particles per
@@ -430,7 +429,7 @@ __device__ __forceinline__ void hash_load4(const float* __restrict__ p, int64_t 
     }
 }
 __global__ void __launch_bounds__(256) k_hash_aos(const float* __restrict__ pos, const float* __restrict__ vel, int64_t n,
-                                                  unsigned long long* hash) {
+                                                  unsigned long long* hash, unsigned long long* part) {
     unsigned long long hp = 0, hv = 0;
     const bool wp = ((uintptr_t)pos & 15u) == 0, wv = ((uintptr_t)vel & 15u) == 0;
     const int64_t nq = n / 4, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
@@ -449,7 +448,7 @@ __global__ void __launch_bounds__(256) k_hash_aos(const float* __restrict__ pos,
         hp += hash3((uint32_t)i, pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]);
         if (vel) hv += hash3((uint32_t)i, vel[3 * i], vel[3 * i + 1], vel[3 * i + 2]);
     }
-    hash_block_add(hp, hv, hash + 4, hash + 2);
+    hash_block_add(hp, hv, part, hash + 2);
 }
 
 // the caller's arrays still hold what the last aw_p2g sorted (positions; velocities too if asked)
@@ -462,7 +461,10 @@ aw_status ParticleWork::ensure(int64_t np, uint32_t ncell) {
     AW_TRY(perm.ensure((size_t)np));
     AW_TRY(perm2.ensure((size_t)np));
     AW_TRY(cell_start.ensure((size_t)ncell + 2));
-    AW_TRY(cell_fill.ensure((size_t)ncell + 2));
+    const size_t at = ((size_t)ncell + 3) & ~size_t(1);  // behind the counts, on 8 bytes
+    AW_TRY(cell_fill.ensure(at + 2 + 2 * (2 * kHashSlots + 1)));
+    ticket = cell_fill.p + at;
+    hash_part = reinterpret_cast<unsigned long long*>(cell_fill.p + at + 2);
     AW_TRY(soa.ensure((size_t)np * 6 + kSoaPad));
     AW_TRY(soa2.ensure((size_t)np * 6 + kSoaPad));
     n = np;
@@ -475,24 +477,23 @@ aw_status ParticleWork::ensure(int64_t np, uint32_t ncell) {
 aw_status sort_core(MsbgState& G, PArr pos, int64_t n, cudaStream_t s) {
     uint32_t nc = G.tot[0];
     ParticleWork& W = G.pw;
+    W.src_valid = false;  // the recorded order of aw_p2g is replaced
     AW_TRY(W.ensure(n, nc));
-    AW_CUDA(cudaMemsetAsync(W.cell_fill.p, 0, ((size_t)nc + 2) * sizeof(uint32_t), s));
+    // the counts, and behind them everything that has to be 0 when a kernel counts its CTAs or adds into it
+    AW_CUDA(cudaMemsetAsync(W.cell_fill.p, 0,
+                            reinterpret_cast<char*>(W.hash_part + 2 * kHashSlots + 1) - reinterpret_cast<char*>(W.cell_fill.p), s));
     const SortPlan P = sort_plan(n, nc);
     if (n > 0) {
         AW_TRY(W.keys2.ensure((size_t)n));
         if (P.passes > 2) AW_TRY(W.keys3.ensure((size_t)n));
         AW_TRY(W.hist.ensure((size_t)P.bins * P.ntiles));
-        if (!W.hscan.p) {
-            AW_TRY(W.hscan.ensure(2 * RADIX_MAX_BINS + 1));
-            AW_CUDA(cudaMemsetAsync(W.hscan.p, 0, (2 * RADIX_MAX_BINS + 1) * sizeof(uint32_t), s));
-        }
+        AW_TRY(W.hscan.ensure(2 * RADIX_MAX_BINS));
         k_keys<<<P.ntiles, KEYS_THREADS, 0, s>>>(G.view0(), pos, n, nc, W.keys.p, W.cell_fill.p, P.bins, P.tile, W.hist.p,
                                                  P.ntiles);
         AW_LAUNCH();
     }
     AW_TRY(exclusive_scan_u32(W.cell_fill.p, W.cell_start.p, (size_t)nc + 1, W.tmp, s));
     W.sorted = W.perm.p;
-    W.src_valid = false;  // the recorded order of aw_p2g is replaced
     if (n > 0) AW_TRY(radix_sort_pairs(P, W, n, &W.sorted, s));
     return AW_OK;
 }
@@ -504,14 +505,12 @@ aw_status sort_particles_soa(MsbgState& G, const float* pos_aos, const float* ve
     ParticleWork& W = G.pw;
     unsigned long long* hash = nullptr;
     if (record) {
-        if (!W.hash.p) {
-            AW_TRY(W.hash.ensure(4 + 2 * kHashSlots + 1));
-            AW_CUDA(cudaMemsetAsync(W.hash.p, 0, W.hash.n * sizeof(unsigned long long), s));
-        }
+        AW_TRY(W.hash.ensure(4));
         hash = W.hash.p;
     }
     if (n > 0) {
-        k_gather<<<nblk(n), 256, 0, s>>>(W.sorted, n, pos, vel, W.soa.p, nullptr, nullptr, nullptr, nullptr, hash);
+        k_gather<<<nblk(n), 256, 0, s>>>(W.sorted, n, pos, vel, W.soa.p, nullptr, nullptr, nullptr, nullptr, hash,
+                                         W.hash_part);
         AW_LAUNCH();
     }
     if (record) {
@@ -2825,7 +2824,7 @@ extern "C" aw_status aw_g2p(aw_msbg* g, float* d_vel, const float* d_pos, int64_
     AW_TRY(ensure_tiles(G));
     const unsigned long long* skip = nullptr;
     if (W.src_valid && W.src_pos == d_pos && W.src_vel == d_vel && W.src_n == n) {
-        k_hash_aos<<<std::min(nblk(n / 4 + 1), 8u * 148u), 256, 0, s>>>(d_pos, d_vel, n, W.hash.p);
+        k_hash_aos<<<std::min(nblk(n / 4 + 1), 8u * 148u), 256, 0, s>>>(d_pos, d_vel, n, W.hash.p, W.hash_part);
         AW_LAUNCH();
         int maxres = 0;
         for (int r : G.h_res) maxres = std::max(maxres, r);
@@ -2861,7 +2860,7 @@ extern "C" aw_status aw_advect(aw_msbg* g, float* d_pos, int64_t n, float dt, aw
     AW_TRY(build_tiles(G, u, G.tiles_new.p, s));  // both paths sample neighbouring blocks' u_new tiles
     const unsigned long long* skip = nullptr;
     if (W.src_valid && W.src_pos == d_pos && W.src_n == n) {
-        k_hash_aos<<<std::min(nblk(n / 4 + 1), 8u * 148u), 256, 0, s>>>(d_pos, nullptr, n, W.hash.p);
+        k_hash_aos<<<std::min(nblk(n / 4 + 1), 8u * 148u), 256, 0, s>>>(d_pos, nullptr, n, W.hash.p, W.hash_part);
         AW_LAUNCH();
         int maxres = 0;
         for (int r : G.h_res) maxres = std::max(maxres, r);
