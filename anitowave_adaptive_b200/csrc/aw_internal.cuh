@@ -185,16 +185,14 @@ struct ParticleWork {
     int64_t n = 0;
     // The particle arrays the last aw_p2g sorted (caller pointers and count) and 64-bit hashes of
     // their contents then: hash[0] positions, hash[1] velocities; hash[2..3] receive the hashes of
-    // the arrays at a later drop-in G2P or advection, which reuses this sort when they match.
+    // the arrays at a later drop-in G2P or advection, which reuses this sort when they match;
+    // hash[4..] holds the partial sums of the hashing kernels and their CTA ticket, and the end of hscan
+    // the one of the sort's row scan: cleared by every sort, 0 between kernels.
     const float* src_pos = nullptr;
     const float* src_vel = nullptr;
     int64_t src_n = -1;
     bool src_valid = false;
     DBuf<unsigned long long> hash;
-    // CTA ticket of the sort's row scan, partial sums and ticket of the hashing kernels: behind the counts in
-    // cell_fill, cleared with them by every sort and left at 0 by every kernel that uses them
-    uint32_t* ticket = nullptr;
-    unsigned long long* hash_part = nullptr;
     aw_status ensure(int64_t np, uint32_t ncell);
 };
 

@@ -100,12 +100,20 @@ __device__ __forceinline__ void hist_add(uint32_t* h, uint32_t dig, unsigned act
     if ((__ffs(peers) - 1) == (int)(threadIdx.x & 31)) atomicAdd(&h[dig], (uint32_t)__popc(peers));
 }
 
+// Content hashes (below): their partial sums lie in kHashSlots slot pairs, a CTA ticket behind them
+constexpr int kHashSlots = 128, kHashPart = 2 * kHashSlots + 1;
+
 // keys, the particle count of every cell, and the first pass's tile histograms
 constexpr int KEYS_THREADS = 512;
 __global__ void __launch_bounds__(KEYS_THREADS) k_keys(LevelView L, PArr pos, int64_t n, uint32_t invalid, uint32_t* keys,
                                                        uint32_t* count, int bins, int64_t tile, uint32_t* __restrict__ hist,
-                                                       uint32_t ntiles) {
+                                                       uint32_t ntiles, uint32_t* ticket, unsigned long long* part) {
     __shared__ uint32_t h[RADIX_MAX_BINS];
+    // what the sort and the hashing kernels count their CTAs in or add to starts at 0 (they leave it so)
+    if (blockIdx.x == 0) {
+        for (int i = threadIdx.x; i < kHashPart; i += KEYS_THREADS) part[i] = 0ull;
+        if (threadIdx.x == 0) *ticket = 0u;
+    }
     for (int i = threadIdx.x; i < bins; i += KEYS_THREADS) h[i] = 0;
     __syncthreads();
     const int64_t i0 = (int64_t)blockIdx.x * tile, i1 = min(i0 + tile, n);
@@ -305,7 +313,7 @@ static aw_status radix_sort_pairs(const SortPlan& P, ParticleWork& W, int64_t n,
             AW_LAUNCH();
         }
         k_radix_rows<<<(P.bins + 7) / 8, 256, 0, s>>>(W.hist.p, P.ntiles, P.bins, W.hscan.p, W.hscan.p + RADIX_MAX_BINS,
-                                                      W.ticket);
+                                                      W.hscan.p + 2 * RADIX_MAX_BINS);
         AW_LAUNCH();
         k_radix_scatter<<<P.ntiles, SORT_THREADS, ssm, s>>>(kin, vin, p + 1 < P.passes ? kout : nullptr, vout, n, shift,
                                                             P.bins, P.tile, W.hist.p, W.hscan.p + RADIX_MAX_BINS, P.ntiles);
@@ -341,7 +349,6 @@ __device__ inline unsigned long long warp_sum_u64(unsigned long long v) {
 // Hash partial sums land in kHashSlots slot pairs (CTA b in slot b mod kHashSlots), so that the
 // atomics of many CTAs do not queue on one address.  The CTA that finishes last adds the slots into
 // out[0], out[1] and clears slots and ticket for the next use.
-constexpr int kHashSlots = 128;
 __device__ inline void hash_block_add(unsigned long long hp, unsigned long long hv, unsigned long long* slots,
                                       unsigned long long* out) {
     __shared__ unsigned long long red[2][32];
@@ -386,11 +393,11 @@ __device__ inline void hash_block_add(unsigned long long hp, unsigned long long 
 }
 
 // gather pos/vel into SoA sorted order, carry the original ids; with hash, the content hashes of the
-// input positions and velocities into hash[0], hash[1] (partial sums in part)
+// input positions and velocities into hash[0], hash[1] (partial sums behind hash[4])
 __global__ void k_gather(const uint32_t* __restrict__ src, int64_t n, PArr pos, PArr vel, float* __restrict__ soa,
                          const uint32_t* __restrict__ ids_in, uint32_t* __restrict__ ids_out,
                          const uint32_t* __restrict__ keys, uint32_t* __restrict__ keys_sorted,
-                         unsigned long long* hash = nullptr, unsigned long long* part = nullptr) {
+                         unsigned long long* hash = nullptr) {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long hp = 0, hv = 0;
     if (j < n) {
@@ -410,7 +417,7 @@ __global__ void k_gather(const uint32_t* __restrict__ src, int64_t n, PArr pos, 
         if (ids_out) ids_out[j] = ids_in ? ids_in[i] : i;
         if (keys_sorted) keys_sorted[j] = keys[i];
     }
-    if (hash) hash_block_add(hp, hv, part, hash);  // uniform across the CTA
+    if (hash) hash_block_add(hp, hv, hash + 4, hash);  // uniform across the CTA
 }
 
 // Content hashes of AoS positions and, when given, velocities into hash[2], hash[3].  Four particles per
@@ -429,7 +436,7 @@ __device__ __forceinline__ void hash_load4(const float* __restrict__ p, int64_t 
     }
 }
 __global__ void __launch_bounds__(256) k_hash_aos(const float* __restrict__ pos, const float* __restrict__ vel, int64_t n,
-                                                  unsigned long long* hash, unsigned long long* part) {
+                                                  unsigned long long* hash) {
     unsigned long long hp = 0, hv = 0;
     const bool wp = ((uintptr_t)pos & 15u) == 0, wv = ((uintptr_t)vel & 15u) == 0;
     const int64_t nq = n / 4, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
@@ -448,7 +455,7 @@ __global__ void __launch_bounds__(256) k_hash_aos(const float* __restrict__ pos,
         hp += hash3((uint32_t)i, pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]);
         if (vel) hv += hash3((uint32_t)i, vel[3 * i], vel[3 * i + 1], vel[3 * i + 2]);
     }
-    hash_block_add(hp, hv, part, hash + 2);
+    hash_block_add(hp, hv, hash + 4, hash + 2);
 }
 
 // the caller's arrays still hold what the last aw_p2g sorted (positions; velocities too if asked)
@@ -461,10 +468,7 @@ aw_status ParticleWork::ensure(int64_t np, uint32_t ncell) {
     AW_TRY(perm.ensure((size_t)np));
     AW_TRY(perm2.ensure((size_t)np));
     AW_TRY(cell_start.ensure((size_t)ncell + 2));
-    const size_t at = ((size_t)ncell + 3) & ~size_t(1);  // behind the counts, on 8 bytes
-    AW_TRY(cell_fill.ensure(at + 2 + 2 * (2 * kHashSlots + 1)));
-    ticket = cell_fill.p + at;
-    hash_part = reinterpret_cast<unsigned long long*>(cell_fill.p + at + 2);
+    AW_TRY(cell_fill.ensure((size_t)ncell + 2));
     AW_TRY(soa.ensure((size_t)np * 6 + kSoaPad));
     AW_TRY(soa2.ensure((size_t)np * 6 + kSoaPad));
     n = np;
@@ -479,17 +483,16 @@ aw_status sort_core(MsbgState& G, PArr pos, int64_t n, cudaStream_t s) {
     ParticleWork& W = G.pw;
     W.src_valid = false;  // the recorded order of aw_p2g is replaced
     AW_TRY(W.ensure(n, nc));
-    // the counts, and behind them everything that has to be 0 when a kernel counts its CTAs or adds into it
-    AW_CUDA(cudaMemsetAsync(W.cell_fill.p, 0,
-                            reinterpret_cast<char*>(W.hash_part + 2 * kHashSlots + 1) - reinterpret_cast<char*>(W.cell_fill.p), s));
+    AW_CUDA(cudaMemsetAsync(W.cell_fill.p, 0, ((size_t)nc + 2) * sizeof(uint32_t), s));
     const SortPlan P = sort_plan(n, nc);
     if (n > 0) {
         AW_TRY(W.keys2.ensure((size_t)n));
         if (P.passes > 2) AW_TRY(W.keys3.ensure((size_t)n));
         AW_TRY(W.hist.ensure((size_t)P.bins * P.ntiles));
-        AW_TRY(W.hscan.ensure(2 * RADIX_MAX_BINS));
+        AW_TRY(W.hscan.ensure(2 * RADIX_MAX_BINS + 1));
+        AW_TRY(W.hash.ensure(4 + kHashPart));
         k_keys<<<P.ntiles, KEYS_THREADS, 0, s>>>(G.view0(), pos, n, nc, W.keys.p, W.cell_fill.p, P.bins, P.tile, W.hist.p,
-                                                 P.ntiles);
+                                                 P.ntiles, W.hscan.p + 2 * RADIX_MAX_BINS, W.hash.p + 4);
         AW_LAUNCH();
     }
     AW_TRY(exclusive_scan_u32(W.cell_fill.p, W.cell_start.p, (size_t)nc + 1, W.tmp, s));
@@ -503,14 +506,9 @@ aw_status sort_particles_soa(MsbgState& G, const float* pos_aos, const float* ve
     PArr pos{pos_aos, 3, 1}, vel{vel_aos, 3, 1};
     AW_TRY(sort_core(G, pos, n, s));
     ParticleWork& W = G.pw;
-    unsigned long long* hash = nullptr;
-    if (record) {
-        AW_TRY(W.hash.ensure(4));
-        hash = W.hash.p;
-    }
+    unsigned long long* hash = record ? W.hash.p : nullptr;
     if (n > 0) {
-        k_gather<<<nblk(n), 256, 0, s>>>(W.sorted, n, pos, vel, W.soa.p, nullptr, nullptr, nullptr, nullptr, hash,
-                                         W.hash_part);
+        k_gather<<<nblk(n), 256, 0, s>>>(W.sorted, n, pos, vel, W.soa.p, nullptr, nullptr, nullptr, nullptr, hash);
         AW_LAUNCH();
     }
     if (record) {
@@ -2824,7 +2822,7 @@ extern "C" aw_status aw_g2p(aw_msbg* g, float* d_vel, const float* d_pos, int64_
     AW_TRY(ensure_tiles(G));
     const unsigned long long* skip = nullptr;
     if (W.src_valid && W.src_pos == d_pos && W.src_vel == d_vel && W.src_n == n) {
-        k_hash_aos<<<std::min(nblk(n / 4 + 1), 8u * 148u), 256, 0, s>>>(d_pos, d_vel, n, W.hash.p, W.hash_part);
+        k_hash_aos<<<std::min(nblk(n / 4 + 1), 8u * 148u), 256, 0, s>>>(d_pos, d_vel, n, W.hash.p);
         AW_LAUNCH();
         int maxres = 0;
         for (int r : G.h_res) maxres = std::max(maxres, r);
@@ -2860,7 +2858,7 @@ extern "C" aw_status aw_advect(aw_msbg* g, float* d_pos, int64_t n, float dt, aw
     AW_TRY(build_tiles(G, u, G.tiles_new.p, s));  // both paths sample neighbouring blocks' u_new tiles
     const unsigned long long* skip = nullptr;
     if (W.src_valid && W.src_pos == d_pos && W.src_n == n) {
-        k_hash_aos<<<std::min(nblk(n / 4 + 1), 8u * 148u), 256, 0, s>>>(d_pos, nullptr, n, W.hash.p, W.hash_part);
+        k_hash_aos<<<std::min(nblk(n / 4 + 1), 8u * 148u), 256, 0, s>>>(d_pos, nullptr, n, W.hash.p);
         AW_LAUNCH();
         int maxres = 0;
         for (int r : G.h_res) maxres = std::max(maxres, r);
