@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <string>
+#include <mutex>
 #include <vector>
 
 #include "anitowave.h"
@@ -41,6 +42,20 @@ extern unsigned long long g_launches;
     do {                                                                    \
         if (!(cond)) return ::aw::set_error(AW_ERR_INVALID_ARGUMENT, "%s", msg); \
     } while (0)
+
+// Lets kernel K be launched with `bytes` of dynamic shared memory.  The limit belongs to the kernel, not to a
+// grid or solver, so it only grows: one of smaller blocks, or another thread, takes nothing from a launch
+// that was set up with more.
+template <auto K>
+aw_status allow_smem(size_t bytes) {
+    static std::mutex lock;
+    static size_t most = 0;
+    std::lock_guard<std::mutex> hold(lock);
+    const size_t want = bytes > most ? bytes : most;
+    AW_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want));
+    most = want;
+    return AW_OK;
+}
 
 // ------------------------------------------------------------------------------------------------
 // Device buffers

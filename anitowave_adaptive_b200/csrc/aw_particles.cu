@@ -304,8 +304,7 @@ static aw_status radix_sort_pairs(const SortPlan& P, ParticleWork& W, int64_t n,
     const uint32_t* vin = nullptr;
     uint32_t *kout = W.keys2.p, *vout = W.perm.p;
     const size_t ssm = (size_t)P.bins * (sizeof(uint32_t) + SORT_WARPS * sizeof(uint16_t));
-    AW_CUDA(cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(RADIX_MAX_BINS * (sizeof(uint32_t) + SORT_WARPS * sizeof(uint16_t)))));
+    AW_TRY(allow_smem<k_radix_scatter>(ssm));
     for (int p = 0; p < P.passes; ++p) {
         const int shift = p * P.digit;
         if (p > 0) {
@@ -1428,11 +1427,11 @@ aw_status p2g_sorted(MsbgState& G, const float* soa, int64_t n, const uint32_t* 
     if (n > 0) {
         if (ph) {
             // always opted in: the pair queues' static shared memory counts against the default 48 KB too
-            AW_CUDA(cudaFuncSetAttribute(k_p2g_own<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            AW_TRY(allow_smem<k_p2g_own<true>>(smem));
             k_p2g_own<true><<<G.nb, nthreads, smem, s>>>(G.view0(), soa, n, cstart, acc, ph->pid, ph->phase,
                                                            (int)smem_f, G.blk_busy.p, order);
         } else {
-            AW_CUDA(cudaFuncSetAttribute(k_p2g_own<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            AW_TRY(allow_smem<k_p2g_own<false>>(smem));
             k_p2g_own<false><<<G.nb, nthreads, smem, s>>>(G.view0(), soa, n, cstart, acc, nullptr, nullptr,
                                                             (int)smem_f, G.blk_busy.p, order);
         }
@@ -2203,7 +2202,7 @@ aw_status g2p_sorted(MsbgState& G, float* soa, int64_t n, const uint32_t* cs, fl
     int maxres = 0;
     for (int r : G.h_res) maxres = std::max(maxres, r);
     const size_t smem = ((size_t)tile_block(maxres) + 2 * 6 * G2P_SLOT) * sizeof(float);
-    AW_CUDA(cudaFuncSetAttribute(k_g2p_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    AW_TRY(allow_smem<k_g2p_fused>(smem));
     Field3 fa{{un[0], un[1], un[2]}}, fb{{uo[0], uo[1], uo[2]}};
     const int arm_only = G.test_copy_timeout ? 1 : 0;
     // AW_TEST_UNTILED (tests of the advection's fallback): every block's u_new tile is reported as not
@@ -2288,8 +2287,7 @@ aw_status advect_sorted(MsbgState& G, float* soa, int64_t n, const uint32_t* cs,
     int maxres = 0;
     for (int r : G.h_res) maxres = std::max(maxres, r);
     const size_t smem = (size_t)tile_block(maxres) * sizeof(float);
-    // (always set: a grid of smaller blocks may have lowered it)
-    AW_CUDA(cudaFuncSetAttribute(k_advect_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    AW_TRY(allow_smem<k_advect_tile>(smem));
     k_advect_tile<<<G.nb, 256, smem, s>>>(G.view0(), soa, n, cs, dt, G.tile_off.p, G.tiles_new.p, G.err.p + 1,
                                           DropIn{nullptr, nullptr, nullptr}, G.blk_busy.p ? G.tile_ok.p : nullptr,
                                           Field3{{un[0], un[1], un[2]}}, G.blk_order_on ? G.blk_order.p : nullptr);
@@ -2827,7 +2825,7 @@ extern "C" aw_status aw_g2p(aw_msbg* g, float* d_vel, const float* d_pos, int64_
         int maxres = 0;
         for (int r : G.h_res) maxres = std::max(maxres, r);
         const size_t smem = ((size_t)tile_block(maxres) + 2 * 6 * G2P_SLOT) * sizeof(float);
-        AW_CUDA(cudaFuncSetAttribute(k_g2p_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        AW_TRY(allow_smem<k_g2p_fused>(smem));
         Field3 fa{{un[0], un[1], un[2]}}, fb{{uo[0], uo[1], uo[2]}};
         k_g2p_fused<<<G.nb, G2P_THREADS, smem, s>>>(G.view0(), W.soa.p, n, W.cell_start.p, alpha, fa, fb, G.tile_off.p,
                                                      nullptr, G.err.p + 1, 1 << 20, 0, DropIn{W.sorted, d_vel, W.hash.p},
@@ -2863,7 +2861,7 @@ extern "C" aw_status aw_advect(aw_msbg* g, float* d_pos, int64_t n, float dt, aw
         int maxres = 0;
         for (int r : G.h_res) maxres = std::max(maxres, r);
         const size_t smem = (size_t)tile_block(maxres) * sizeof(float);
-        AW_CUDA(cudaFuncSetAttribute(k_advect_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        AW_TRY(allow_smem<k_advect_tile>(smem));
         k_advect_tile<<<G.nb, 256, smem, s>>>(G.view0(), W.soa.p, n, W.cell_start.p, dt, G.tile_off.p, G.tiles_new.p,
                                               G.err.p + 1, DropIn{W.sorted, d_pos, W.hash.p}, nullptr, Field3{},
                                               G.blk_order_on ? G.blk_order.p : nullptr);

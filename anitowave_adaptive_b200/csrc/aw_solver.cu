@@ -2871,14 +2871,13 @@ static aw_status solver_build(aw_solver* S) {
     S->lv.resize(used);
     // coefficients of every level
     AW_TRY(build_coefficients(S, 0));
-    {  // always opted in: static shared memory (k_smooth's per-slot state) counts against the default 48 KB too
-        AW_CUDA(cudaFuncSetAttribute(k_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S->smem_max));
-        AW_CUDA(cudaFuncSetAttribute(k_residual<SrcX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S->smem_max));
-        AW_CUDA(cudaFuncSetAttribute(k_prolong, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S->smem_max));
-        AW_CUDA(cudaFuncSetAttribute(k_restrict, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S->smem_max));
-    }
-    AW_CUDA(cudaFuncSetAttribute(k_residual<SrcD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S->smem_max64));
-    AW_CUDA(cudaFuncSetAttribute(k_apply_dot, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S->smem_max64));
+    // always opted in: static shared memory (k_smooth's per-slot state) counts against the default 48 KB too
+    AW_TRY(allow_smem<k_smooth>(S->smem_max));
+    AW_TRY(allow_smem<k_residual<SrcX>>(S->smem_max));
+    AW_TRY(allow_smem<k_prolong>(S->smem_max));
+    AW_TRY(allow_smem<k_restrict>(S->smem_max));
+    AW_TRY(allow_smem<k_residual<SrcD>>(S->smem_max64));
+    AW_TRY(allow_smem<k_apply_dot>(S->smem_max64));
     if (S->d.precision == AW_PRECISION_MIXED) {
         const size_t nc0 = S->lv[0].ncell();
         AW_TRY(S->cg_r.ensure(nc0));
@@ -2930,7 +2929,7 @@ static aw_status solver_build(aw_solver* S) {
         for (int k = j + 1; ok && k < nl; ++k) ok = S->lv[k].dense && S->lv[k].ncell() <= (size_t)TAIL_MAX_CELLS;
         if (ok) {
             S->tail = j;
-            AW_CUDA(cudaFuncSetAttribute(k_dense_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+            AW_TRY(allow_smem<k_dense_tail>(200 * 1024));
             DenseTail T = tail_args(S);
             if (tail_layout(T) > 200 * 1024) S->tail = 0;  // a lattice so thin that its ghost layer dominates
         }
