@@ -111,13 +111,19 @@ struct aw_solver {
     aw::DBuf<float> cg32_d, cg32_q, cg32_sc, partials32;
     aw::DBuf<double> partials, norm;
     size_t smem_max = 0, smem_max64 = 0;
-    // the whole V-cycle as a CUDA graph, captured once per (x0, b0) binding
+    // the whole V-cycle as a CUDA graph, captured once per (x0, b0) binding: aw_solve's and aw_vcycle_run's, so
+    // that a program that calls both in turn captures neither again
     cudaStream_t cap = nullptr;
-    cudaGraphExec_t cycle = nullptr;
-    const void* cycle_x0 = nullptr;
-    const void* cycle_b0 = nullptr;
-    unsigned cycle_form = ~0u;  // 2 * gen + (level-0 x starts at zero)
-    unsigned long long cycle_kernels = 0;
+    struct Cycle {
+        cudaGraphExec_t exec = nullptr;
+        const void *x0 = nullptr, *b0 = nullptr;
+        unsigned form = ~0u;  // 2 * gen + (level-0 x starts at zero)
+        unsigned long long kernels = 0;
+        void drop() {
+            if (exec) cudaGraphExecDestroy(exec);
+            exec = nullptr;
+        }
+    } solve_cycle, call_cycle;
     bool vcycle_called = false;  // aw_vcycle_run ran since the solver was built
     // the mixed-precision CG iterations as one graph with a device-side while loop, per pressure
     // array; cgst = {iterations, restart flag, iteration limit}, cgprm = {||b||, tolerance}
@@ -136,7 +142,8 @@ struct aw_solver {
     double* h_norm = nullptr;  // pinned host words: a squared norm, uniform_check's counts
     double* h_cg = nullptr;    // pinned host words of the device-loop state
     ~aw_solver() {
-        if (cycle) cudaGraphExecDestroy(cycle);
+        solve_cycle.drop();
+        call_cycle.drop();
         if (cgloop) cudaGraphExecDestroy(cgloop);
         if (cap) cudaStreamDestroy(cap);
         if (h_norm) cudaFreeHost(h_norm);
@@ -2752,14 +2759,12 @@ static aw_status solver_build(aw_solver* S) {
     S->exact = false;
     S->coef_dirty = true;
     S->smem_max = S->smem_max64 = 0;
-    if (S->cycle) cudaGraphExecDestroy(S->cycle);
-    S->cycle = nullptr;
-    S->cycle_x0 = S->cycle_b0 = nullptr;
+    S->solve_cycle.drop();
+    S->call_cycle.drop();
     S->vcycle_called = false;
     if (S->cgloop) cudaGraphExecDestroy(S->cgloop);
     S->cgloop = nullptr;
     S->cgloop_p = nullptr;
-    S->cycle_kernels = 0;
     S->x0 = nullptr;
     S->b0 = nullptr;
     const bool ref = S->d.operator_mode == AW_OPERATOR_REFERENCE;
@@ -3065,41 +3070,38 @@ static aw_status solve_vcycle(aw_solver* S, bool zero, cudaStream_t s) {
     return vcycle(S, 0, s);
 }
 // ... replayed from a CUDA graph (captured on first use for the current level-0 x/b and form).
-static aw_status run_vcycle(aw_solver* S, bool zero, cudaStream_t s) {
+static aw_status run_vcycle(aw_solver* S, aw_solver::Cycle& C, bool zero, cudaStream_t s) {
     if (!S->use_graph) return solve_vcycle(S, zero, s);
     const void* x0 = S->x0 ? (const void*)S->x0 : (const void*)S->lv[0].x.p;
     const void* b0 = S->b0 ? (const void*)S->b0 : (const void*)S->lv[0].b.p;
     const unsigned form = 2 * S->gen + (zero ? 1u : 0u);
-    if (!S->cycle || S->cycle_x0 != x0 || S->cycle_b0 != b0 || S->cycle_form != form) {
-        if (S->cycle) {
-            cudaGraphExecDestroy(S->cycle);
-            S->cycle = nullptr;
-        }
+    if (!C.exec || C.x0 != x0 || C.b0 != b0 || C.form != form) {
+        C.drop();
         if (!S->cap) AW_CUDA(cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking));
         const unsigned long long l0 = g_launches;
         AW_CUDA(cudaStreamBeginCapture(S->cap, cudaStreamCaptureModeThreadLocal));
         aw_status st = solve_vcycle(S, zero, S->cap);
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(S->cap, &graph);
-        S->cycle_kernels = g_launches - l0;
+        C.kernels = g_launches - l0;
         g_launches = l0;
         if (st != AW_OK) {
             if (graph) cudaGraphDestroy(graph);
             return st;
         }
         if (e != cudaSuccess) return set_error(AW_ERR_CUDA, "V-cycle capture: %s", cudaGetErrorString(e));
-        e = cudaGraphInstantiate(&S->cycle, graph, 0);
+        e = cudaGraphInstantiate(&C.exec, graph, 0);
         cudaGraphDestroy(graph);
         if (e != cudaSuccess) {
-            S->cycle = nullptr;
+            C.exec = nullptr;
             return set_error(AW_ERR_CUDA, "V-cycle graph instantiate: %s", cudaGetErrorString(e));
         }
-        S->cycle_x0 = x0;
-        S->cycle_b0 = b0;
-        S->cycle_form = form;
+        C.x0 = x0;
+        C.b0 = b0;
+        C.form = form;
     }
-    AW_CUDA(cudaGraphLaunch(S->cycle, s));
-    g_launches += S->cycle_kernels;
+    AW_CUDA(cudaGraphLaunch(C.exec, s));
+    g_launches += C.kernels;
     return AW_OK;
 }
 
@@ -3121,7 +3123,7 @@ extern "C" aw_status aw_vcycle_run(aw_solver* S, aw_stream s) {
         S->vcycle_called = true;
         return solve_vcycle(S, false, (cudaStream_t)s);
     }
-    return run_vcycle(S, false, (cudaStream_t)s);
+    return run_vcycle(S, S->call_cycle, false, (cudaStream_t)s);
 }
 
 // *out = sqrt of the sum in S->norm[0], read back with uniform_check's counts (syncs)
@@ -3181,7 +3183,7 @@ static aw_status cg_iteration(aw_solver* S, double* p, unsigned ndot, cudaStream
     const int cf = fv(S) ? 1 : 0;
     double* sc = S->cg_sc.p;
     if (h) AW_TRY(solve_vcycle(S, true, s));
-    else AW_TRY(run_vcycle(S, true, s));
+    else AW_TRY(run_vcycle(S, S->solve_cycle, true, s));
     AW_TRY(launch_dep(S, k_dot64, ndot, 256, 0, s, (const double*)S->cg_r.p, (const float*)L0.x.p,
                       (const uint8_t*)L0.fluid.p, nc, S->partials.p, S->ticket.p, sc + 0));
     CgVec K{};
@@ -3312,7 +3314,7 @@ static aw_status solve_aligned(aw_solver* S, const float* d_b, void* d_p, int32_
                 st = set_error(AW_ERR_NOT_CONVERGED, "relative residual %.3e after %d cycles", rel, it);
                 break;
             }
-            st = run_vcycle(S, false, s);
+            st = run_vcycle(S, S->solve_cycle, false, s);
             if (st != AW_OK) break;
         }
         S->x0 = nullptr;
@@ -3364,7 +3366,7 @@ static aw_status solve_aligned(aw_solver* S, const float* d_b, void* d_p, int32_
                 st = set_error(AW_ERR_NOT_CONVERGED, "relative residual %.3e after %d iterations", rel, it);
                 break;
             }
-            st = run_vcycle(S, true, s);
+            st = run_vcycle(S, S->solve_cycle, true, s);
             if (st != AW_OK) break;
             // the kernels of one iteration as programmatic dependents of one another
             if ((st = launch_dep(S, k_dot32, ndot32, 256, 0, s, L0.b.p, L0.x.p, L0.fluid.p, nc, S->partials32.p)) != AW_OK) break;

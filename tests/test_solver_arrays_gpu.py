@@ -1,6 +1,8 @@
 """Which arrays the solver takes and what it leaves in its own."""
 import ctypes as C
 import os
+import statistics
+import time
 
 import numpy as np
 import pytest
@@ -233,4 +235,34 @@ def test_vcycle_after_a_solve_leaves_every_levels_arrays(env):
         got.append(_levels(sv, aw.PRECISION_MIXED))
         sv.close()
     assert all(torch.equal(got[0][k], got[1][k]) for k in got[1])
+    g.close()
+
+
+def test_solves_and_vcycles_by_turns_capture_nothing_again():
+    """A V-cycle solve and aw_vcycle_run called in turn take about as long as each on its own (medians; capturing and
+    instantiating the cycle's graph in every call made the pair take several times that)."""
+    g = _grid(8, (8, 8, 4))
+    n, fluid, b0 = _problem(g, 8)
+    sv = aw.Solver(g, precision=aw.PRECISION_FP32, tolerance=1e-30, max_cycles=2)
+    sv.setup(fluid)
+    p = torch.zeros(n, device="cuda")
+    sv.level_array(0, 1).copy_(b0)
+
+    def solve():
+        sv.solve(b0, p, raise_on_error=False)
+
+    def seconds(*calls):
+        t = []
+        for _ in range(60):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            for c in calls:
+                c()
+            torch.cuda.synchronize()
+            t.append(time.perf_counter() - t0)
+        return statistics.median(t[10:])
+
+    alone = seconds(solve) + seconds(sv.vcycle)
+    assert seconds(solve, sv.vcycle) <= 1.5 * alone
+    sv.close()
     g.close()
