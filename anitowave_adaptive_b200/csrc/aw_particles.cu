@@ -16,14 +16,6 @@ namespace aw {
 
 static inline unsigned nblk(size_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
 
-// grid-stride kernels over n items: at most 8 CTAs of 256 threads per SM
-static unsigned resample_grid(int64_t n) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sms * 8));
-}
-
 // Strided particle array: element (i, a) at p[i * si + a * sa]  (AoS: si=3, sa=1; SoA: si=1, sa=n)
 struct PArr {
     const float* p;
@@ -2220,47 +2212,72 @@ aw_status g2p_sorted(MsbgState& G, float* soa, int64_t n, const uint32_t* cs, fl
     return AW_OK;
 }
 
-__global__ void k_advect_tiles(LevelView L, PArrW pos, int64_t n, float dt, const uint32_t* __restrict__ toff,
-                               const float* __restrict__ tiles,
-                               const unsigned long long* __restrict__ skip = nullptr, InactiveAos I = {}) {
-    if (skip && sort_reusable(skip, false)) {  // the drop-in advection took the sorted path
+// The general kernels of the drop-in calls, on particles in any order, RUN of them a thread; 0: one, and no
+// sorted path before.  Behind the sorted path, which the device may have taken (then only the inactive blocks'
+// particles are left), each thread takes 4 from GENERAL_LONG particles on, since idle CTAs cost too (11 us for
+// 4.1M particles at one a thread, 3 at 4); below, 4 in sequence cost a call that does come here more (60 instead
+// of 47 us at 30,000).  A grid-stride loop of 8 CTAs per SM took registers and left a part-filled last wave: 218
+// instead of 180 us for 4.1M particles in cell order (G2P).
+constexpr int64_t GENERAL_LONG = 148 * 16 * 256;
+template <int RUN, class F>
+__device__ __forceinline__ void general_particles(int64_t n, F particle) {
+    int64_t i = (int64_t)blockIdx.x * blockDim.x * (RUN ? RUN : 1) + threadIdx.x;
+    if (RUN <= 1) {
+        if (i < n) particle(i);
+        return;
+    }
+#pragma unroll 1
+    for (int k = 0; k < RUN; ++k) {
+        const int64_t j = i + k * (int64_t)blockDim.x;
+        if (j >= n) return;
+        particle(j);
+    }
+}
+
+template <int RUN>
+__global__ void __launch_bounds__(256, 6) k_advect_tiles(LevelView L, PArrW pos, int64_t n, float dt,
+                                                         const uint32_t* __restrict__ toff, const float* __restrict__ tiles,
+                                                         const unsigned long long* __restrict__ skip, InactiveAos I) {
+    if (RUN && sort_reusable(skip, false)) {  // the drop-in advection took the sorted path
         inactive_aos(L.g, I, 1, 0.f);
         return;
     }
     const Geo& g = L.g;
     const float h0 = g.bs / (float)g.R0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    float x[3] = {pos(i, 0), pos(i, 1), pos(i, 2)};
-    float k1[3], k2[3], k3[3], y[3];
+    general_particles<RUN>(n, [&](int64_t i) {
+        float x[3] = {pos(i, 0), pos(i, 1), pos(i, 2)};
+        float k1[3], k2[3], k3[3], y[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) k1[a] = sample_tiles(L, toff, tiles, a, x);
+        for (int a = 0; a < 3; ++a) k1[a] = sample_tiles(L, toff, tiles, a, x);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) y[a] = x[a] + 0.5f * dt * k1[a];
+        for (int a = 0; a < 3; ++a) y[a] = x[a] + 0.5f * dt * k1[a];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) k2[a] = sample_tiles(L, toff, tiles, a, y);
+        for (int a = 0; a < 3; ++a) k2[a] = sample_tiles(L, toff, tiles, a, y);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) y[a] = x[a] + 0.75f * dt * k2[a];
+        for (int a = 0; a < 3; ++a) y[a] = x[a] + 0.75f * dt * k2[a];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) k3[a] = sample_tiles(L, toff, tiles, a, y);
+        for (int a = 0; a < 3; ++a) k3[a] = sample_tiles(L, toff, tiles, a, y);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        float v = (2.f / 9.f) * k1[a] + (3.f / 9.f) * k2[a] + (4.f / 9.f) * k3[a];
-        float lo = g.dmin[a] + 0.01f * h0;
-        float hi = g.dmin[a] + (float)g.D[a] * g.bs - 0.01f * h0;
-        pos(i, a) = fminf(fmaxf(x[a] + dt * v, lo), hi);
-    }
-    }
+        for (int a = 0; a < 3; ++a) {
+            float v = (2.f / 9.f) * k1[a] + (3.f / 9.f) * k2[a] + (4.f / 9.f) * k3[a];
+            float lo = g.dmin[a] + 0.01f * h0;
+            float hi = g.dmin[a] + (float)g.D[a] * g.bs - 0.01f * h0;
+            pos(i, a) = fminf(fmaxf(x[a] + dt * v, lo), hi);
+        }
+    });
 }
 
 // G2P / sampling on arbitrary (unsorted, AoS) particles through the ghosted tiles
-__global__ void k_g2p_tiles(LevelView L, PArr pos, PArrW vel, int64_t n, float alpha, const uint32_t* __restrict__ toff,
-                            const float* __restrict__ tn, const float* __restrict__ to,
-                            const unsigned long long* __restrict__ skip = nullptr, InactiveAos I = {}) {
-    if (skip && sort_reusable(skip, true)) {  // the drop-in G2P took the sorted path
+template <int RUN>
+__global__ void __launch_bounds__(256, 8) k_g2p_tiles(LevelView L, PArr pos, PArrW vel, int64_t n, float alpha,
+                                                      const uint32_t* __restrict__ toff, const float* __restrict__ tn,
+                                                      const float* __restrict__ to,
+                                                      const unsigned long long* __restrict__ skip, InactiveAos I) {
+    if (RUN && sort_reusable(skip, true)) {  // the drop-in G2P took the sorted path
         inactive_aos(L.g, I, 0, alpha);
         return;
     }
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    general_particles<RUN>(n, [&](int64_t i) {
         float X[3] = {pos(i, 0), pos(i, 1), pos(i, 2)};
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
@@ -2269,7 +2286,7 @@ __global__ void k_g2p_tiles(LevelView L, PArr pos, PArrW vel, int64_t n, float a
             const float vp = vel(i, a);
             vel(i, a) = alpha * (vp + (vn - vo)) + (1.f - alpha) * vn;
         }
-    }
+    });
 }
 
 __global__ void k_sample_tiles(LevelView L, PArr pts, int64_t n, const uint32_t* __restrict__ toff,
@@ -2298,7 +2315,7 @@ aw_status advect_sorted(MsbgState& G, float* soa, int64_t n, const uint32_t* cs,
 aw_status advect_tiles(MsbgState& G, float* pos, int pos_soa, int64_t n, float dt, const float* tiles, cudaStream_t s) {
     if (n <= 0) return AW_OK;
     PArrW P = pos_soa ? PArrW{pos, 1, n} : PArrW{pos, 3, 1};
-    k_advect_tiles<<<nblk(n), 256, 0, s>>>(G.view0(), P, n, dt, G.tile_off.p, tiles);
+    k_advect_tiles<0><<<nblk(n), 256, 0, s>>>(G.view0(), P, n, dt, G.tile_off.p, tiles, nullptr, InactiveAos{});
     AW_LAUNCH();
     return AW_OK;
 }
@@ -2363,7 +2380,8 @@ aw_status g2p_with_tiles(MsbgState& G, float* d_vel, const float* d_pos, int64_t
     AW_LAUNCH();
     k_build_tiles<<<G.nb, 128, 0, s>>>(G.view0(), uo, toff, to);
     AW_LAUNCH();
-    k_g2p_tiles<<<nblk(n), 256, 0, s>>>(G.view0(), PArr{d_pos, 3, 1}, PArrW{d_vel, 3, 1}, n, alpha, toff, tn, to);
+    k_g2p_tiles<0><<<nblk(n), 256, 0, s>>>(G.view0(), PArr{d_pos, 3, 1}, PArrW{d_vel, 3, 1}, n, alpha, toff, tn, to,
+                                           nullptr, InactiveAos{});
     AW_LAUNCH();
     return AW_OK;
 }
@@ -2374,7 +2392,7 @@ aw_status preload_g2p_with_tiles() {
     cudaFuncAttributes fa;
     AW_CUDA(cudaFuncGetAttributes(&fa, k_tile_offsets));
     AW_CUDA(cudaFuncGetAttributes(&fa, k_build_tiles));
-    AW_CUDA(cudaFuncGetAttributes(&fa, k_g2p_tiles));
+    AW_CUDA(cudaFuncGetAttributes(&fa, k_g2p_tiles<0>));
     return AW_OK;
 }
 
@@ -2836,10 +2854,12 @@ extern "C" aw_status aw_g2p(aw_msbg* g, float* d_vel, const float* d_pos, int64_
     Field3 a{{un[0], un[1], un[2]}}, b{{uo[0], uo[1], uo[2]}};
     k_build_tiles2<<<G.nb, 128, 0, s>>>(G.view0(), a, b, G.tile_off.p, G.tiles_new.p, G.tiles_old.p, skip);
     AW_LAUNCH();
-    // (a full grid of idle CTAs took 11 us at 4.1M particles: 8 CTAs per SM walk the particles)
-    k_g2p_tiles<<<resample_grid(n), 256, 0, s>>>(G.view0(), PArr{d_pos, 3, 1}, PArrW{d_vel, 3, 1}, n, alpha, G.tile_off.p,
-                                                 G.tiles_new.p, G.tiles_old.p, skip,
-                                                 InactiveAos{W.sorted, W.cell_start.p + G.tot[0], d_vel});
+    const PArr pos{d_pos, 3, 1};
+    const PArrW vel{d_vel, 3, 1};
+    const InactiveAos rest = skip ? InactiveAos{W.sorted, W.cell_start.p + G.tot[0], d_vel} : InactiveAos{};
+    auto general = !skip ? k_g2p_tiles<0> : (n < GENERAL_LONG ? k_g2p_tiles<1> : k_g2p_tiles<4>);
+    general<<<nblk(n, skip && n >= GENERAL_LONG ? 1024 : 256), 256, 0, s>>>(G.view0(), pos, vel, n, alpha, G.tile_off.p,
+                                                                            G.tiles_new.p, G.tiles_old.p, skip, rest);
     AW_LAUNCH();
     return AW_OK;
 }
@@ -2868,8 +2888,11 @@ extern "C" aw_status aw_advect(aw_msbg* g, float* d_pos, int64_t n, float dt, aw
         AW_LAUNCH();
         skip = W.hash.p;
     }
-    k_advect_tiles<<<resample_grid(n), 256, 0, s>>>(G.view0(), PArrW{d_pos, 3, 1}, n, dt, G.tile_off.p, G.tiles_new.p,
-                                                    skip, InactiveAos{W.sorted, W.cell_start.p + G.tot[0], d_pos});
+    const PArrW pos{d_pos, 3, 1};
+    const InactiveAos rest = skip ? InactiveAos{W.sorted, W.cell_start.p + G.tot[0], d_pos} : InactiveAos{};
+    auto general = !skip ? k_advect_tiles<0> : (n < GENERAL_LONG ? k_advect_tiles<1> : k_advect_tiles<4>);
+    general<<<nblk(n, skip && n >= GENERAL_LONG ? 1024 : 256), 256, 0, s>>>(G.view0(), pos, n, dt, G.tile_off.p,
+                                                                            G.tiles_new.p, skip, rest);
     AW_LAUNCH();
     W.src_valid = false;  // the positions have moved
     return AW_OK;
@@ -2961,6 +2984,14 @@ static aw_status make_lattice(const MsbgState& G, const int32_t out_dims[3], Lat
         T.sp[a] = (float)G.geo.D[a] * G.geo.bs / (float)out_dims[a];
     }
     return AW_OK;
+}
+
+// grid-stride kernels over n items: at most 8 CTAs of 256 threads per SM
+static unsigned resample_grid(int64_t n) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sms * 8));
 }
 
 extern "C" aw_status aw_resample_lattice(aw_msbg* g, const int32_t out_dims[3], float origin[3], float spacing[3]) {
