@@ -899,7 +899,7 @@ __global__ void k_cg_direction(double* __restrict__ d, const float* __restrict__
     d[i] = fluid[i] ? (double)z[i] + beta * d[i] : 0.0;
 }
 // The end of one CG iteration.  qn = -A d; alpha = rho / (d . A d); on fluid cells p += alpha d,
-// r += alpha qn, and the FP32 copy of r for the next V-cycle; rho_old = rho for the next iteration's
+// r += alpha qn (with `air` on every cell), and the FP32 copy of r for the next V-cycle; rho_old = rho for the next iteration's
 // direction (sc[1] is read by no CTA of this kernel).  The last CTA to finish has |r|^2: it stores it,
 // counts the iteration, clears the restart flag and, in the device-side loop (DEV), runs the loop body
 // again while the residual is finite, at or above the tolerance and the iteration limit is not reached.
@@ -913,6 +913,7 @@ struct CgVec {
     const double *d0, *d1, *qn;
     double* sc;
     const uint8_t* fluid;
+    int air;  // the operator has rows on air cells (reference mode): r and its copy follow there too
     size_t n;
     double* norm2;
     const double* prm;
@@ -929,31 +930,34 @@ __global__ void __launch_bounds__(256) k_cg_update(CgVec K, double* part, unsign
     const size_t n2 = K.n / 2, step = (size_t)gridDim.x * blockDim.x, t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (size_t i = t0; i < n2; i += step) {
         const uchar2 f = reinterpret_cast<const uchar2*>(K.fluid)[i];
-        if (!(f.x | f.y)) continue;
+        if (!(f.x | f.y | K.air)) continue;
         const double2 dv = reinterpret_cast<const double2*>(d)[i], qv = reinterpret_cast<const double2*>(K.qn)[i];
         double2 rv = reinterpret_cast<const double2*>(K.r)[i];
         double2 pv = reinterpret_cast<const double2*>(K.p)[i];
+        const bool rx = f.x || K.air, ry = f.y || K.air;
+        if (rx) rv.x = rv.x + alpha * qv.x;
+        if (ry) rv.y = rv.y + alpha * qv.y;
         if (f.x) {
             pv.x += alpha * dv.x;
-            rv.x = rv.x + alpha * qv.x;
             acc += rv.x * rv.x;
         }
         if (f.y) {
             pv.y += alpha * dv.y;
-            rv.y = rv.y + alpha * qv.y;
             acc += rv.y * rv.y;
         }
         reinterpret_cast<double2*>(K.p)[i] = pv;
         reinterpret_cast<double2*>(K.r)[i] = rv;
-        reinterpret_cast<float2*>(K.rf)[i] = make_float2(f.x ? (float)rv.x : 0.f, f.y ? (float)rv.y : 0.f);
+        reinterpret_cast<float2*>(K.rf)[i] = make_float2(rx ? (float)rv.x : 0.f, ry ? (float)rv.y : 0.f);
     }
-    if (t0 == 0 && (K.n & 1) && K.fluid[K.n - 1]) {
+    if (t0 == 0 && (K.n & 1) && (K.fluid[K.n - 1] || K.air)) {
         const size_t i = K.n - 1;
-        K.p[i] += alpha * d[i];
         const double rv = K.r[i] + alpha * K.qn[i];
         K.r[i] = rv;
         K.rf[i] = (float)rv;
-        acc += rv * rv;
+        if (K.fluid[i]) {
+            K.p[i] += alpha * d[i];
+            acc += rv * rv;
+        }
     }
     last_cta_sum(acc, part, ticket, [&](double t) {
         K.norm2[0] = t;
@@ -3209,6 +3213,7 @@ static aw_status cg_iteration(aw_solver* S, double* p, unsigned ndot, cudaStream
     K.qn = S->cg_q.p;
     K.sc = sc;
     K.fluid = L0.fluid.p;
+    K.air = cf ? 0 : 1;
     K.n = nc;
     K.norm2 = S->norm.p;
     K.prm = S->cgprm.p;

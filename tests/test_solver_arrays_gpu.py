@@ -266,3 +266,35 @@ def test_solves_and_vcycles_by_turns_capture_nothing_again():
     assert seconds(solve, sv.vcycle) <= 1.5 * alone
     sv.close()
     g.close()
+
+
+@pytest.mark.parametrize("R0", [8, 1])
+def test_reference_operator_iterates_on_air_cells_too(R0):
+    """The reference's operator has a row on every cell, flagged or not: after one mixed CG iteration the V-cycle's
+    next input (level-0 b) is b - A p on air cells as on fluid ones.  R0 = 1: an odd number of cells."""
+    g = aw.MSBG((3, 3, 3), 1.0, (0.0, 0.0, 0.0), R0, 1)
+    g.init_refinement_map(0)
+    g.allocate()
+    n = g.totals()[0]
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    b = torch.randn(n, generator=gen, device="cuda")
+    fluid = (torch.rand(n, generator=gen, device="cuda") < 0.6).to(torch.uint8)
+    fluid[-1], fluid[-2], fluid[-3] = 0, 1, 0
+    sv = aw.Solver(g, operator_mode=aw.OPERATOR_REFERENCE, precision=aw.PRECISION_MIXED, tolerance=1e-30, max_cycles=1)
+    sv.setup(fluid)
+    p = torch.zeros(n, dtype=torch.float64, device="cuda")
+    sv.solve(b, p, raise_on_error=False)
+    got = sv.level_array(0, 1).clone()
+    sv.level_array(0, 1).copy_(b)
+    sv.level_array(0, 0).copy_(p.float())
+    torch.cuda.synchronize()
+    sv.residual(0)
+    torch.cuda.synchronize()
+    want = sv.level_array(0, 2).clone()
+    # FP32 residual: p rounded once, at most 13 rounded products and sums of values up to 12 |w| |p|
+    w = max(float(sv.level_array(0, 3 + a).abs().max()) for a in range(3))
+    tol = 16 * 2.0 ** -24 * (float(b.abs().max()) + 12 * w * float(p.abs().max()))
+    assert float((got - want).abs().max()) <= tol
+    assert float((want - b)[fluid == 0].abs().max()) > 100 * tol
+    sv.close()
+    g.close()
