@@ -607,10 +607,15 @@ __device__ __forceinline__ void p2g_cross(const CrossNb& N, int rn, const float 
 constexpr int P2G_THREADS = 512;  // the most threads a P2G CTA is launched with
 constexpr int P2G_XQ = 96;  // per-warp queue of cross-resolution pairs: < 32 waiting + 2 per lane
 constexpr int P2G_SLICE = 16;  // particles of one cell per register-accumulation task
-constexpr int P2G_BINS = 64;   // counts told apart when a block's cells are ordered
+constexpr int P2G_BINS = 128;  // counts told apart when a block's cells are ordered: 1 .. 63, then 8 an octave
 constexpr int P2G_MAX_SLICES = 1 << 19;  // 6 * 8^3 * this stays below 2^31
 constexpr int P2G_MAX_CELLS = 16 * 16 * 16;  // cells of the largest block (base resolution <= 16)
 constexpr int P2G_NEAR_CELLS = 8 * 8 * 8;    // blocks up to this size list their near cells
+__device__ __forceinline__ int p2g_bin(uint32_t cnt) {
+    if (cnt < 64u) return (int)cnt;
+    const int e = 31 - __clz((int)cnt);  // >= 6; the last bin takes 15360 and more
+    return min(64 + 8 * (e - 6) + (int)((cnt >> (e - 3)) & 7u), P2G_BINS - 1);
+}
 
 // one queued (particle, neighbour direction d) pair: the particle's weights on neighbour d's faces
 template <bool PH>
@@ -691,13 +696,13 @@ __global__ void __launch_bounds__(P2G_THREADS, 2) k_p2g_own(LevelView L, const f
     __shared__ int ccount[P2G_MAX_CELLS / 32], cocount[P2G_MAX_CELLS / 32];
     __shared__ uint16_t clist[P2G_MAX_CELLS], colist[P2G_MAX_CELLS];
     __shared__ int nonempty, nnear, ncoarse;
-    __shared__ int hist[P2G_BINS];  // cells by particle count, then where a count's cells go in clist
     __shared__ int tctr[2];  // next own / coarse task to hand out
     // near-cell list of the cross-resolution pass (blocks of at most P2G_NEAR_CELLS cells)
     __shared__ uint16_t nl_cell[P2G_NEAR_CELLS];
     __shared__ uint32_t nl_mask[P2G_NEAR_CELLS], nl_pre[P2G_NEAR_CELLS + 1];
     __shared__ uint32_t nmask_tmp[P2G_NEAR_CELLS];
     __shared__ int ncnt_tmp[P2G_NEAR_CELLS];
+    int* hist = ncnt_tmp;  // before the near-cell list: cells by particle count, then where a count's cells go in clist
     __shared__ uint32_t xq_v[(P2G_THREADS / 32) * P2G_XQ];
     __shared__ uint8_t xq_d[(P2G_THREADS / 32) * P2G_XQ];
     const int b = order ? order[blockIdx.x] : (int)blockIdx.x;
@@ -790,8 +795,9 @@ __global__ void __launch_bounds__(P2G_THREADS, 2) k_p2g_own(LevelView L, const f
     // The block's non-empty cells, fullest first: tasks run over these only, so that lanes do not idle on the
     // air cells of a surface block, and the lanes of a warp take cells of one count (in cell order a warp ran
     // as long as its fullest cell, 13 steps for a mean of 8, and a second slice took a pass over all cells:
-    // with the loads below 243 to 207 us at 4.1M particles).  Counts of P2G_BINS - 1 and more are not told
-    // apart.
+    // with the loads below 243 to 207 us at 4.1M particles).  Crowded cells are told apart too (p2g_bin), since the
+    // cells that reach a slice have to be the first of the list: 4M particles thickening towards a corner took
+    // 2.83 ms in cell order, 2.87 with one bin from 63 on, 1.89 now (two phases 6.23, 6.76 and 4.85).
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     // A cell is listed for the coarse tile too when it lies within two of b's cells (one coarse
     // cell, the reach there) of a side towards a coarser neighbour, on every axis that neighbour's
@@ -820,7 +826,7 @@ __global__ void __launch_bounds__(P2G_THREADS, 2) k_p2g_own(LevelView L, const f
         }
         if (cnt > 0) {
             atomicMax(&maxcnt, cnt);
-            atomicAdd(&hist[min(cnt, (uint32_t)(P2G_BINS - 1))], 1);
+            atomicAdd(&hist[p2g_bin(cnt)], 1);
         }
         const unsigned mc = __ballot_sync(0xffffffffu, cnt > 0 && cmask && coarse_near(c));
         if (lane == 0) cocount[ch] = __popc(mc);
@@ -863,7 +869,7 @@ __global__ void __launch_bounds__(P2G_THREADS, 2) k_p2g_own(LevelView L, const f
         const bool ne = c < nc3 && cst[c + 1] > cst[c];
         const bool cn = ne && cmask && coarse_near(c);
         const unsigned mc = __ballot_sync(0xffffffffu, cn);
-        if (ne) clist[atomicAdd(&hist[min(cst[c + 1] - cst[c], (uint32_t)(P2G_BINS - 1))], 1)] = (uint16_t)c;
+        if (ne) clist[atomicAdd(&hist[p2g_bin(cst[c + 1] - cst[c])], 1)] = (uint16_t)c;
         if (cn) colist[cocount[ch] + __popc(mc & ((1u << lane) - 1u))] = (uint16_t)c;
     }
     __syncthreads();
