@@ -112,7 +112,8 @@ struct aw_solver {
     aw::DBuf<double> partials, norm;
     size_t smem_max = 0, smem_max64 = 0;
     // the whole V-cycle as a CUDA graph, captured once per (x0, b0) binding: aw_solve's and aw_vcycle_run's, so
-    // that a program that calls both in turn captures neither again
+    // that a program that calls both in turn captures neither again.  Of aw_solve's graphs the last two are kept:
+    // a program may solve for one density and for a varying one, or for two pressure arrays, in turn.
     cudaStream_t cap = nullptr;
     struct Cycle {
         cudaGraphExec_t exec = nullptr;
@@ -123,14 +124,22 @@ struct aw_solver {
             if (exec) cudaGraphExecDestroy(exec);
             exec = nullptr;
         }
-    } solve_cycle, call_cycle;
+    } solve_cycle[2], call_cycle;
+    int solve_last = 0;          // the solve_cycle used last
     bool vcycle_called = false;  // aw_vcycle_run ran since the solver was built
     // the mixed-precision CG iterations as one graph with a device-side while loop, per pressure
-    // array; cgst = {iterations, restart flag, iteration limit}, cgprm = {||b||, tolerance}
-    cudaGraphExec_t cgloop = nullptr;
-    const void* cgloop_p = nullptr;
-    unsigned cgloop_gen = 0;
-    unsigned long long cgloop_kernels = 0;
+    // array and gen (the last two); cgst = {iterations, restart flag, iteration limit}, cgprm = {||b||, tolerance}
+    struct Loop {
+        cudaGraphExec_t exec = nullptr;
+        const void* p = nullptr;
+        unsigned gen = 0;
+        unsigned long long kernels = 0;
+        void drop() {
+            if (exec) cudaGraphExecDestroy(exec);
+            exec = nullptr;
+        }
+    } cgloop[2];
+    int cgloop_last = 0;  // the one used last
     bool use_devloop = true;
     aw::DBuf<int> cgst;
     aw::DBuf<double> cgprm;
@@ -142,9 +151,9 @@ struct aw_solver {
     double* h_norm = nullptr;  // pinned host words: a squared norm, uniform_check's counts
     double* h_cg = nullptr;    // pinned host words of the device-loop state
     ~aw_solver() {
-        solve_cycle.drop();
+        for (Cycle& c : solve_cycle) c.drop();
         call_cycle.drop();
-        if (cgloop) cudaGraphExecDestroy(cgloop);
+        for (Loop& l : cgloop) l.drop();
         if (cap) cudaStreamDestroy(cap);
         if (h_norm) cudaFreeHost(h_norm);
         if (h_cg) cudaFreeHost(h_cg);
@@ -2763,12 +2772,10 @@ static aw_status solver_build(aw_solver* S) {
     S->exact = false;
     S->coef_dirty = true;
     S->smem_max = S->smem_max64 = 0;
-    S->solve_cycle.drop();
+    for (aw_solver::Cycle& c : S->solve_cycle) c.drop();
     S->call_cycle.drop();
+    for (aw_solver::Loop& l : S->cgloop) l.drop();
     S->vcycle_called = false;
-    if (S->cgloop) cudaGraphExecDestroy(S->cgloop);
-    S->cgloop = nullptr;
-    S->cgloop_p = nullptr;
     S->x0 = nullptr;
     S->b0 = nullptr;
     const bool ref = S->d.operator_mode == AW_OPERATOR_REFERENCE;
@@ -3073,13 +3080,17 @@ static aw_status solve_vcycle(aw_solver* S, bool zero, cudaStream_t s) {
     if (zero) AW_TRY(zero_x(S, 0, s));
     return vcycle(S, 0, s);
 }
-// ... replayed from a CUDA graph (captured on first use for the current level-0 x/b and form).
-static aw_status run_vcycle(aw_solver* S, aw_solver::Cycle& C, bool zero, cudaStream_t s) {
+// ... replayed from a CUDA graph (captured on first use for the current level-0 x/b and form): aw_vcycle_run's
+// (call), or the one of aw_solve's two that fits, else in the place of the one used longer ago.
+static aw_status run_vcycle(aw_solver* S, bool call, bool zero, cudaStream_t s) {
     if (!S->use_graph) return solve_vcycle(S, zero, s);
     const void* x0 = S->x0 ? (const void*)S->x0 : (const void*)S->lv[0].x.p;
     const void* b0 = S->b0 ? (const void*)S->b0 : (const void*)S->lv[0].b.p;
     const unsigned form = 2 * S->gen + (zero ? 1u : 0u);
-    if (!C.exec || C.x0 != x0 || C.b0 != b0 || C.form != form) {
+    auto fits = [&](const aw_solver::Cycle& c) { return c.exec && c.x0 == x0 && c.b0 == b0 && c.form == form; };
+    if (!call && !fits(S->solve_cycle[S->solve_last])) S->solve_last ^= 1;
+    aw_solver::Cycle& C = call ? S->call_cycle : S->solve_cycle[S->solve_last];
+    if (!fits(C)) {
         C.drop();
         if (!S->cap) AW_CUDA(cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking));
         const unsigned long long l0 = g_launches;
@@ -3127,7 +3138,7 @@ extern "C" aw_status aw_vcycle_run(aw_solver* S, aw_stream s) {
         S->vcycle_called = true;
         return solve_vcycle(S, false, (cudaStream_t)s);
     }
-    return run_vcycle(S, S->call_cycle, false, (cudaStream_t)s);
+    return run_vcycle(S, true, false, (cudaStream_t)s);
 }
 
 // *out = sqrt of the sum in S->norm[0], read back with uniform_check's counts (syncs)
@@ -3187,7 +3198,7 @@ static aw_status cg_iteration(aw_solver* S, double* p, unsigned ndot, cudaStream
     const int cf = fv(S) ? 1 : 0;
     double* sc = S->cg_sc.p;
     if (h) AW_TRY(solve_vcycle(S, true, s));
-    else AW_TRY(run_vcycle(S, S->solve_cycle, true, s));
+    else AW_TRY(run_vcycle(S, false, true, s));
     AW_TRY(launch_dep(S, k_dot64, ndot, 256, 0, s, (const double*)S->cg_r.p, (const float*)L0.x.p,
                       (const uint8_t*)L0.fluid.p, nc, S->partials.p, S->ticket.p, sc + 0));
     CgVec K{};
@@ -3227,11 +3238,8 @@ static aw_status cg_iteration(aw_solver* S, double* p, unsigned ndot, cudaStream
 // iteration; the update kernel's last CTA sets the loop condition, so no host round trip separates
 // iterations.  The graph is built per pressure array and form.  Returns false (state unchanged) when
 // the device cannot build such a graph; the caller then keeps the host loop.
-static bool cg_devloop_build(aw_solver* S, double* p, unsigned ndot) {
-    if (S->cgloop) {
-        cudaGraphExecDestroy(S->cgloop);
-        S->cgloop = nullptr;
-    }
+static bool cg_devloop_build(aw_solver* S, aw_solver::Loop& C, double* p, unsigned ndot) {
+    C.drop();
     if (!S->cap && cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking) != cudaSuccess) return false;
     cudaGraph_t g = nullptr;
     if (cudaGraphCreate(&g, 0) != cudaSuccess) return false;
@@ -3252,20 +3260,20 @@ static bool cg_devloop_build(aw_solver* S, double* p, unsigned ndot) {
                 const aw_status st = cg_iteration(S, p, ndot, S->cap, &h);
                 cudaGraph_t out = nullptr;
                 const cudaError_t e = cudaStreamEndCapture(S->cap, &out);
-                S->cgloop_kernels = g_launches - l0;
+                C.kernels = g_launches - l0;
                 g_launches = l0;
-                ok = st == AW_OK && e == cudaSuccess && cudaGraphInstantiate(&S->cgloop, g, 0) == cudaSuccess;
+                ok = st == AW_OK && e == cudaSuccess && cudaGraphInstantiate(&C.exec, g, 0) == cudaSuccess;
             }
         }
     }
     cudaGraphDestroy(g);
     if (!ok) {
-        S->cgloop = nullptr;
+        C.exec = nullptr;
         cudaGetLastError();
         return false;
     }
-    S->cgloop_p = p;
-    S->cgloop_gen = S->gen;
+    C.p = p;
+    C.gen = S->gen;
     return true;
 }
 
@@ -3319,7 +3327,7 @@ static aw_status solve_aligned(aw_solver* S, const float* d_b, void* d_p, int32_
                 st = set_error(AW_ERR_NOT_CONVERGED, "relative residual %.3e after %d cycles", rel, it);
                 break;
             }
-            st = run_vcycle(S, S->solve_cycle, false, s);
+            st = run_vcycle(S, false, false, s);
             if (st != AW_OK) break;
         }
         S->x0 = nullptr;
@@ -3371,7 +3379,7 @@ static aw_status solve_aligned(aw_solver* S, const float* d_b, void* d_p, int32_
                 st = set_error(AW_ERR_NOT_CONVERGED, "relative residual %.3e after %d iterations", rel, it);
                 break;
             }
-            st = run_vcycle(S, S->solve_cycle, true, s);
+            st = run_vcycle(S, false, true, s);
             if (st != AW_OK) break;
             // the kernels of one iteration as programmatic dependents of one another
             if ((st = launch_dep(S, k_dot32, ndot32, 256, 0, s, L0.b.p, L0.x.p, L0.fluid.p, nc, S->partials32.p)) != AW_OK) break;
@@ -3433,8 +3441,10 @@ static aw_status solve_aligned(aw_solver* S, const float* d_b, void* d_p, int32_
                 st = set_error(AW_ERR_NOT_CONVERGED, "relative residual %.3e after %d iterations", rel, it);
                 break;
             }
-            if (S->use_graph && S->use_devloop && (S->cgloop_p != (const void*)p || S->cgloop_gen != S->gen) &&
-                !cg_devloop_build(S, p, ndot))
+            auto fits = [&](const aw_solver::Loop& l) { return l.exec && l.p == (const void*)p && l.gen == S->gen; };
+            if (!fits(S->cgloop[S->cgloop_last])) S->cgloop_last ^= 1;
+            aw_solver::Loop& loop = S->cgloop[S->cgloop_last];
+            if (S->use_graph && S->use_devloop && !fits(loop) && !cg_devloop_build(S, loop, p, ndot))
                 S->use_devloop = false;  // no such graph on this device: the host loop below
             if (restart) {
                 // {iterations, restart flag, limit} and {||b||, tolerance}, kept on the device by the iterations
@@ -3449,13 +3459,13 @@ static aw_status solve_aligned(aw_solver* S, const float* d_b, void* d_p, int32_
             if (S->use_graph && S->use_devloop) {
                 // iterations on the device until the recursive residual converges, turns NaN or the
                 // limit is reached; then one read-back of ||r||^2 and the iteration count
-                AW_CUDA(cudaGraphLaunch(S->cgloop, s));
+                AW_CUDA(cudaGraphLaunch(loop.exec, s));
                 AW_CUDA(cudaMemcpyAsync(S->h_cg, S->norm.p, sizeof(double), cudaMemcpyDeviceToHost, s));
                 AW_CUDA(cudaMemcpyAsync(S->h_cg + 1, S->cgst.p, sizeof(int), cudaMemcpyDeviceToHost, s));
                 AW_CUDA(cudaStreamSynchronize(s));
                 int it1 = 0;
                 memcpy(&it1, S->h_cg + 1, sizeof(int));
-                g_launches += S->cgloop_kernels * (unsigned long long)(it1 - it);
+                g_launches += loop.kernels * (unsigned long long)(it1 - it);
                 it = it1;
                 rn = std::sqrt(S->h_cg[0]);
                 continue;

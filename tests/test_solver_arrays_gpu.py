@@ -298,3 +298,47 @@ def test_reference_operator_iterates_on_air_cells_too(R0):
     assert float((want - b)[fluid == 0].abs().max()) > 100 * tol
     sv.close()
     g.close()
+
+
+@pytest.mark.parametrize("precision", [aw.PRECISION_FP32, aw.PRECISION_MIXED])
+def test_operators_by_turns_capture_nothing_again(precision):
+    """Solves of one density and of a varying one in turn take about as long as each on its own (medians): the graphs
+    of both forms are kept."""
+    g = _grid(8, (8, 8, 4))
+    n, fluid, b0 = _problem(g, 8)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    sv = aw.Solver(g, precision=precision, tolerance=1e-30, max_cycles=2)
+    p = torch.zeros(n, dtype=torch.float64 if precision == aw.PRECISION_MIXED else torch.float32, device="cuda")
+    beta = [g.channel(aw.BETA_COEFF_X + a) for a in range(3)]
+    varied = [0.3 + 0.7 * torch.rand(t.numel(), generator=gen, device="cuda") for t in beta]
+    plain = [torch.ones_like(t) for t in beta]
+
+    def solve(values):
+        for t, v in zip(beta, values):
+            t.copy_(v)
+        sv.update_coefficients()
+        sv.setup(fluid)
+        p.zero_()
+        sv.solve(b0, p, raise_on_error=False)
+        return p.clone()
+
+    def seconds(*calls):
+        t = []
+        for _ in range(60):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            for c in calls:
+                solve(c)
+            torch.cuda.synchronize()
+            t.append(time.perf_counter() - t0)
+        return statistics.median(t[10:])
+
+    ref = [solve(plain), solve(varied)]
+    assert not torch.equal(*ref)
+    alone = seconds(plain) + seconds(varied)
+    pair = seconds(plain, varied)
+    for _ in range(2):
+        assert torch.equal(solve(plain), ref[0]) and torch.equal(solve(varied), ref[1])
+    assert pair < 1.3 * alone, (pair, alone)
+    sv.close()
+    g.close()
