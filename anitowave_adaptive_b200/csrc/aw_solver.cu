@@ -977,10 +977,6 @@ __global__ void __launch_bounds__(256) k_cg_update(CgVec K, double* part, unsign
         if constexpr (DEV) cudaGraphSetConditional(h, (rel == rel && rel >= K.prm[1] && it < K.st[2]) ? 1u : 0u);
     });
 }
-__global__ void k_fill_zero(float* __restrict__ x, size_t n) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) x[i] = 0.f;
-}
 
 // ---- conjugate gradients with every vector and scalar in FP32 (AW_PRECISION_FP32_PCG) ----------
 // The same V-cycle preconditioner as the mixed form, without its FP64 residual, direction and
@@ -1872,79 +1868,79 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) k_dense_tail(const __grid_con
     for (int step = 0;; ++step) {
         if (step == npre) {
 #pragma unroll
-    for (int j = 0; j < 2 * TAIL_PAIRS; ++j) {
-        const int i = j >> 1;
-        float r = 0.f;
-        if ((fl >> j) & 1u) {
-            float v[6];
-            neighbours(i, j & 1, v);
-            r = b[j] - (T.from_msbg ? tail_block_resid(w[j], v, diag[j], x[j]) : ufma(diag[j], x[j], tail_uniform(w[j], v)));
-            rs[2 * (tid + i * TAIL_THREADS) + (odd[i] ^ (j & 1))] = r;
-        }
-        if (T.r && ((act >> j) & 1u)) T.r[at[j]] = r;
-    }
-    __syncthreads();
-    // ---- the levels below, by the warps that cover the first of them
-    const int nt = (lattice_cells(T.lv[0].d) + 31) & ~31;
-    if (tid < nt) {
-#pragma unroll 1
-        for (int l = 0; l < T.n; ++l) {
-            const TailLow L = tail_low(T, low, l);
-            if (L.mine) {
-                const float* r = l == 0 ? rs : low + T.low[l - 1] + lattice_padded(T.lv[l - 1].d) + lattice_cells(T.lv[l - 1].d);
-                const float s = tail_restrict(r + L.child, l == 0 ? d0 : T.lv[l - 1].d);
-                const float b = L.fluid ? s : 0.f;
-                L.b[tid] = b;
-                T.lb[l][tid] = b;
+            for (int j = 0; j < 2 * TAIL_PAIRS; ++j) {
+                const int i = j >> 1;
+                float r = 0.f;
+                if ((fl >> j) & 1u) {
+                    float v[6];
+                    neighbours(i, j & 1, v);
+                    r = b[j] - (T.from_msbg ? tail_block_resid(w[j], v, diag[j], x[j]) : ufma(diag[j], x[j], tail_uniform(w[j], v)));
+                    rs[2 * (tid + i * TAIL_THREADS) + (odd[i] ^ (j & 1))] = r;
+                }
+                if (T.r && ((act >> j) & 1u)) T.r[at[j]] = r;
             }
-            tail_bar(nt);
-            if (l + 1 == T.n) break;
-            tail_low_smooth(L, T.sweeps, 0, T.omega, nt);
-            if (L.mine) {
-                float v[6];
-                tail_nb(L.own, L.sy, L.sz, v);
-                const float r = L.fluid ? L.b[tid] - ufma(L.diag, *L.own, tail_uniform(L.w, v)) : 0.f;
-                L.r[tid] = r;
-                if (T.r) T.lr[l][tid] = r;
-            }
-            tail_bar(nt);
-        }
+            __syncthreads();
+            // ---- the levels below, by the warps that cover the first of them
+            const int nt = (lattice_cells(T.lv[0].d) + 31) & ~31;
+            if (tid < nt) {
 #pragma unroll 1
-        for (int l = T.n - 1; l >= 0; --l) {
-            const TailLow L = tail_low(T, low, l);
-            if (l + 1 == T.n) {  // the coarsest
-                if (T.exact) {
-                    const double* M = nex <= TAIL_INV ? inv : T.Minv;
-                    const DenseView& d = T.lv[l].d;
-                    for (int i = tid >> 5; i < nex; i += nt >> 5) {  // a warp per row
-                        double s = 0.0;
-                        for (int k = tid & 31; k < nex; k += 32) s += M[(size_t)i * nex + k] * (double)L.b[idx[k]];
-                        s = warp_sum(s);
-                        const int p = idx[i];
-                        if ((tid & 31) == 0)
-                            L.x[pad_index(d, p % d.D[0], (p / d.D[0]) % d.D[1], p / (d.D[0] * d.D[1]))] = (float)s;
+                for (int l = 0; l < T.n; ++l) {
+                    const TailLow L = tail_low(T, low, l);
+                    if (L.mine) {
+                        const float* r = l == 0 ? rs : low + T.low[l - 1] + lattice_padded(T.lv[l - 1].d) + lattice_cells(T.lv[l - 1].d);
+                        const float s = tail_restrict(r + L.child, l == 0 ? d0 : T.lv[l - 1].d);
+                        const float b = L.fluid ? s : 0.f;
+                        L.b[tid] = b;
+                        T.lb[l][tid] = b;
                     }
                     tail_bar(nt);
-                } else {
-                    tail_low_smooth(L, T.coarsest_iters, 0, T.omega, nt);
+                    if (l + 1 == T.n) break;
+                    tail_low_smooth(L, T.sweeps, 0, T.omega, nt);
+                    if (L.mine) {
+                        float v[6];
+                        tail_nb(L.own, L.sy, L.sz, v);
+                        const float r = L.fluid ? L.b[tid] - ufma(L.diag, *L.own, tail_uniform(L.w, v)) : 0.f;
+                        L.r[tid] = r;
+                        if (T.r) T.lr[l][tid] = r;
+                    }
+                    tail_bar(nt);
                 }
-                if (L.mine) T.lx[l][tid] = *L.own;
-                continue;
+#pragma unroll 1
+                for (int l = T.n - 1; l >= 0; --l) {
+                    const TailLow L = tail_low(T, low, l);
+                    if (l + 1 == T.n) {  // the coarsest
+                        if (T.exact) {
+                            const double* M = nex <= TAIL_INV ? inv : T.Minv;
+                            const DenseView& d = T.lv[l].d;
+                            for (int i = tid >> 5; i < nex; i += nt >> 5) {  // a warp per row
+                                double s = 0.0;
+                                for (int k = tid & 31; k < nex; k += 32) s += M[(size_t)i * nex + k] * (double)L.b[idx[k]];
+                                s = warp_sum(s);
+                                const int p = idx[i];
+                                if ((tid & 31) == 0)
+                                    L.x[pad_index(d, p % d.D[0], (p / d.D[0]) % d.D[1], p / (d.D[0] * d.D[1]))] = (float)s;
+                            }
+                            tail_bar(nt);
+                        } else {
+                            tail_low_smooth(L, T.coarsest_iters, 0, T.omega, nt);
+                        }
+                        if (L.mine) T.lx[l][tid] = *L.own;
+                        continue;
+                    }
+                    if (L.fluid) *L.own += (low + T.low[l + 1])[L.parent];
+                    tail_bar(nt);
+                    tail_low_smooth(L, T.sweeps, 1, T.omega, nt);
+                    if (L.mine) T.lx[l][tid] = *L.own;
+                }
             }
-            if (L.fluid) *L.own += (low + T.low[l + 1])[L.parent];
-            tail_bar(nt);
-            tail_low_smooth(L, T.sweeps, 1, T.omega, nt);
-            if (L.mine) T.lx[l][tid] = *L.own;
-        }
-    }
-    __syncthreads();
+            __syncthreads();
 #pragma unroll
-    for (int j = 0; j < 2 * TAIL_PAIRS; ++j)
-        if ((fl >> j) & 1u) {
-            x[j] += (low + T.low[0])[parent[j >> 1]];
-            xs[(j & 1) * np0 + cell[j >> 1]] = x[j];
-        }
-    __syncthreads();
+            for (int j = 0; j < 2 * TAIL_PAIRS; ++j)
+                if ((fl >> j) & 1u) {
+                    x[j] += (low + T.low[0])[parent[j >> 1]];
+                    xs[(j & 1) * np0 + cell[j >> 1]] = x[j];
+                }
+            __syncthreads();
         }
         if (step == npass) break;
         if (((step - npre) & 1) == (step < npre ? 0 : 1)) pass(0);

@@ -48,12 +48,12 @@ enum { US_AIR = 0, US_UNIFORM = 1, US_GENERAL = 2 };
 
 // The arrays of a level start on 16 bytes (the solver's own do, aw_solve sees to the caller's): a pair of cells
 // at an even index is one access.
+//
 // One block-structured level as the kernels below see it.  Slots: the level's active blocks, colour 0
 // then colour 1, resolutions descending.  Warp w serves desc[w] = {first slot, count | res << 8}.
 //   rec: {cell offset, block, kinds, coarse cell offset}, neighbour cell offsets (6), neighbour blocks
-//        (6), neighbour coarse cell offsets (6), face offsets (3), coarse resolution
-//   kinds: 4 bits per face direction (NB_*), bit 24 + f: neighbour f is halved on the coarse level,
-//        bit 30: the block itself is
+//        (6), neighbour coarse cell offsets (6), face offsets (3)
+//   kinds: 4 bits per face direction (NB_*), bit 24 + f: neighbour f is halved on the coarse level
 //   wt:  {interior, -x, +x, -y}, {+y, -z, +z, state}
 //   mask: fluid bit 2 z + i of the lane's cell (2 xp + i, y, z), 32 lanes per warp
 struct UniView {
@@ -204,7 +204,6 @@ struct ULane {
     __device__ __forceinline__ int nbblk(int f) const { return word(10 + f); }
     __device__ __forceinline__ uint32_t nbcoff(int f) const { return (uint32_t)word(16 + f); }
     __device__ __forceinline__ uint32_t foff(int a) const { return (uint32_t)word(22 + a); }
-    __device__ __forceinline__ int cres() const { return word(25); }
 };
 
 // One face of the block's halo: the neighbouring cell layer at (u, v) along the axes (a + 1, a + 2) mod
@@ -1524,14 +1523,12 @@ __global__ void k_build_records(Geo geo, const int* __restrict__ blocks, int n, 
         rec[10 + f] = nbk;
         rec[16 + f] = oc;
     }
-    if (coarser.res && r == 2 * coarser.res[b]) kinds |= 1 << 30;
     rec[0] = (int)h.off[0][b];
     rec[1] = b;
     rec[2] = kinds;
     rec[3] = coarser.res ? (int)coarser.off[0][b] : 0;
     for (int a = 0; a < 3; ++a) rec[22 + a] = (int)h.off[1 + a][b];
-    rec[25] = coarser.res ? coarser.res[b] : 0;
-    for (int k = 26; k < 4 * UREC; ++k) rec[k] = 0;
+    for (int k = 25; k < 4 * UREC; ++k) rec[k] = 0;
 }
 
 }  // namespace aw
