@@ -611,6 +611,7 @@ constexpr int P2G_BINS = 128;  // counts told apart when a block's cells are ord
 constexpr int P2G_MAX_SLICES = 1 << 19;  // 6 * 8^3 * this stays below 2^31
 constexpr int P2G_MAX_CELLS = 16 * 16 * 16;  // cells of the largest block (base resolution <= 16)
 constexpr int P2G_NEAR_CELLS = 8 * 8 * 8;    // blocks up to this size list their near cells
+static_assert(P2G_BINS % 32 == 0 && P2G_BINS <= 256 && P2G_BINS <= P2G_NEAR_CELLS, "a warp scans them, a thread clears each");
 __device__ __forceinline__ int p2g_bin(uint32_t cnt) {
     if (cnt < 64u) return (int)cnt;
     const int e = 31 - __clz((int)cnt);  // >= 6; the last bin takes 15360 and more
