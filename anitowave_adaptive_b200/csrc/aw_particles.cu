@@ -835,8 +835,9 @@ __global__ void __launch_bounds__(P2G_THREADS, 2) k_p2g_own(LevelView L, const f
     __syncthreads();
     if (wid == 0) {  // exclusive scans: the bins from the fullest down, the chunks' counts of coarse-near cells
         int carry = 0, carry2 = 0;
-        for (int base = 0; base < P2G_BINS; base += 32) {
-            const int k = P2G_BINS - 1 - base - lane;
+        const int top = p2g_bin(maxcnt) | 31;  // no cell lies in the bins above
+        for (int base = 0; base <= top; base += 32) {
+            const int k = top - base - lane;
             const int v = hist[k];
             int incl = v;
 #pragma unroll
